@@ -766,14 +766,14 @@ int build_plans(ns_handle* h) {
   const bool xper = P.kind[0] == 0;
   const int nxs = xper ? nxh : nx / 2;
   // Twiddles W_N^m = exp(-2 pi i m / N), computed in long double (FFT axes only).
-  auto twid = [](int N, int count, std::vector<double2>& out) {
+  auto twid = [](int N, int count, std::vector<int4>& out) {
     const long double pi = 3.141592653589793238462643383279502884L;
     for (int m = 0; m < count; ++m) {
       const long double th = 2.0L * pi * (long double)m / (long double)N;
-      out.push_back(make_double2((double)cosl(th), (double)(-sinl(th))));
+      out.push_back(q60_entry(cosl(th), -sinl(th)));
     }
   };
-  std::vector<double2> tw;
+  std::vector<int4> tw;
   size_t o_xr = 0, o_y = 0, o_z = 0;
   if (xper) {
     twid(M, M, tw);
@@ -799,12 +799,13 @@ int build_plans(ns_handle* h) {
     o_dwf = tw.size();
     for (int k = 0; k <= ny; ++k) {
       const long double th = pi * (long double)k / (2.0L * ny);
-      tw.push_back(make_double2((double)(cosl(th) / 2.0L), (double)(-sinl(th) / 2.0L)));
+      tw.push_back(q60_entry(cosl(th) / 2.0L, -sinl(th) / 2.0L));
     }
     o_dwi = tw.size();
+    const long double f = std::ldexp(1.0L, std::ilogb(ny));
     for (int k = 0; k < ny; ++k) {
       const long double th = pi * (long double)k / (2.0L * ny);
-      tw.push_back(make_double2((double)(cosl(th) / ny), (double)(sinl(th) / ny)));
+      tw.push_back(q60_entry(cosl(th) * f / ny, sinl(th) * f / ny));
     }
   }
   // The same for a wall x axis (NS_DENSE_X keeps the dense products).
@@ -818,17 +819,18 @@ int build_plans(ns_handle* h) {
     o_xwf = tw.size();
     for (int k = 0; k <= nx; ++k) {
       const long double th = pi * (long double)k / (2.0L * nx);
-      tw.push_back(make_double2((double)(cosl(th) / 2.0L), (double)(-sinl(th) / 2.0L)));
+      tw.push_back(q60_entry(cosl(th) / 2.0L, -sinl(th) / 2.0L));
     }
     o_xwi = tw.size();
+    const long double f = std::ldexp(1.0L, std::ilogb(nx));
     for (int k = 0; k < nx; ++k) {
       const long double th = pi * (long double)k / (2.0L * nx);
-      tw.push_back(make_double2((double)(cosl(th) / nx), (double)(sinl(th) / nx)));
+      tw.push_back(q60_entry(cosl(th) * f / nx, sinl(th) * f / nx));
     }
   }
-  if (tw.empty()) tw.push_back(make_double2(1.0, 0.0));
-  NS_CUDA(h, cudaMalloc(&h->tw, tw.size() * sizeof(double2)));
-  NS_CUDA(h, cudaMemcpyAsync(h->tw, tw.data(), tw.size() * sizeof(double2), cudaMemcpyHostToDevice, h->stream));
+  if (tw.empty()) tw.push_back(int4{});
+  NS_CUDA(h, cudaMalloc(&h->tw, tw.size() * sizeof(int4)));
+  NS_CUDA(h, cudaMemcpyAsync(h->tw, tw.data(), tw.size() * sizeof(int4), cudaMemcpyHostToDevice, h->stream));
   // Per-axis eigenvalues lambda = -4 sin^2(..)/h^2 of each mode.
   std::vector<double> e3[3];
   for (int a = 0; a < 3; ++a) {

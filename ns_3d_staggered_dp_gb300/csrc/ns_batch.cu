@@ -650,26 +650,32 @@ int ns_batch_destroy(ns_batch* b) {
   return NS_OK;
 }
 
-// The tables of an FFT-based DCT line of N points as (re, im) pairs: the
-// N-point twiddles exp(-2 pi i m / N), m < N, the forward post-twiddles
-// exp(-i pi k / (2N)) / 2, k <= N, and the inverse pre-twiddles
-// exp(i pi k / (2N)) / N, k < N; computed in long double.
+// The tables of an FFT-based DCT line of N points as fixed-point (re, im)
+// entries (two doubles of storage each): the N-point twiddles
+// exp(-2 pi i m / N), m < N, the forward post-twiddles exp(-i pi k / (2N)) / 2,
+// k <= N, and the inverse pre-twiddles exp(i pi k / (2N)) 2^f / N,
+// f = floor(log2 N), k < N; computed in long double.
 static void append_dct_tables(int N, std::vector<double>& tab) {
   const long double pi = 3.141592653589793238462643383279502884L;
+  auto put = [&](long double re, long double im) {
+    const int4 q = q60_entry(re, im);
+    double d[2];
+    std::memcpy(d, &q, sizeof(q));
+    tab.push_back(d[0]);
+    tab.push_back(d[1]);
+  };
   for (int m = 0; m < N; ++m) {
     const long double th = 2.0L * pi * (long double)m / (long double)N;
-    tab.push_back((double)cosl(th));
-    tab.push_back((double)(-sinl(th)));
+    put(cosl(th), -sinl(th));
   }
   for (int k = 0; k <= N; ++k) {
     const long double th = pi * (long double)k / (2.0L * N);
-    tab.push_back((double)(cosl(th) / 2.0L));
-    tab.push_back((double)(-sinl(th) / 2.0L));
+    put(cosl(th) / 2.0L, -sinl(th) / 2.0L);
   }
+  const long double f = std::ldexp(1.0L, std::ilogb(N));
   for (int k = 0; k < N; ++k) {
     const long double th = pi * (long double)k / (2.0L * N);
-    tab.push_back((double)(cosl(th) / N));
-    tab.push_back((double)(sinl(th) / N));
+    put(cosl(th) * f / N, sinl(th) * f / N);
   }
 }
 
@@ -906,12 +912,12 @@ int ns_batch_create(const ns_batch_config* cfg, const ns_subdomain* subs, int n,
     S.eig_x = b->tables + ex[d.nx];
     S.eig_o = b->tables + ey[d.ny];
     if (dct_x_on && dct_size(d.nx)) {
-      const double2* t2 = reinterpret_cast<const double2*>(b->tables + dtab[d.nx]);
+      const int4* t2 = reinterpret_cast<const int4*>(b->tables + dtab[d.nx]);
       S.dct_x = c.pbc;
       S.dctx_tw = t2; S.dctx_wf = t2 + d.nx; S.dctx_wi = t2 + 2 * d.nx + 1;
     }
     if (dct_y_on && dct_size(d.ny)) {
-      const double2* t2 = reinterpret_cast<const double2*>(b->tables + dtab[d.ny]);
+      const int4* t2 = reinterpret_cast<const int4*>(b->tables + dtab[d.ny]);
       S.dct_y = c.pbc;
       S.dct_tw = t2; S.dct_wf = t2 + d.ny; S.dct_wi = t2 + 2 * d.ny + 1;
     }

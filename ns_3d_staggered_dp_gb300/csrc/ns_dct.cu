@@ -821,7 +821,7 @@ __device__ __forceinline__ void batch_dct(int pass, const BatchSpecArgs& a, doub
   constexpr int LPC = batch_dct_lpc(N);
   const FOne c{a.d.one, a.d.mzero};
   const int l = threadIdx.x % LPC, t = threadIdx.x / LPC;
-  if (pass == 0) dct_x_fwd_body<N, PB, false, LPC>(a.S, nullptr, a.spec, sb, bx, l, t, c);
+  if (pass == 0) dct_x_fwd_body<N, PB, LPC>(a.S, a.spec, sb, bx, l, t, c);
   else if (pass == 1) dct_x_inv_body<N, PB, LPC>(a.S, a.spec, a.dp, a.L, sb, bx, l, t, c);
   else if (pass == 2) dct_y_body<N, true, PB, LPC>(a.S, a.spec, sb, bx, l, t, c);
   else dct_y_body<N, false, PB, LPC>(a.S, a.spec, sb, bx, l, t, c);
@@ -964,9 +964,9 @@ void spec_pass_grid(int pass, const SpecPlan& S, int& gx, int& gy) {
 size_t spec_pass_smem(int pass, const SpecPlan& S) {
   if ((pass == 0 || pass == 1) && S.dct_x) {
     const size_t L = batch_dct_lpc(S.nx);
-    return (size_t)S.nx * L * sizeof(double2) + L * (S.nx + 1) * sizeof(double2);
+    return (size_t)S.nx * L * sizeof(i2) + L * (S.nx + 1) * sizeof(double2) + 128 * sizeof(FxExp);
   }
-  if ((pass == 2 || pass == 3) && S.dct_y) return (size_t)S.ny * batch_dct_lpc(S.ny) * sizeof(double2);
+  if ((pass == 2 || pass == 3) && S.dct_y) return (size_t)S.ny * batch_dct_lpc(S.ny) * sizeof(i2) + 128 * sizeof(FxExp);
   if (pass == 0) return (size_t)(128 / dense_x_group(S.nx)) * S.nx * sizeof(double);
   if (pass == 1) return (size_t)(128 / dense_x_inv_group(S.sym[0], S.nx)) * S.nx * sizeof(double);
   if (pass == 2 || pass == 3) return (size_t)S.ny * 16 * sizeof(double2);

@@ -13,13 +13,19 @@
 //   y-inverse, x-inverse (c2r, writes dp slots 1..nx)
 // A line of N = R1*R2 points is transformed in two register passes
 // ("four-step"): R1 threads each do an R2-point DFT, a twiddle multiply and a
-// shared-memory transpose, then R1-point DFTs.  Register DFTs are radix-2
-// decimation-in-time with every butterfly in Linzer-Feig FMA form (6 FMAs
-// for a general twiddle, 4 for the trivial ones).  The spectrum is
+// shared-memory transpose, then R1-point DFTs, all on block fixed-point
+// integers (ns_fixed.cuh).  The spectrum is
 // (nx/2+1, ny, nz) complex with x fastest, as the reference's DFTI
 // descriptor (cstrides, :217-221).  The overall scale of the forward split,
 // the inverse split and the 1/N of the backward transform are folded into
 // the inverse-eigenvalue table.
+//
+// What bounds the passes at 256^3 (FP64 transforms before, in parentheses):
+// y forward 0.112 ms (0.372), y inverse 0.108 (0.371), x inverse 0.117
+// (0.440): integer issue at half of the slots beside the FP64 pipe at 50% (the
+// conversions back), DRAM at 2 TB/s; the FP64 transforms held that pipe at
+// 85-90%.  x forward 0.297 (0.626): the divergence and the conversions back,
+// 18 FP64 instructions a cell pair, hold the pipe at 75%.
 #include "ns_fft_core.cuh"
 #include "ns_internal.cuh"
 #include "ns_kernels.cuh"
@@ -62,36 +68,56 @@ template <int AXIS, int N, int DIR>
 __global__ void __launch_bounds__(lpc<N>() * Split<N>::R1) fft_yz_kernel(FftPlan P, double2* __restrict__ spec, FOne c,
                                                                           int o0, int o1) {
   using F = YZ<N>;
-  constexpr int LPC = F::LPC;
+  constexpr int LPC = F::LPC, T = F::T, R1 = F::R1, R2 = F::R2, KQ = F::KQ;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double2* sb = reinterpret_cast<double2*>(smem_raw);
+  i2* sb = reinterpret_cast<i2*>(smem_raw);
+  FxExp* se = reinterpret_cast<FxExp*>(sb + N * LPC);
   const int l = threadIdx.x, t = threadIdx.y;
   const LineGeo G = yz_line(AXIS, P.nxh, P.ny, l, LPC, o0, o1);
   if ((int)blockIdx.x == yz_nblk(P.nxh, LPC) && (int)(blockIdx.y * LPC) >= o1 - o0) return;  // whole block idle
   double2* g = spec + G.base;
   const long long st = AXIS == 1 ? (long long)P.nxh : (long long)P.nxh * P.ny;
-  const double2* tw = AXIS == 1 ? P.tw_y : P.tw_z;
+  const int4* tw = AXIS == 1 ? P.tw_y : P.tw_z;
   if (DIR < 0) {
-    if (G.valid) F::fwdA(g, st, sb, tw, l, t, c);
+    double2 d[R2];
+#pragma unroll
+    for (int n2 = 0; n2 < R2; ++n2)
+      d[n2] = G.valid ? g[(long long)(t + R1 * n2) * st] : make_double2(0.0, 0.0);
+    F::fwdA(d, sb, se, tw, l, t);
     __syncthreads();
-    double2 xk[F::KQ][F::R1];
-    F::fwdB(xk, sb, l, t, c);
+    i2 xk[KQ][R1];
+    const FxOut fo = fx_out(F::fwdB(xk, sb, se, l, t));
     if (G.valid) {
 #pragma unroll
-      for (int q = 0; q < F::KQ; ++q)
+      for (int q = 0; q < KQ; ++q)
 #pragma unroll
-        for (int k1 = 0; k1 < F::R1; ++k1) g[(long long)(t + F::T * q + F::R2 * k1) * st] = xk[q][k1];
+        for (int k1 = 0; k1 < R1; ++k1) g[(long long)(t + T * q + R2 * k1) * st] = fx_to(xk[q][k1], fo, c);
+      if (fo.odd)
+#pragma unroll 1
+        for (int i = 0; i < R2; ++i) fx_rescale(g[(long long)(t + T * i) * st], fo);
     }
   } else {
-    double2 xk[F::KQ][F::R1];
+    double2 d[KQ][R1];
 #pragma unroll
-    for (int q = 0; q < F::KQ; ++q)
+    for (int q = 0; q < KQ; ++q)
 #pragma unroll
-      for (int k1 = 0; k1 < F::R1; ++k1)
-        xk[q][k1] = G.valid ? g[(long long)(t + F::T * q + F::R2 * k1) * st] : make_double2(0.0, 0.0);
-    F::invA(xk, sb, tw, l, t, c);
+      for (int k1 = 0; k1 < R1; ++k1)
+        d[q][k1] = G.valid ? g[(long long)(t + T * q + R2 * k1) * st] : make_double2(0.0, 0.0);
+    {
+      i2 xk[KQ][R1];
+      const int eb = F::block(d, xk);
+      F::invA(xk, eb, sb, se, tw, l, t);
+    }
     __syncthreads();
-    if (G.valid) F::invB(g, st, sb, l, t, c);
+    i2 x[R2];
+    const FxOut fo = fx_out(F::invB(x, sb, se, l, t));
+    if (G.valid) {
+#pragma unroll
+      for (int b = 0; b < R2; ++b) g[(long long)(t + R1 * b) * st] = fx_to(x[b], fo, c);
+      if (fo.odd)
+#pragma unroll 1
+        for (int b = 0; b < R2; ++b) fx_rescale(g[(long long)(t + R1 * b) * st], fo);
+    }
   }
 }
 
@@ -105,52 +131,83 @@ __global__ void __launch_bounds__(lpc<N>() * Split<N>::R1) dct_y_kernel(FftPlan 
 template <int N>
 __global__ void __launch_bounds__(lpc<N>() * Split<N>::R1) fft_z_solve_kernel(FftPlan P, double2* __restrict__ spec, FOne c) {
   using F = YZ<N>;
-  constexpr int LPC = F::LPC;
+  constexpr int LPC = F::LPC, T = F::T, R1 = F::R1, R2 = F::R2, KQ = F::KQ;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double2* sb = reinterpret_cast<double2*>(smem_raw);
+  i2* sb = reinterpret_cast<i2*>(smem_raw);
+  FxExp* se = reinterpret_cast<FxExp*>(sb + N * LPC);
   const int l = threadIdx.x, t = threadIdx.y;
   if ((int)blockIdx.x == yz_nblk(P.nxh, LPC) && blockIdx.y * LPC >= (unsigned)P.ny) return;
   const LineGeo G = yz_line(2, P.nxh, P.ny, l, LPC, 0, P.ny);
   double2* g = spec + G.base;
   const double* lam = P.inv_lam + G.base;
   const long long st = (long long)P.nxh * P.ny;
-  if (G.valid) F::fwdA(g, st, sb, P.tw_z, l, t, c);
+  {
+    double2 d[R2];
+#pragma unroll
+    for (int n2 = 0; n2 < R2; ++n2)
+      d[n2] = G.valid ? g[(long long)(t + R1 * n2) * st] : make_double2(0.0, 0.0);
+    F::fwdA(d, sb, se, P.tw_z, l, t);
+  }
   __syncthreads();
-  double2 xk[F::KQ][F::R1];
-  F::fwdB(xk, sb, l, t, c);
+  {
+    i2 xk[KQ][R1];
+    const FxOut fo = fx_out(F::fwdB(xk, sb, se, l, t));
+    double2 d[KQ][R1];
 #pragma unroll
-  for (int q = 0; q < F::KQ; ++q)
+    for (int q = 0; q < KQ; ++q)
 #pragma unroll
-    for (int k1 = 0; k1 < F::R1; ++k1) {
-      const int kz = t + F::T * q + F::R2 * k1;
-      const double s = G.valid ? __ldg(lam + (long long)kz * st) : 0.0;
-      xk[q][k1].x = fmul(c, xk[q][k1].x, s);
-      xk[q][k1].y = fmul(c, xk[q][k1].y, s);
-      // singular mode of a Neumann/periodic mix: fixed mean (NS_functions.f90:1576-1577)
-      if (P.has_mean && G.valid && G.base == 0 && kz == 0) xk[q][k1] = make_double2(P.mean_val, 0.0);
+      for (int k1 = 0; k1 < R1; ++k1) d[q][k1] = fx_to(xk[q][k1], fo, c);
+    if (fo.odd) {
+#pragma unroll
+      for (int q = 0; q < KQ; ++q)
+#pragma unroll
+        for (int k1 = 0; k1 < R1; ++k1) fx_rescale(d[q][k1], fo);
     }
+#pragma unroll
+    for (int q = 0; q < KQ; ++q)
+#pragma unroll
+      for (int k1 = 0; k1 < R1; ++k1) {
+        const int kz = t + T * q + R2 * k1;
+        const double s = G.valid ? __ldg(lam + (long long)kz * st) : 0.0;
+        d[q][k1] = make_double2(fmul(c, d[q][k1].x, s), fmul(c, d[q][k1].y, s));
+        // singular mode of a Neumann/periodic mix: fixed mean (NS_functions.f90:1576-1577)
+        if (P.has_mean && G.valid && G.base == 0 && kz == 0) d[q][k1] = make_double2(P.mean_val, 0.0);
+      }
+    const int eb = F::block(d, xk);
+    __syncthreads();
+    F::invA(xk, eb, sb, se, P.tw_z, l, t);
+  }
   __syncthreads();
-  F::invA(xk, sb, P.tw_z, l, t, c);
-  __syncthreads();
-  if (G.valid) F::invB(g, st, sb, l, t, c);
+  i2 x[R2];
+  const FxOut fo = fx_out(F::invB(x, sb, se, l, t));
+  if (G.valid) {
+#pragma unroll
+    for (int b = 0; b < R2; ++b) g[(long long)(t + R1 * b) * st] = fx_to(x[b], fo, c);
+    if (fo.odd)
+#pragma unroll 1
+      for (int b = 0; b < R2; ++b) fx_rescale(g[(long long)(t + R1 * b) * st], fo);
+  }
 }
 
 // ---------------------------------------------------------------------------
 // x passes: T threads per line are consecutive lanes (lines are contiguous).
 // Shared buffer per line: R1 rows of (R2 + 1) entries, then the packed
-// M-point spectrum for the real/complex split.
+// M-point spectrum for the real/complex split; then the exponents of the
+// line's threads, two sets (the inverse exchanges blocks twice).
 // ---------------------------------------------------------------------------
 template <int M>
 struct XP {
   static constexpr int R1 = Split<M>::R1, R2 = Split<M>::R2, T = R1, KQ = R2 / T;
+  static constexpr int B1 = 60 - log2up(R1), B2 = 60 - log2up(R2);
   static constexpr int LINES = 256 / T;          // lines per CTA
   static constexpr int ROW = R2 + 1;             // padded row (bank spread)
   static constexpr int LS = (R1 * ROW > M + 2) ? R1 * ROW : M + 2;  // transpose area, reused by the split
+  static constexpr size_t kSmem = (size_t)LINES * (LS * sizeof(i2) + 2 * T * sizeof(FxExp));
   __device__ static __forceinline__ int sidx(int r, int q) { return r * ROW + q; }
 };
 
 template <int M, bool FROM_RHS, bool HAS_BC>
-__global__ void __launch_bounds__(256) fft_x_fwd_kernel(FftPlan P, DivArgs d, double2* __restrict__ spec) {
+__global__ void __launch_bounds__(256, 2) fft_x_fwd_kernel(FftPlan P, DivArgs d, double2* __restrict__ spec) {
   using X = XP<M>;
   constexpr int R1 = X::R1, R2 = X::R2, T = X::T, KQ = X::KQ;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -162,8 +219,9 @@ __global__ void __launch_bounds__(256) fft_x_fwd_kernel(FftPlan P, DivArgs d, do
   const bool valid = line < ny * nz;
   const int j = valid ? 1 + line % ny : 1;
   const int k = valid ? 1 + line / ny : 1;
-  double2* sb = reinterpret_cast<double2*>(smem_raw) + (long long)l * X::LS;
-  double2* zb = sb;  // the split area reuses the transpose area after a barrier
+  i2* sb = reinterpret_cast<i2*>(smem_raw) + (long long)l * X::LS;
+  i2* zb = sb;  // the split area reuses the transpose area after a barrier
+  FxExp* se = reinterpret_cast<FxExp*>(reinterpret_cast<i2*>(smem_raw) + X::LINES * X::LS) + l * 2 * T;
   const FOne& cc = c;
   // Step A: packed input z[m] = r[2m] + i r[2m+1], m = n1 + R1 n2, n1 = t.
   {
@@ -199,24 +257,41 @@ __global__ void __launch_bounds__(256) fft_x_fwd_kernel(FftPlan P, DivArgs d, do
       }
       x[n2] = make_double2(r0, r1);
     }
-    dft<R2, -1>(x, cc);
-    sb[X::sidx(t, 0)] = x[0];
+    i2 v[R2];
+    const int eb = fx_block2<X::B2>(x, v);
+    dft<R2, -1>(v);
+    unsigned acc = 0;
+    fx_bits(acc, v[0]);
+    sb[X::sidx(t, 0)] = v[0];
 #pragma unroll
-    for (int k2 = 1; k2 < R2; ++k2) sb[X::sidx(t, k2)] = cmul(cc, x[k2], __ldg(P.tw_x + ((t * k2) % M)));
+    for (int k2 = 1; k2 < R2; ++k2) {
+      const i2 y = fx_cmul(v[k2], fx_ldg(P.tw_x + ((t * k2) % M)));
+      fx_bits(acc, y);
+      sb[X::sidx(t, k2)] = y;
+    }
+    se[t] = fx_publish<X::B1 - 1>(eb, acc);  // one bit for the split's sums
   }
   __syncthreads();
   // Step B: Z[k2 + R2 k1] to the split area.
+  int ec = -kFxNonfinite;
   {
-    double2 x[KQ][R1];
+    int eb[R1];
+#pragma unroll
+    for (int n1 = 0; n1 < R1; ++n1) {
+      const FxExp e = se[n1];
+      eb[n1] = e.eb;
+      ec = max(ec, e.p);
+    }
+    i2 x[KQ][R1];
 #pragma unroll
     for (int q = 0; q < KQ; ++q)
 #pragma unroll
-      for (int n1 = 0; n1 < R1; ++n1) x[q][n1] = sb[X::sidx(n1, t + T * q)];
+      for (int n1 = 0; n1 < R1; ++n1) x[q][n1] = fx_align(sb[X::sidx(n1, t + T * q)], eb[n1], ec);
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < KQ; ++q) {
       const int k2 = t + T * q;
-      dft<R1, -1>(x[q], cc);
+      dft<R1, -1>(x[q]);
 #pragma unroll
       for (int k1 = 0; k1 < R1; ++k1) zb[k2 + R2 * k1] = x[q][k1];
     }
@@ -225,28 +300,32 @@ __global__ void __launch_bounds__(256) fft_x_fwd_kernel(FftPlan P, DivArgs d, do
   // Split: X[k] = E - F, X[M-k] = conj(E + F), E = Z[k] + conj(Z[M-k]),
   // F = i W^k (Z[k] - conj(Z[M-k])), W = exp(-2 pi i / nx)   (all times 2).
   if (valid) {
+    const FxOut fo = fx_out(ec);
     double2* out = spec + (long long)P.nxh * ((j - 1) + (long long)P.ny * (k - 1));
     for (int kk = t; kk <= M / 2; kk += T) {
-      const double2 zk = zb[kk];
-      const double2 zm = zb[(M - kk) % M];
-      const double2 E = make_double2(fadd(cc, zk.x, zm.x), fsub(cc, zk.y, zm.y));
-      const double2 O = make_double2(fsub(cc, zk.x, zm.x), fadd(cc, zk.y, zm.y));
-      const double2 w = __ldg(P.tw_xr + kk);
-      // F = i * W * O
-      const double2 WO = cmul(cc, O, w);
-      const double2 Fv = make_double2(-WO.y, WO.x);
-      out[kk] = make_double2(fsub(cc, E.x, Fv.x), fsub(cc, E.y, Fv.y));
-      if (kk == 0) out[M] = make_double2(fadd(cc, E.x, Fv.x), 0.0);
-      else if (kk != M / 2) out[M - kk] = make_double2(fadd(cc, E.x, Fv.x), -fadd(cc, E.y, Fv.y));
+      const i2 zk = zb[kk];
+      const i2 zm = zb[(M - kk) % M];
+      const i2 E{zk.x + zm.x, zk.y - zm.y};
+      const i2 O{zk.x - zm.x, zk.y + zm.y};
+      const i2 WO = fx_cmul(O, fx_ldg(P.tw_xr + kk));  // F = i W O
+      out[kk] = fx_to(i2{E.x + WO.y, E.y - WO.x}, fo, cc);
+      if (kk == 0) out[M] = fx_to(i2{E.x - WO.y, 0}, fo, cc);
+      else if (kk != M / 2) out[M - kk] = fx_to(i2{E.x - WO.y, -(E.y + WO.x)}, fo, cc);
     }
+    if (fo.odd)
+      for (int kk = t; kk <= M / 2; kk += T) {
+        fx_rescale(out[kk], fo);
+        if (kk != M / 2) fx_rescale(out[M - kk], fo);
+      }
   }
 }
 
 template <int M, bool ALIGNED>
-__global__ void __launch_bounds__(256) fft_x_inv_kernel(FftPlan P, const double2* __restrict__ spec, double* dp,
+__global__ void __launch_bounds__(256, 2) fft_x_inv_kernel(FftPlan P, const double2* __restrict__ spec, double* dp,
                                                         Layout L, FOne c, int line0, int line1) {
   using X = XP<M>;
   constexpr int R1 = X::R1, R2 = X::R2, T = X::T, KQ = X::KQ;
+  constexpr int NP = M / 2 / T;  // pairs (kk, M - kk) per thread; thread 0 also takes kk = M/2
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int t = threadIdx.x, l = threadIdx.y;
   const int line = line0 + blockIdx.x * X::LINES + l;
@@ -254,70 +333,119 @@ __global__ void __launch_bounds__(256) fft_x_inv_kernel(FftPlan P, const double2
   const bool valid = line < line1;
   const int j = valid ? 1 + line % ny : 1;
   const int k = valid ? 1 + line / ny : 1;
-  double2* sb = reinterpret_cast<double2*>(smem_raw) + (long long)l * X::LS;
-  double2* zb = sb;  // the unsplit area is reused by the transpose after a barrier
+  i2* sb = reinterpret_cast<i2*>(smem_raw) + (long long)l * X::LS;
+  i2* zb = sb;  // the unsplit area is reused by the transpose after a barrier
+  FxExp* se = reinterpret_cast<FxExp*>(reinterpret_cast<i2*>(smem_raw) + X::LINES * X::LS) + l * 2 * T;
   const double2* in = spec + (long long)P.nxh * ((j - 1) + (long long)P.ny * (k - 1));
   // Unsplit: Z[k] = E + F, Z[M-k] = conj(E - F), E = X[k] + conj(X[M-k]),
   // F = i conj(W^k) (X[k] - conj(X[M-k]))   (all times 2).
-  if (valid) {
-    for (int kk = t; kk <= M / 2; kk += T) {
-      double2 xk = in[kk];
-      double2 xm = in[M - kk];
-      if (kk == 0) { xk.y = 0.0; xm.y = 0.0; }
-      const double2 E = make_double2(fadd(c, xk.x, xm.x), fsub(c, xk.y, xm.y));
-      const double2 D = make_double2(fsub(c, xk.x, xm.x), fadd(c, xk.y, xm.y));
-      const double2 w = __ldg(P.tw_xr + kk);
-      const double2 WD = cmulc(c, D, w);
-      const double2 Fv = make_double2(-WD.y, WD.x);
-      zb[kk] = make_double2(fadd(c, E.x, Fv.x), fadd(c, E.y, Fv.y));
-      if (kk != 0 && kk != M / 2) zb[M - kk] = make_double2(fsub(c, E.x, Fv.x), -fsub(c, E.y, Fv.y));
+  {
+    double2 d[2 * NP + 1];
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+      const int kk = t + T * i;
+      d[2 * i] = valid ? in[kk] : make_double2(0.0, 0.0);
+      d[2 * i + 1] = valid ? in[M - kk] : make_double2(0.0, 0.0);
     }
+    d[2 * NP] = (valid && t == 0) ? in[M / 2] : make_double2(0.0, 0.0);
+    if (t == 0) d[0].y = d[1].y = 0.0;
+    i2 v[2 * NP + 1];
+    const int eb = fx_block2<57>(d, v);
+    unsigned acc = 0;
+#pragma unroll
+    for (int i = 0; i <= NP; ++i) {
+      const int kk = t + T * i;
+      if (i == NP && t != 0) break;
+      const i2 xk = v[2 * i], xm = v[i < NP ? 2 * i + 1 : 2 * NP];
+      const i2 E{xk.x + xm.x, xk.y - xm.y};
+      const i2 D{xk.x - xm.x, xk.y + xm.y};
+      const i2 WD = fx_cmulc(D, fx_ldg(P.tw_xr + kk));  // F = i conj(W) D
+      const i2 zk{E.x - WD.y, E.y + WD.x};
+      fx_bits(acc, zk);
+      zb[kk] = zk;
+      if (kk != 0 && kk != M / 2) {
+        const i2 zm{E.x + WD.y, WD.x - E.y};
+        fx_bits(acc, zm);
+        zb[M - kk] = zm;
+      }
+    }
+    se[t] = fx_publish<X::B1>(eb, acc);
   }
   __syncthreads();
-  // Inverse step A: k2 = t + T q, R1-point inverse DFT over k1, twiddle.
+  // Inverse step A: k2 = t + T q, R1-point inverse DFT over k1, twiddle.  Z[p] with p = t mod T was
+  // written by thread t (p <= M/2) or thread -t mod T, each at its own exponent.
   {
-    double2 x[KQ][R1];
+    const FxExp ea = se[t], em = se[(T - t) % T];
+    const int ec = max(ea.p, em.p);
+    i2 x[KQ][R1];
 #pragma unroll
     for (int q = 0; q < KQ; ++q)
 #pragma unroll
-      for (int k1 = 0; k1 < R1; ++k1) x[q][k1] = zb[t + T * q + R2 * k1];
+      for (int k1 = 0; k1 < R1; ++k1) {
+        const int p = t + T * q + R2 * k1;
+        x[q][k1] = fx_align(zb[p], p <= M / 2 ? ea.eb : em.eb, ec);
+      }
     __syncthreads();
+    unsigned acc = 0;
 #pragma unroll
     for (int q = 0; q < KQ; ++q) {
       const int k2 = t + T * q;
-      dft<R1, 1>(x[q], c);
+      dft<R1, 1>(x[q]);
+      fx_bits(acc, x[q][0]);
       sb[X::sidx(0, k2)] = x[q][0];
 #pragma unroll
-      for (int a = 1; a < R1; ++a) sb[X::sidx(a, k2)] = cmulc(c, x[q][a], __ldg(P.tw_x + ((a * k2) % M)));
+      for (int a = 1; a < R1; ++a) {
+        const i2 y = fx_cmulc(x[q][a], fx_ldg(P.tw_x + ((a * k2) % M)));
+        fx_bits(acc, y);
+        sb[X::sidx(a, k2)] = y;
+      }
     }
+    se[T + t] = fx_publish<X::B2>(ec, acc);
   }
   __syncthreads();
   // Inverse step B: alpha = t, R2-point inverse DFT over k2, z[alpha + R1 beta].
   {
-    double2 x[R2];
+    int eb[T], ec = -kFxNonfinite;
 #pragma unroll
-    for (int k2 = 0; k2 < R2; ++k2) x[k2] = sb[X::sidx(t, k2)];
-    dft<R2, 1>(x, c);
+    for (int q = 0; q < T; ++q) {
+      const FxExp e = se[T + q];
+      eb[q] = e.eb;
+      ec = max(ec, e.p);
+    }
+    i2 x[R2];
+#pragma unroll
+    for (int k2 = 0; k2 < R2; ++k2) x[k2] = fx_align(sb[X::sidx(t, k2)], eb[k2 % T], ec);
+    dft<R2, 1>(x);
     if (valid) {
+      const FxOut fo = fx_out(ec);
       double* o = dp + L.at(0, j, k);
 #pragma unroll
       for (int b = 0; b < R2; ++b) {
         const int m = t + R1 * b;
+        const double2 r = fx_to(x[b], fo, c);
         if (ALIGNED) {
-          *reinterpret_cast<double2*>(o + 2 * m + 1) = x[b];
+          *reinterpret_cast<double2*>(o + 2 * m + 1) = r;
         } else {
-          o[2 * m + 1] = x[b].x;
-          o[2 * m + 2] = x[b].y;
+          o[2 * m + 1] = r.x;
+          o[2 * m + 2] = r.y;
         }
       }
+      if (fo.odd)
+#pragma unroll 1
+        for (int b = 0; b < R2; ++b) {
+          double2 r = make_double2(o[2 * (t + R1 * b) + 1], o[2 * (t + R1 * b) + 2]);
+          fx_rescale(r, fo);
+          o[2 * (t + R1 * b) + 1] = r.x;
+          o[2 * (t + R1 * b) + 2] = r.y;
+        }
     }
   }
 }
 
 template <int M>
-size_t xp_smem() { return (size_t)XP<M>::LINES * XP<M>::LS * sizeof(double2); }
+size_t xp_smem() { return XP<M>::kSmem; }
 template <int N>
-size_t yz_smem() { return (size_t)N * lpc<N>() * sizeof(double2); }
+size_t yz_smem() { return YZ<N>::kSmem; }
 
 template <int N, bool FWD, int PB>
 cudaError_t launch_dct_y_n(const FftPlan& P, double2* spec, cudaStream_t st) {
@@ -461,8 +589,7 @@ __global__ void __launch_bounds__(256) dct_x_bc_kernel(FftPlan P, double* __rest
 template <int N, int PB>
 __global__ void __launch_bounds__(lpc<N>() * Split<N>::R1) dct_x_fwd_kernel(FftPlan P, double2* spec, FOne c) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  dct_x_fwd_body<N, PB, false>(P, nullptr, spec, reinterpret_cast<double2*>(smem_raw), blockIdx.x, threadIdx.x,
-                               threadIdx.y, c);
+  dct_x_fwd_body<N, PB>(P, spec, reinterpret_cast<double2*>(smem_raw), blockIdx.x, threadIdx.x, threadIdx.y, c);
 }
 
 template <int N, int PB>
@@ -476,7 +603,7 @@ template <int N, int PB>
 cudaError_t launch_dct_x_n(bool fwd, const FftPlan& P, const DivArgs* d, double2* spec, const double2* cspec,
                            double* dp, const Layout& L, cudaStream_t st, const Marker* mk) {
   constexpr int LPC = lpc<N>();
-  const size_t sm = yz_smem<N>() + (size_t)LPC * (N + 1) * sizeof(double2);
+  const size_t sm = dct_x_smem<N>();
   const int grid = (P.ny * P.nz + 2 * LPC - 1) / (2 * LPC);
   const FOne c{1.0, -0.0};
   cudaError_t e;

@@ -1,190 +1,16 @@
-// Register DFTs, the four-step line engine and the FFT-based (Makhoul)
-// DCT-II/III line bodies, shared by the session passes (ns_fft.cu) and the
-// batched spectral passes (ns_dct.cu).  Everything here is a template or an
-// inline device function with internal linkage in each translation unit.
+// The four-step line engine and the FFT-based (Makhoul) DCT-II/III line
+// bodies, shared by the session passes (ns_fft.cu) and the batched spectral
+// passes (ns_dct.cu).  Lines are doubles in memory; the transforms run on
+// block fixed-point integers (ns_fixed.cuh).  Everything here is a template
+// or an inline device function with internal linkage in each translation unit.
 #pragma once
 
+#include "ns_fixed.cuh"
 #include "ns_internal.cuh"
 #include "ns_kernels.cuh"
 
 namespace ns {
 namespace {
-
-// ---------------------------------------------------------------------------
-// Register DFTs
-// ---------------------------------------------------------------------------
-__host__ __device__ constexpr int ilog2c(int n) { return n <= 1 ? 0 : 1 + ilog2c(n >> 1); }
-__host__ __device__ constexpr int brevc(int i, int bits) {
-  return bits == 0 ? 0 : (((i & 1) << (bits - 1)) | brevc(i >> 1, bits - 1));
-}
-
-// Linzer-Feig constants of W32^q = exp(-2 pi i q / 32), q in [0,16):
-// mode 0: W = f (1 + i t);  mode 1: W = f (t + i).
-__device__ __forceinline__ void lf32(int q, double& f, double& t, int& mode) {
-  switch (q) {
-    case 1: f = 0.9807852804032304; t = -0.19891236737965798; mode = 0; break;
-    case 2: f = 0.9238795325112867; t = -0.4142135623730951; mode = 0; break;
-    case 3: f = 0.8314696123025452; t = -0.6681786379192989; mode = 0; break;
-    case 5: f = -0.8314696123025452; t = -0.668178637919299; mode = 1; break;
-    case 6: f = -0.9238795325112867; t = -0.41421356237309515; mode = 1; break;
-    case 7: f = -0.9807852804032304; t = -0.19891236737965806; mode = 1; break;
-    case 9: f = -0.9807852804032304; t = 0.19891236737965792; mode = 1; break;
-    case 10: f = -0.9238795325112867; t = 0.41421356237309503; mode = 1; break;
-    case 11: f = -0.8314696123025455; t = 0.6681786379192984; mode = 1; break;
-    case 13: f = -0.8314696123025453; t = 0.6681786379192988; mode = 0; break;
-    case 14: f = -0.9238795325112867; t = 0.4142135623730952; mode = 0; break;
-    case 15: f = -0.9807852804032304; t = 0.19891236737965837; mode = 0; break;
-    default: f = 1.0; t = 0.0; mode = 0; break;
-  }
-}
-
-constexpr double SQH = 0.70710678118654752440;  // sqrt(1/2)
-
-// DIT butterfly a' = a + W b, b' = a - W b with W = W32^q (DIR = -1) or its
-// conjugate (DIR = +1).
-template <int DIR>
-__device__ __forceinline__ void bfly(double2& a, double2& b, int q, const FOne& c) {
-  double2 y;
-  double f;
-  if (q == 0) {
-    const double2 a0 = a;
-    a.x = fadd(c, a0.x, b.x); a.y = fadd(c, a0.y, b.y);
-    b.x = fsub(c, a0.x, b.x); b.y = fsub(c, a0.y, b.y);
-    return;
-  }
-  if (q == 8) {  // W = -i (forward) / +i (inverse)
-    const double2 a0 = a, b0 = b;
-    if (DIR < 0) {
-      a.x = fadd(c, a0.x, b0.y); a.y = fsub(c, a0.y, b0.x);
-      b.x = fsub(c, a0.x, b0.y); b.y = fadd(c, a0.y, b0.x);
-    } else {
-      a.x = fsub(c, a0.x, b0.y); a.y = fadd(c, a0.y, b0.x);
-      b.x = fadd(c, a0.x, b0.y); b.y = fsub(c, a0.y, b0.x);
-    }
-    return;
-  }
-  if (q == 4) {  // W = sqrt(1/2)(1 -+ i)
-    if (DIR < 0) { y.x = fadd(c, b.x, b.y); y.y = fsub(c, b.y, b.x); }
-    else { y.x = fsub(c, b.x, b.y); y.y = fadd(c, b.y, b.x); }
-    f = SQH;
-  } else if (q == 12) {  // W = -sqrt(1/2)(1 +- i)
-    if (DIR < 0) { y.x = fsub(c, b.x, b.y); y.y = fadd(c, b.y, b.x); }
-    else { y.x = fadd(c, b.x, b.y); y.y = fsub(c, b.y, b.x); }
-    f = -SQH;
-  } else {
-    double t;
-    int mode;
-    lf32(q, f, t, mode);
-    if (DIR > 0) {  // conjugate root
-      if (mode == 0) t = -t;
-      else { f = -f; t = -t; }
-    }
-    if (mode == 0) { y.x = fma(-t, b.y, b.x); y.y = fma(t, b.x, b.y); }
-    else { y.x = fma(t, b.x, -b.y); y.y = fma(t, b.y, b.x); }
-  }
-  const double2 a0 = a;
-  a.x = fma(f, y.x, a0.x); a.y = fma(f, y.y, a0.y);
-  b.x = fma(-f, y.x, a0.x); b.y = fma(-f, y.y, a0.y);
-}
-
-// Radix-2 in-place R-point DFT (R a power of two, R <= 32), natural order in and out.
-// Every index is a template constant, so the array stays in registers.
-template <int R, int I>
-struct BitRev {
-  static __device__ __forceinline__ void run(double2 (&x)[R]) {
-    constexpr int J = brevc(I, ilog2c(R));
-    if constexpr (J > I) {
-      const double2 t = x[I];
-      x[I] = x[J];
-      x[J] = t;
-    }
-    BitRev<R, I + 1>::run(x);
-  }
-};
-template <int R>
-struct BitRev<R, R> {
-  static __device__ __forceinline__ void run(double2 (&)[R]) {}
-};
-template <int R, int LEN, int S, int K, int DIR>
-struct Bfly {  // butterfly K of group S of stage LEN, then the next one
-  static __device__ __forceinline__ void run(double2 (&x)[R], const FOne& c) {
-    bfly<DIR>(x[S + K], x[S + K + LEN / 2], K * (32 / LEN), c);
-    if constexpr (K + 1 < LEN / 2) Bfly<R, LEN, S, K + 1, DIR>::run(x, c);
-    else if constexpr (S + LEN < R) Bfly<R, LEN, S + LEN, 0, DIR>::run(x, c);
-  }
-};
-template <int R, int LEN, int DIR>
-struct Stage {
-  static __device__ __forceinline__ void run(double2 (&x)[R], const FOne& c) {
-    Bfly<R, LEN, 0, 0, DIR>::run(x, c);
-    if constexpr (LEN < R) Stage<R, 2 * LEN, DIR>::run(x, c);
-  }
-};
-template <int R, int DIR>
-__device__ __forceinline__ void dft_pow2(double2 (&x)[R], const FOne& c) {
-  BitRev<R, 0>::run(x);
-  Stage<R, 2, DIR>::run(x, c);
-}
-
-// 3-point DFT in FMA form: with s = a1 + a2, d = a1 - a2 and t = a0 - s/2,
-// X0 = a0 + s, X1 = t - i (sqrt(3)/2) d, X2 = t + i (sqrt(3)/2) d (forward;
-// the inverse takes the conjugate roots).
-template <int DIR>
-__device__ __forceinline__ void dft3(double2& a0, double2& a1, double2& a2, const FOne& c) {
-  constexpr double H3 = 0.86602540378443864676;  // sqrt(3)/2
-  const double2 s = make_double2(fadd(c, a1.x, a2.x), fadd(c, a1.y, a2.y));
-  const double2 d = make_double2(fsub(c, a1.x, a2.x), fsub(c, a1.y, a2.y));
-  const double2 t = make_double2(fma(s.x, -0.5, a0.x), fma(s.y, -0.5, a0.y));
-  a0 = make_double2(fadd(c, a0.x, s.x), fadd(c, a0.y, s.y));
-  const double g = DIR < 0 ? H3 : -H3;
-  a1 = make_double2(fma(g, d.y, t.x), fma(-g, d.x, t.y));
-  a2 = make_double2(fma(-g, d.y, t.x), fma(g, d.x, t.y));
-}
-
-// 12-point DFT by the prime-factor (Good-Thomas) split 12 = 3 x 4, which
-// needs no twiddles: 3-point DFTs over n1 of x[(4 n1 + 3 n2) mod 12] for each
-// n2, then 4-point DFTs over n2, whose output k2 of row k1 is
-// X[(4 k1 + 9 k2) mod 12] (9 = 3 x (3^-1 mod 4), 4 = 4 x (4^-1 mod 3)).
-template <int DIR>
-__device__ __forceinline__ void dft12(double2 (&x)[12], const FOne& c) {
-  double2 y[4][3];
-#pragma unroll
-  for (int n2 = 0; n2 < 4; ++n2) {
-    double2 a0 = x[(3 * n2) % 12], a1 = x[(4 + 3 * n2) % 12], a2 = x[(8 + 3 * n2) % 12];
-    dft3<DIR>(a0, a1, a2, c);
-    y[n2][0] = a0;
-    y[n2][1] = a1;
-    y[n2][2] = a2;
-  }
-#pragma unroll
-  for (int k1 = 0; k1 < 3; ++k1) {
-    double2 z[4] = {y[0][k1], y[1][k1], y[2][k1], y[3][k1]};
-    dft_pow2<4, DIR>(z, c);
-#pragma unroll
-    for (int k2 = 0; k2 < 4; ++k2) x[(4 * k1 + 9 * k2) % 12] = z[k2];
-  }
-}
-
-// In-place R-point DFT, natural order in and out: R a power of two up to 32,
-// or 12.
-template <int R, int DIR>
-__device__ __forceinline__ void dft(double2 (&x)[R], const FOne& c) {
-  if constexpr (R == 12) dft12<DIR>(x, c);
-  else dft_pow2<R, DIR>(x, c);
-}
-
-__device__ __forceinline__ double2 cmul(const FOne& c, double2 a, double2 w) {
-  double2 r;
-  r.x = fma(a.x, w.x, -fmul(c, a.y, w.y));
-  r.y = fma(a.x, w.y, fmul(c, a.y, w.x));
-  return r;
-}
-__device__ __forceinline__ double2 cmulc(const FOne& c, double2 a, double2 w) {  // a * conj(w)
-  double2 r;
-  r.x = fma(a.x, w.x, fmul(c, a.y, w.y));
-  r.y = fma(a.y, w.x, -fmul(c, a.x, w.y));
-  return r;
-}
 
 // Four-step split N = R1 * R2 (R1 <= R2), T = R1 threads per line.
 template <int N> struct Split;
@@ -201,7 +27,8 @@ template <> struct Split<512> { static constexpr int R1 = 16, R2 = 32; };
 // ---------------------------------------------------------------------------
 // Line engine: LPC lines per CTA (lanes over lines, coalesced when the lines
 // are neighbouring columns), T = R1 threads per line.
-// Shared buffer index for line l: (r * R2 + q) * LPC + l.
+// Shared buffer index for line l: (r * R2 + q) * LPC + l; the exponents of
+// thread t's block: t * LPC + l.
 // ---------------------------------------------------------------------------
 // Lines per CTA of the session kernels: 8 for the long lines (register-heavy
 // 16-point DFTs), else 16.
@@ -212,51 +39,91 @@ template <int N, int LPC_ = lpc<N>()>
 struct YZ {
   static constexpr int R1 = Split<N>::R1, R2 = Split<N>::R2, T = R1, KQ = R2 / T;
   static constexpr int LPC = LPC_;
+  static constexpr int B1 = 60 - log2up(R1), B2 = 60 - log2up(R2);
+  static constexpr size_t kSmem = (size_t)N * LPC * sizeof(i2) + (size_t)T * LPC * sizeof(FxExp);
   __device__ static __forceinline__ int sidx(int r, int q, int l) { return (r * R2 + q) * LPC + l; }
 
-  // Forward step A: thread n1 = t loads x[n1 + R1 n2], R2-point DFT, twiddle, to smem (n1, k2).
-  __device__ static __forceinline__ void fwdA(const double2* __restrict__ g, long long st, double2* sb,
-                                              const double2* __restrict__ tw, int l, int t, const FOne& c) {
-    double2 x[R2];
-#pragma unroll
-    for (int n2 = 0; n2 < R2; ++n2) x[n2] = g[(long long)(t + R1 * n2) * st];
-    dft<R2, -1>(x, c);
+  // Forward step A: thread n1 = t holds x[n1 + R1 n2], R2-point DFT, twiddle, to smem (n1, k2).
+  __device__ static __forceinline__ void fwdA(const double2 (&d)[R2], i2* sb, FxExp* se, const int4* __restrict__ tw,
+                                              int l, int t) {
+    i2 x[R2];
+    const int eb = fx_block2<B2>(d, x);
+    dft<R2, -1>(x);
+    unsigned acc = 0;
+    fx_bits(acc, x[0]);
     sb[sidx(t, 0, l)] = x[0];
 #pragma unroll
-    for (int k2 = 1; k2 < R2; ++k2) sb[sidx(t, k2, l)] = cmul(c, x[k2], __ldg(tw + ((t * k2) % N)));
-  }
-  // Forward step B: for k2 = t + T*q: R1-point DFT over n1 -> X[k2 + R2 k1] in xk[q][k1].
-  __device__ static __forceinline__ void fwdB(double2 (&xk)[KQ][R1], const double2* sb, int l, int t,
-                                              const FOne& c) {
-#pragma unroll
-    for (int q = 0; q < KQ; ++q) {
-      const int k2 = t + T * q;
-#pragma unroll
-      for (int n1 = 0; n1 < R1; ++n1) xk[q][n1] = sb[sidx(n1, k2, l)];
-      dft<R1, -1>(xk[q], c);
+    for (int k2 = 1; k2 < R2; ++k2) {
+      const i2 y = fx_cmul(x[k2], fx_ldg(tw + ((t * k2) % N)));
+      fx_bits(acc, y);
+      sb[sidx(t, k2, l)] = y;
     }
+    se[t * LPC + l] = fx_publish<B1>(eb, acc);
   }
-  // Inverse step A: from X[k2 + R2 k1] held in xk, R1-point inverse DFT, twiddle, to smem (k2, alpha).
-  __device__ static __forceinline__ void invA(double2 (&xk)[KQ][R1], double2* sb, const double2* __restrict__ tw,
-                                              int l, int t, const FOne& c) {
+  // Forward step B: for k2 = t + T*q: R1-point DFT over n1 -> X[k2 + R2 k1] in xk[q][k1]; returns
+  // the line's exponent.
+  __device__ static __forceinline__ int fwdB(i2 (&xk)[KQ][R1], const i2* sb, const FxExp* se, int l, int t) {
+    int eb[R1], ec = -kFxNonfinite;
+#pragma unroll
+    for (int n1 = 0; n1 < R1; ++n1) {
+      const FxExp e = se[n1 * LPC + l];
+      eb[n1] = e.eb;
+      ec = max(ec, e.p);
+    }
 #pragma unroll
     for (int q = 0; q < KQ; ++q) {
       const int k2 = t + T * q;
-      dft<R1, 1>(xk[q], c);
+#pragma unroll
+      for (int n1 = 0; n1 < R1; ++n1) xk[q][n1] = fx_align(sb[sidx(n1, k2, l)], eb[n1], ec);
+      dft<R1, -1>(xk[q]);
+    }
+    return ec;
+  }
+  // Inverse step A: from X[k2 + R2 k1] held in xk (exponent eb, B1 bits), R1-point inverse DFT,
+  // twiddle, to smem (k2, alpha).
+  __device__ static __forceinline__ void invA(i2 (&xk)[KQ][R1], int eb, i2* sb, FxExp* se,
+                                              const int4* __restrict__ tw, int l, int t) {
+    unsigned acc = 0;
+#pragma unroll
+    for (int q = 0; q < KQ; ++q) {
+      const int k2 = t + T * q;
+      dft<R1, 1>(xk[q]);
+      fx_bits(acc, xk[q][0]);
       sb[sidx(0, k2, l)] = xk[q][0];
 #pragma unroll
-      for (int a = 1; a < R1; ++a) sb[sidx(a, k2, l)] = cmulc(c, xk[q][a], __ldg(tw + ((a * k2) % N)));
+      for (int a = 1; a < R1; ++a) {
+        const i2 y = fx_cmulc(xk[q][a], fx_ldg(tw + ((a * k2) % N)));
+        fx_bits(acc, y);
+        sb[sidx(a, k2, l)] = y;
+      }
     }
+    se[t * LPC + l] = fx_publish<B2>(eb, acc);
   }
-  // Inverse step B: thread alpha = t, R2-point inverse DFT over k2, x[alpha + R1 beta] to global.
-  __device__ static __forceinline__ void invB(double2* __restrict__ g, long long st, const double2* sb, int l, int t,
-                                              const FOne& c) {
-    double2 x[R2];
+  // The thread's X[k2 + R2 k1] as a block for invA.
+  __device__ static __forceinline__ int block(const double2 (&d)[KQ][R1], i2 (&xk)[KQ][R1]) {
+    double2 f[R2];
+    i2 v[R2];
 #pragma unroll
-    for (int k2 = 0; k2 < R2; ++k2) x[k2] = sb[sidx(t, k2, l)];
-    dft<R2, 1>(x, c);
+    for (int i = 0; i < R2; ++i) f[i] = d[i / R1][i % R1];
+    const int eb = fx_block2<B1>(f, v);
 #pragma unroll
-    for (int b = 0; b < R2; ++b) g[(long long)(t + R1 * b) * st] = x[b];
+    for (int i = 0; i < R2; ++i) xk[i / R1][i % R1] = v[i];
+    return eb;
+  }
+  // Inverse step B: thread alpha = t, R2-point inverse DFT over k2: x[beta] is point alpha + R1 beta;
+  // returns the line's exponent.
+  __device__ static __forceinline__ int invB(i2 (&x)[R2], const i2* sb, const FxExp* se, int l, int t) {
+    int eb[T], ec = -kFxNonfinite;
+#pragma unroll
+    for (int q = 0; q < T; ++q) {
+      const FxExp e = se[q * LPC + l];
+      eb[q] = e.eb;
+      ec = max(ec, e.p);
+    }
+#pragma unroll
+    for (int k2 = 0; k2 < R2; ++k2) x[k2] = fx_align(sb[sidx(t, k2, l)], eb[k2 % T], ec);
+    dft<R2, 1>(x);
+    return ec;
   }
 };
 
@@ -271,55 +138,60 @@ struct YZ {
 // samples negated, modes reversed (k -> N-1-k).  The inverse is the exact
 // inverse (DCT-III with its 1/N): V_k = exp(i pi k / (2N)) (X_k - i X_{N-k}) / N
 // (X_N = 0), v = the unnormalised inverse DFT of V, x_{2m} = v_m,
-// x_{2m+1} = v_{N-1-m}.  About 2.8 log2(N) / 2 + 3 FP64 instructions per real
-// value against 3N/8 + 1.5 for the folded dense products.  Lines are numbered
+// x_{2m+1} = v_{N-1-m}.  The pre-twiddle table holds exp(i pi k / (2N)) 2^f / N
+// with f = floor(log2 N), the 2^-f goes into the block's exponent.  Lines are numbered
 // tl = col + nxs kz; block blk of a pass takes lines blk LPC .. blk LPC + LPC-1.
 template <int N, bool FWD, int PB, int LPC_ = lpc<N>()>
-__device__ __forceinline__ void dct_y_body(const FftPlan& P, double2* __restrict__ spec, double2* sb, int blk, int l,
+__device__ __forceinline__ void dct_y_body(const FftPlan& P, double2* __restrict__ spec, double2* smem, int blk, int l,
                                            int t, const FOne& c) {
   using F = YZ<N, LPC_>;
   constexpr int LPC = F::LPC, R1 = F::R1, R2 = F::R2, T = F::T, KQ = F::KQ;
+  i2* sb = reinterpret_cast<i2*>(smem);
+  FxExp* se = reinterpret_cast<FxExp*>(sb + N * LPC);
   const int tl = blk * LPC + l;
   const bool valid = tl < P.nxs * P.nz;
   const int col = valid ? tl % P.nxs : 0, o = valid ? tl / P.nxs : 0;
   const long long st = P.nxs;
   double2* g = spec + col + (long long)P.nxs * P.ny * o;
-  const double2* tw = P.dct_tw;
   auto src_of = [](int n) { return n < N / 2 ? 2 * n : 2 * (N - 1 - n) + 1; };  // the sample v_n holds
   auto mode_of = [](int k) { return PB == 2 ? N - 1 - k : k; };
   auto neg = [](double2 v) { return make_double2(-v.x, -v.y); };
   if (FWD) {
-    double2 x[R2];
+    double2 d[R2];
 #pragma unroll
     for (int n2 = 0; n2 < R2; ++n2) {
       const int s = src_of(t + R1 * n2);
       double2 v = valid ? g[(long long)s * st] : make_double2(0.0, 0.0);
       if (PB == 2 && (s & 1) == 0) v = neg(v);
-      x[n2] = v;
+      d[n2] = v;
     }
-    dft<R2, -1>(x, c);
-    sb[F::sidx(t, 0, l)] = x[0];
-#pragma unroll
-    for (int k2 = 1; k2 < R2; ++k2) sb[F::sidx(t, k2, l)] = cmul(c, x[k2], __ldg(tw + ((t * k2) % N)));
+    F::fwdA(d, sb, se, P.dct_tw, l, t);
     __syncthreads();
-    double2 xk[KQ][R1];
-    F::fwdB(xk, sb, l, t, c);  // xk[q][k1] = V[k2 + R2 k1], k2 = t + T q
+    i2 xk[KQ][R1];
+    const int ec = F::fwdB(xk, sb, se, l, t);  // xk[q][k1] = V[k2 + R2 k1], k2 = t + T q
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < KQ; ++q)
 #pragma unroll
       for (int k1 = 0; k1 < R1; ++k1) sb[(t + T * q + R2 * k1) * LPC + l] = xk[q][k1];
     __syncthreads();
-    if (valid)
+    const FxOut fo = fx_out(ec);
+    if (valid) {
       for (int k = t; k <= N / 2; k += R1) {
-        const double2 Uk = cmul(c, sb[k * LPC + l], __ldg(P.dct_wf + k));
-        const double2 Um = cmul(c, sb[((N - k) % N) * LPC + l], __ldg(P.dct_wf + (N - k)));
-        g[(long long)mode_of(k) * st] = make_double2(fsub(c, Uk.x, Um.y), fadd(c, Uk.y, Um.x));
+        const i2 Uk = fx_cmul(sb[k * LPC + l], fx_ldg(P.dct_wf + k));
+        const i2 Um = fx_cmul(sb[((N - k) % N) * LPC + l], fx_ldg(P.dct_wf + (N - k)));
+        g[(long long)mode_of(k) * st] = fx_to(i2{Uk.x - Um.y, Uk.y + Um.x}, fo, c);
         if (k != 0 && k != N / 2)
-          g[(long long)mode_of(N - k) * st] = make_double2(fsub(c, Um.x, Uk.y), fadd(c, Um.y, Uk.x));
+          g[(long long)mode_of(N - k) * st] = fx_to(i2{Um.x - Uk.y, Um.y + Uk.x}, fo, c);
       }
+      if (fo.odd)
+        for (int k = t; k <= N / 2; k += R1) {
+          fx_rescale(g[(long long)mode_of(k) * st], fo);
+          if (k != 0 && k != N / 2) fx_rescale(g[(long long)mode_of(N - k) * st], fo);
+        }
+    }
   } else {
-    double2 xk[KQ][R1];
+    double2 d[KQ][R1];
 #pragma unroll
     for (int q = 0; q < KQ; ++q)
 #pragma unroll
@@ -327,22 +199,28 @@ __device__ __forceinline__ void dct_y_body(const FftPlan& P, double2* __restrict
         const int k = t + T * q + R2 * k1;
         const double2 X = valid ? g[(long long)mode_of(k) * st] : make_double2(0.0, 0.0);
         const double2 Xm = (valid && k != 0) ? g[(long long)mode_of(N - k) * st] : make_double2(0.0, 0.0);
-        const double2 d = make_double2(fadd(c, X.x, Xm.y), fsub(c, X.y, Xm.x));  // X_k - i X_{N-k}
-        xk[q][k1] = cmul(c, d, __ldg(P.dct_wi + k));
+        d[q][k1] = make_double2(fadd(c, X.x, Xm.y), fsub(c, X.y, Xm.x));  // X_k - i X_{N-k}
       }
-    F::invA(xk, sb, tw, l, t, c);
-    __syncthreads();
-    double2 x[R2];
+    i2 xk[KQ][R1];
+    const int eb = F::block(d, xk) - ilog2c(N);
 #pragma unroll
-    for (int k2 = 0; k2 < R2; ++k2) x[k2] = sb[F::sidx(t, k2, l)];
-    dft<R2, 1>(x, c);
+    for (int q = 0; q < KQ; ++q)
+#pragma unroll
+      for (int k1 = 0; k1 < R1; ++k1) xk[q][k1] = fx_cmul(xk[q][k1], fx_ldg(P.dct_wi + (t + T * q + R2 * k1)));
+    F::invA(xk, eb, sb, se, P.dct_tw, l, t);
+    __syncthreads();
+    i2 x[R2];
+    const FxOut fo = fx_out(F::invB(x, sb, se, l, t));
 #pragma unroll
     for (int b = 0; b < R2; ++b) {
       const int s = src_of(t + R1 * b);
-      double2 v = x[b];
+      double2 v = fx_to(x[b], fo, c);
       if (PB == 2 && (s & 1) == 0) v = neg(v);
       if (valid) g[(long long)s * st] = v;
     }
+    if (fo.odd && valid)
+#pragma unroll 1
+      for (int b = 0; b < R2; ++b) fx_rescale(g[(long long)src_of(t + R1 * b) * st], fo);
   }
 }
 
@@ -353,80 +231,63 @@ __device__ __forceinline__ void dct_y_body(const FftPlan& P, double2* __restrict
 // sample or mode n (stride N+1 keeps the per-pair reads conflict-free), so
 // the global side moves whole rows with coalesced accesses.  A packed
 // spectrum row read as doubles is the modes in order.
-// Forward: the real rows (row = (j-1) + ny (k-1), block blk takes rows
-// 2 LPC blk ..) become their packed modes in spec.  DIV: the rows are the
-// divergence of d (plus the pressure-BC terms, or d->rhs as it is), computed
-// here with the two rows of a pair interleaved (element e: row 2 (e / 2N) +
-// e % 2, point (e / 2) % N); else the rows are read from spec, in place.
-template <int N, int PB, bool DIV, int LPC_ = lpc<N>()>
-__device__ __forceinline__ void dct_x_fwd_body(const FftPlan& P, const DivArgs* d, double2* spec, double2* sb, int blk,
-                                               int l, int t, const FOne& c) {
+// Forward, in place: the real rows in spec (block blk takes rows 2 LPC blk ..)
+// become their packed modes.
+template <int N, int LPC_ = lpc<N>()>
+constexpr size_t dct_x_smem() { return YZ<N, LPC_>::kSmem + (size_t)LPC_ * (N + 1) * sizeof(double2); }
+
+template <int N, int PB, int LPC_ = lpc<N>()>
+__device__ __forceinline__ void dct_x_fwd_body(const FftPlan& P, double2* spec, double2* smem, int blk, int l, int t,
+                                               const FOne& c) {
   using F = YZ<N, LPC_>;
   constexpr int LPC = F::LPC, R1 = F::R1, R2 = F::R2, T = F::T, KQ = F::KQ, PS = N + 1;
-  double2* pr = sb + N * LPC;
+  i2* sb = reinterpret_cast<i2*>(smem);
+  double2* pr = smem + N * LPC;
+  FxExp* se = reinterpret_cast<FxExp*>(pr + LPC * PS);
   double* prd = reinterpret_cast<double*>(pr);
   const int nrows = P.ny * P.nz;
   const int row0 = blk * 2 * LPC;
   const int tid = t * LPC + l, nth = LPC * R1;
   double* out = reinterpret_cast<double*>(spec);
-  if (DIV) {
-    const Layout L = d->L;
-    for (int e = tid; e < 2 * LPC * N; e += nth) {
-      const int pair = e / (2 * N), i = (e >> 1) % N, row = row0 + 2 * pair + (e & 1);
-      double v = 0.0;
-      if (row < nrows) {
-        const int j = 1 + row % P.ny, k = 1 + row / P.ny;
-        const long long g = L.at(i + 1, j, k);
-        if (d->rhs) {
-          v = d->rhs[g];
-        } else {
-          v = fmul(c, fsub(c, d->us[g + 1], d->us[g]), d->cdx);
-          v = fma(fsub(c, d->vs[g + L.sy], d->vs[g]), d->cdy, v);
-          v = fma(fsub(c, d->ws[g + L.sz], d->ws[g]), d->cdz, v);
-          v = v + P.bc_term(i + 1, j, k);
-        }
-      }
-      prd[2 * PS * pair + 2 * i + (e & 1)] = v;
-    }
-  } else {
-    for (int e = tid; e < 2 * LPC * N; e += nth) {
-      const int rr = e / N, i = e % N, row = row0 + rr;
-      prd[2 * PS * (rr >> 1) + 2 * i + (rr & 1)] = row < nrows ? out[(long long)N * row + i] : 0.0;
-    }
+  for (int e = tid; e < 2 * LPC * N; e += nth) {
+    const int rr = e / N, i = e % N, row = row0 + rr;
+    prd[2 * PS * (rr >> 1) + 2 * i + (rr & 1)] = row < nrows ? out[(long long)N * row + i] : 0.0;
   }
   __syncthreads();
   auto src_of = [](int n) { return n < N / 2 ? 2 * n : 2 * (N - 1 - n) + 1; };
   auto mode_of = [](int k) { return PB == 2 ? N - 1 - k : k; };
-  const double2* tw = P.dctx_tw;
   {
-    double2 x[R2];
+    double2 d[R2];
 #pragma unroll
     for (int n2 = 0; n2 < R2; ++n2) {
       const int s = src_of(t + R1 * n2);
       double2 v = pr[l * PS + s];
       if (PB == 2 && (s & 1) == 0) v = make_double2(-v.x, -v.y);
-      x[n2] = v;
+      d[n2] = v;
     }
-    dft<R2, -1>(x, c);
-    sb[F::sidx(t, 0, l)] = x[0];
-#pragma unroll
-    for (int k2 = 1; k2 < R2; ++k2) sb[F::sidx(t, k2, l)] = cmul(c, x[k2], __ldg(tw + ((t * k2) % N)));
+    F::fwdA(d, sb, se, P.dctx_tw, l, t);
   }
   __syncthreads();
-  double2 xk[KQ][R1];
-  F::fwdB(xk, sb, l, t, c);
+  i2 xk[KQ][R1];
+  const int ec = F::fwdB(xk, sb, se, l, t);
   __syncthreads();
 #pragma unroll
   for (int q = 0; q < KQ; ++q)
 #pragma unroll
     for (int k1 = 0; k1 < R1; ++k1) sb[(t + T * q + R2 * k1) * LPC + l] = xk[q][k1];
   __syncthreads();
+  const FxOut fo = fx_out(ec);
   for (int k = t; k <= N / 2; k += R1) {
-    const double2 Uk = cmul(c, sb[k * LPC + l], __ldg(P.dctx_wf + k));
-    const double2 Um = cmul(c, sb[((N - k) % N) * LPC + l], __ldg(P.dctx_wf + (N - k)));
-    pr[l * PS + mode_of(k)] = make_double2(fsub(c, Uk.x, Um.y), fadd(c, Uk.y, Um.x));
-    if (k != 0 && k != N / 2) pr[l * PS + mode_of(N - k)] = make_double2(fsub(c, Um.x, Uk.y), fadd(c, Um.y, Uk.x));
+    const i2 Uk = fx_cmul(sb[k * LPC + l], fx_ldg(P.dctx_wf + k));
+    const i2 Um = fx_cmul(sb[((N - k) % N) * LPC + l], fx_ldg(P.dctx_wf + (N - k)));
+    pr[l * PS + mode_of(k)] = fx_to(i2{Uk.x - Um.y, Uk.y + Um.x}, fo, c);
+    if (k != 0 && k != N / 2) pr[l * PS + mode_of(N - k)] = fx_to(i2{Um.x - Uk.y, Um.y + Uk.x}, fo, c);
   }
+  if (fo.odd)
+    for (int k = t; k <= N / 2; k += R1) {
+      fx_rescale(pr[l * PS + mode_of(k)], fo);
+      if (k != 0 && k != N / 2) fx_rescale(pr[l * PS + mode_of(N - k)], fo);
+    }
   __syncthreads();
   for (int e = tid; e < 2 * LPC * N; e += nth) {
     const int rr = e / N, i = e % N, row = row0 + rr;
@@ -437,10 +298,12 @@ __device__ __forceinline__ void dct_x_fwd_body(const FftPlan& P, const DivArgs* 
 // Inverse: packed modes of the rows of block blk -> dp slots 1..nx.
 template <int N, int PB, int LPC_ = lpc<N>()>
 __device__ __forceinline__ void dct_x_inv_body(const FftPlan& P, const double2* __restrict__ spec, double* dp,
-                                               const Layout& L, double2* sb, int blk, int l, int t, const FOne& c) {
+                                               const Layout& L, double2* smem, int blk, int l, int t, const FOne& c) {
   using F = YZ<N, LPC_>;
   constexpr int LPC = F::LPC, R1 = F::R1, R2 = F::R2, T = F::T, KQ = F::KQ, PS = N + 1;
-  double2* pr = sb + N * LPC;
+  i2* sb = reinterpret_cast<i2*>(smem);
+  double2* pr = smem + N * LPC;
+  FxExp* se = reinterpret_cast<FxExp*>(pr + LPC * PS);
   double* prd = reinterpret_cast<double*>(pr);
   const int nrows = P.ny * P.nz;
   const int row0 = blk * 2 * LPC;
@@ -453,31 +316,39 @@ __device__ __forceinline__ void dct_x_inv_body(const FftPlan& P, const double2* 
   __syncthreads();
   auto src_of = [](int n) { return n < N / 2 ? 2 * n : 2 * (N - 1 - n) + 1; };
   auto mode_of = [](int k) { return PB == 2 ? N - 1 - k : k; };
-  double2 xk[KQ][R1];
+  {
+    double2 d[KQ][R1];
 #pragma unroll
-  for (int q = 0; q < KQ; ++q)
+    for (int q = 0; q < KQ; ++q)
 #pragma unroll
-    for (int k1 = 0; k1 < R1; ++k1) {
-      const int k = t + T * q + R2 * k1;
-      const double2 X = pr[l * PS + mode_of(k)];
-      const double2 Xm = k ? pr[l * PS + mode_of(N - k)] : make_double2(0.0, 0.0);
-      const double2 dd = make_double2(fadd(c, X.x, Xm.y), fsub(c, X.y, Xm.x));  // X_k - i X_{N-k}
-      xk[q][k1] = cmul(c, dd, __ldg(P.dctx_wi + k));
-    }
-  F::invA(xk, sb, P.dctx_tw, l, t, c);
+      for (int k1 = 0; k1 < R1; ++k1) {
+        const int k = t + T * q + R2 * k1;
+        const double2 X = pr[l * PS + mode_of(k)];
+        const double2 Xm = k ? pr[l * PS + mode_of(N - k)] : make_double2(0.0, 0.0);
+        d[q][k1] = make_double2(fadd(c, X.x, Xm.y), fsub(c, X.y, Xm.x));  // X_k - i X_{N-k}
+      }
+    i2 xk[KQ][R1];
+    const int eb = F::block(d, xk) - ilog2c(N);
+#pragma unroll
+    for (int q = 0; q < KQ; ++q)
+#pragma unroll
+      for (int k1 = 0; k1 < R1; ++k1) xk[q][k1] = fx_cmul(xk[q][k1], fx_ldg(P.dctx_wi + (t + T * q + R2 * k1)));
+    F::invA(xk, eb, sb, se, P.dctx_tw, l, t);
+  }
   __syncthreads();
   {
-    double2 x[R2];
-#pragma unroll
-    for (int k2 = 0; k2 < R2; ++k2) x[k2] = sb[F::sidx(t, k2, l)];
-    dft<R2, 1>(x, c);
+    i2 x[R2];
+    const FxOut fo = fx_out(F::invB(x, sb, se, l, t));
 #pragma unroll
     for (int b = 0; b < R2; ++b) {
       const int s = src_of(t + R1 * b);
-      double2 v = x[b];
+      double2 v = fx_to(x[b], fo, c);
       if (PB == 2 && (s & 1) == 0) v = make_double2(-v.x, -v.y);
       pr[l * PS + s] = v;
     }
+    if (fo.odd)
+#pragma unroll 1
+      for (int b = 0; b < R2; ++b) fx_rescale(pr[l * PS + src_of(t + R1 * b)], fo);
   }
   __syncthreads();
   for (int e = tid; e < 2 * LPC * N; e += nth) {

@@ -1,6 +1,7 @@
 // Kernel argument blocks and launchers of the FP64 staggered step.
 #pragma once
 #include <cuda.h>
+#include <cmath>
 #include <vector>
 
 #include "ns_internal.cuh"
@@ -207,14 +208,20 @@ cudaError_t launch_adi_batch(int axis, const BatchAdiArgs* tab, const BatchItem*
 // ---------------------------------------------------------------------------
 // Periodic FFT Poisson (ns_fft.cu)
 // ---------------------------------------------------------------------------
+// A twiddle table entry: re and im (|.| <= 1) in units of 2^-60, each split at bit 30.
+inline int4 q60_entry(long double re, long double im) {
+  const long long r = llroundl(re * 0x1p60L), i = llroundl(im * 0x1p60L), low = (1ll << 30) - 1;
+  return make_int4((int)(r >> 30), (int)(r & low), (int)(i >> 30), (int)(i & low));
+}
 // Plan of the spectral pressure solve: per axis an FFT (periodic) or a dense
 // trigonometric transform pair (non-periodic, ns_dct.cu).
 struct FftPlan {
   int nx, ny, nz, nxh;
-  const double2* tw_x;   // twiddles for the nx/2-point complex FFT (x)
-  const double2* tw_xr;  // r2c split twiddles: exp(-2 pi i k / nx), k < nx/2
-  const double2* tw_y;
-  const double2* tw_z;
+  // Twiddle tables hold fixed-point entries (q60_entry): re and im in units of 2^-60, split at bit 30
+  const int4* tw_x;      // twiddles for the nx/2-point complex FFT (x)
+  const int4* tw_xr;  // r2c split twiddles: exp(-2 pi i k / nx), k < nx/2
+  const int4* tw_y;
+  const int4* tw_z;
   const double* inv_lam;  // scale/lambda per spectrum entry (FFT z solve), 0 at the mean mode
   int dp_unaligned;       // 1: dp slot pairs (2m+1, 2m+2) are not 16-byte aligned (scalar stores)
   int nxs;                // spectrum row length: nx/2+1 (periodic x) or nx/2 (packed wall x)
@@ -225,14 +232,14 @@ struct FftPlan {
   // A dense y axis of power-of-two length 32..512 with pbc 2 or 3 transformed through an FFT
   // (Makhoul) instead of the dense products (session plans; ns_fft.cu dct_y_kernel):
   int dct_y;              // 0: dense products; 2 or 3: the pressure code of the FFT-based transform
-  const double2* dct_tw;  // exp(-2 pi i m / ny), m < ny
-  const double2* dct_wf;  // exp(-i pi k / (2 ny)) / 2, k = 0..ny (forward post-twiddle)
-  const double2* dct_wi;  // exp(+i pi k / (2 ny)) / ny, k < ny (inverse pre-twiddle)
+  const int4* dct_tw;  // exp(-2 pi i m / ny), m < ny
+  const int4* dct_wf;  // exp(-i pi k / (2 ny)) / 2, k = 0..ny (forward post-twiddle)
+  const int4* dct_wi;  // exp(+i pi k / (2 ny)) 2^f / ny, f = floor(log2 ny), k < ny (inverse pre-twiddle)
   // The same for a wall x axis (packed modes; two x lines per complex FFT):
   int dct_x;
-  const double2* dctx_tw;  // exp(-2 pi i m / nx), m < nx
-  const double2* dctx_wf;  // exp(-i pi k / (2 nx)) / 2, k = 0..nx
-  const double2* dctx_wi;  // exp(+i pi k / (2 nx)) / nx, k < nx
+  const int4* dctx_tw;  // exp(-2 pi i m / nx), m < nx
+  const int4* dctx_wf;  // exp(-i pi k / (2 nx)) / 2, k = 0..nx
+  const int4* dctx_wi;  // exp(+i pi k / (2 nx)) 2^f / nx, f = floor(log2 nx), k < nx
   int has_mean;           // 1: the singular mode is set to mean_val (after the forward passes)
   double mean_val;        // FFT z solve: the singular entry; tridiagonal solve: the singular line's mean
   const double* mean_dev; // non-null: the line mean is mean_val * (*mean_dev) (a mean_dp set on the device)

@@ -51,7 +51,7 @@ double* g_scratch_addr[kMaxDevices] = {nullptr};
 
 // Twiddles W_N^m = exp(-2 pi i m/N) of the four transforms and the inverse
 // eigenvalues 1/(2 N lambda) (lambda as big_periodic_3D.f90:242-255; mean mode 0).
-__global__ void noalloc_tables(double2* tw, int M, int nx, int ny, int nz, double* inv_lam, double dx, double dy,
+__global__ void noalloc_tables(int4* tw, int M, int nx, int ny, int nz, double* inv_lam, double dx, double dy,
                                double dz) {
   const int nxh = M + 1;
   const int ntw = M + (M / 2 + 1) + ny + nz;
@@ -67,7 +67,8 @@ __global__ void noalloc_tables(double2* tw, int M, int nx, int ny, int nz, doubl
       else { m -= ny; N = nz; }
       double s, c;
       sincospi(2.0 * (double)m / (double)N, &s, &c);
-      tw[t] = make_double2(c, -s);
+      const long long re = __double2ll_rn(c * 0x1p60), im = __double2ll_rn(-s * 0x1p60), low = (1ll << 30) - 1;
+      tw[t] = make_int4((int)(re >> 30), (int)(re & low), (int)(im >> 30), (int)(im & low));  // as q60_entry
     } else {
       const long long q = t - ntw;
       const int i = (int)(q % nxh), j = (int)((q / nxh) % ny), k = (int)(q / ((long long)nxh * ny));
@@ -127,7 +128,7 @@ extern "C" int ns_poisson_fft_noalloc(const double* rhs_dev, double* dp_dev, int
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   double2* spec = reinterpret_cast<double2*>(base);  // 256-byte aligned
   double* inv_lam = base + n_spec;
-  double2* tw = reinterpret_cast<double2*>(base + n_spec + n_lam + ((n_spec + n_lam) & 1));
+  int4* tw = reinterpret_cast<int4*>(base + n_spec + n_lam + ((n_spec + n_lam) & 1));
   const double dx = lx / nx, dy = ly / ny, dz = lz / nz;
 
   noalloc_tables<<<152, 256, 0, st>>>(tw, M, nx, ny, nz, inv_lam, dx, dy, dz);

@@ -41,7 +41,7 @@ struct ns_handle {
   double* cyc_buf = nullptr;  // tables of the cyclic z solve (all-periodic boxes)
   double2* tri_tab = nullptr;  // the wall-axis line solve's twisted multipliers (one per spectrum entry)
   double* sing_cm = nullptr;   // its singular line's scratch
-  double2* tw = nullptr;  // twiddle tables (x, xr, y, z)
+  int4* tw = nullptr;  // twiddle tables (x, xr, y, z; fixed-point entries)
   ns::FftPlan plan{};
   // ADI factors
   double* adi_buf = nullptr;
