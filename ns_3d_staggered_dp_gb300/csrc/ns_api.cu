@@ -525,6 +525,7 @@ PredictArgs predict_args(ns_handle* h) {
   a.hx = h->hx; a.hy = h->hy; a.hz = h->hz;
   a.err = h->dev_err;
   set_predict_coeffs(a, c.bc, h->dx, h->dy, h->dz, c.dt, c.nu);
+  set_predict_fixed(a, c.scheme, h->pmax);
   return a;
 }
 
@@ -636,7 +637,7 @@ int enqueue_step(ns_handle* h, bool first, cudaEvent_t after_predict = nullptr) 
   const ns_config& c = h->cfg;
   PredictArgs a = predict_args(h);
   NS_CUDA(h, launch_predict(a, c.scheme, first, c.dp_flag != 0, 0, h->stream, &h->tma));
-  mark(h, "predict");
+  mark(h, "predict", 2);
   if (after_predict) NS_CUDA(h, cudaEventRecord(after_predict, h->stream));
   return enqueue_tail(h, false);
 }
@@ -1047,6 +1048,7 @@ void free_all(ns_handle* h) {
   for (cudaEvent_t e : h->ev_slab) cudaEventDestroy(e);
   for (cudaEvent_t e : h->trace_pool) cudaEventDestroy(e);
   if (h->tw) cudaFree(h->tw);
+  if (h->pmax) cudaFree(h->pmax);
   if (h->diag_bits) cudaFree(h->diag_bits);
   if (h->dev_err) cudaFree(h->dev_err);
   if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
@@ -1169,11 +1171,12 @@ int ns_create(const ns_config* cfg, ns_handle** out) {
       for (int f = 0; f < 4; ++f)
         for (int d = 0; d < 2; ++d) h->faces[set].ax[a].f[f][d] = h->face_buf + face_offset(h->L, set, a, f, d);
   if (cudaMalloc(&h->diag_bits, sizeof(unsigned long long)) != cudaSuccess) return bail(NS_ERR_NOMEM);
+  if (cudaMalloc(&h->pmax, 3 * (size_t)(h->L.nz + 2) * sizeof(unsigned)) != cudaSuccess) return bail(NS_ERR_NOMEM);
   if (cudaMalloc(&h->dev_err, sizeof(int)) != cudaSuccess) return bail(NS_ERR_NOMEM);
   if (cudaMemsetAsync(h->dev_err, 0, sizeof(int), h->stream) != cudaSuccess) return bail(NS_ERR_CUDA);
-  // The predictor stages its tiles with cp.async.  NS_PREDICT_TMA=1 in the
-  // environment selects the tensor-memory-access loader instead (the same
-  // bits; measured 3.3 ms against 2.1 ms per 256^3 launch, so not the default).
+  // The predictor prefetches its planes into registers.  NS_PREDICT_TMA=1 in
+  // the environment selects the tensor-memory-access loader instead (the same
+  // bits).
   // A requested loader that cannot be set up fails ns_create rather than
   // running the other one silently.
   const char* tma_env = std::getenv("NS_PREDICT_TMA");
@@ -1415,15 +1418,17 @@ int ns_step_host(ns_handle* h, const double* u, const double* v, const double* w
   for (int s = 0; s < nslab; ++s) {
     const int lo = fb[s], hi = fb[s + 1];
     NS_CUDA(h, cudaStreamWaitEvent(h->stream, h->ev_slab[ev_scat + s], 0));
-    // cell planes whose stencil and the two planes above it (read by the
-    // prefetch) have arrived; a quarter of the range per CTA, at most
-    // KC planes: short ranges at the top spread over as many CTAs as a
-    // full slab, so the compute left after the last copy is short.
-    const int e = hi >= nz + 2 ? nz + 1 : std::min(nz + 1, hi - 2);
+    // cell planes whose stencil has arrived (whole groups of the predictor's
+    // block exponents: the slabs end KC + 2 planes into the box and multiples
+    // of KC further); a quarter of the range per CTA, at most KC planes and a
+    // divisor of a group: short ranges at the top spread over as many CTAs as
+    // a full slab, so the compute left after the last copy is short.
+    const int e = hi >= nz + 2 ? nz + 1 : std::min(nz + 1, hi - 1);
     if (e > pred_done) {
-      const int kc = std::max(2, std::min(KC, (e - pred_done) / 4));
+      int kc = KC;
+      while (kc > 2 && kc > (e - pred_done) / 4) kc /= 2;
       NS_CUDA(h, launch_predict_planes(pa, c.scheme, first, c.dp_flag != 0, pred_done, e, kc, h->stream, &h->tma));
-      mark(h, "predict");
+      mark(h, "predict", 2);
       trace_mark(h, h->stream, "predict", s, lo, hi);
       pred_done = e;
       // the history of the finished planes is final: out on the copy stream

@@ -58,6 +58,26 @@ __device__ __forceinline__ long long fx_mul(long long a, FxW w) {
   const long long t = fx_wide(l, w.h, fx_wide(h, w.l, 1ll << 29));
   return fx_wide(h, w.h, t >> 30);
 }
+// (a b) >> 60 of two variables below 2^61, rounded (the mean of the dropped
+// product of the low parts included).
+__device__ __forceinline__ long long fx_mulv(long long a, long long b) {
+  const int ah = fx_hi(a), al = fx_lo(a), bh = fx_hi(b), bl = fx_lo(b);
+  const long long t = fx_wide(al, bh, fx_wide(ah, bl, (1ll << 29) + (1ll << 28)));
+  return fx_wide(ah, bh, t >> 30);
+}
+__device__ __forceinline__ long long fx_sqr(long long a) {
+  const int ah = fx_hi(a), al = fx_lo(a);
+  return fx_wide(ah, ah, fx_wide(ah, 2 * al, (1ll << 29) + (1ll << 28)) >> 30);
+}
+// a * w for |a| < 2^62 and |w| <= 1/2: the constant split at bit 29, its low part times 4.
+__host__ __device__ constexpr FxW fxw62(long long q60) {
+  return FxW{(int)(q60 >> 29), (int)((q60 & ((1ll << 29) - 1)) << 2)};
+}
+__device__ __forceinline__ long long fx_mul62(long long a, FxW w) {
+  const int h = (int)(a >> 31), l = (int)a & 0x7fffffff;
+  const long long t = fx_wide(l, w.h, fx_wide(h, w.l, 1ll << 30));
+  return fx_wide(h, w.h, t >> 31);
+}
 // a * w and a * conj(w), complex, |a| < 2^61.
 __device__ __forceinline__ i2 fx_cmul(i2 a, FxC w) {
   const int rh = fx_hi(a.x), rl = fx_lo(a.x), ih = fx_hi(a.y), il = fx_lo(a.y);
@@ -92,13 +112,13 @@ __device__ __forceinline__ int fx_max_exp(const double (&d)[N]) {
   for (int i = 0; i < N; ++i) m = max(m, (unsigned)__double2hiint(d[i]) << 1);
   return (int)(m >> 21);
 }
-// d as an integer of B bits for biased exponent E (>= d's own); truncated.
+// d as an integer of B bits for biased exponent E, truncated; 0 or -1 when d's own exponent is larger.
 template <int B>
 __device__ __forceinline__ long long fx_from(double d, int E) {
   const int hi = __double2hiint(d);
   const unsigned long long m = ((unsigned long long)(unsigned)((hi & 0xfffff) | 0x100000) << 32) |
                                (unsigned)__double2loint(d);
-  const int s = min(E - ((hi >> 20) & 0x7ff), 63);
+  const unsigned s = min((unsigned)(E - ((hi >> 20) & 0x7ff)), 63u);
   const long long v = (long long)((m << (B - 53)) >> s), sg = (long long)(hi >> 31);
   return (v ^ sg) - sg;
 }
@@ -194,6 +214,22 @@ __device__ __forceinline__ double2 fx_to(i2 v, const FxOut& o, const FOne& c) {
 __device__ __forceinline__ void fx_rescale(double2& r, const FxOut& o) {
   const double s = o.up ? 0x1p512 : 0x1p-512;
   r = make_double2(r.x * s, r.y * s);
+}
+
+// The same on the integer pipes, for kernels whose FP64 pipe is the busier
+// one: |v| < 2^63, rounded half up, 33 clocks (the leading bit comes from the
+// exponent of the 32-bit integer -> float conversion, which runs 4 times
+// faster than the leading-zero count).  The result must be a normal number.
+__device__ __forceinline__ double fx_to_int(long long v, int ec) {
+  const int sg = (int)(v >> 32) >> 31;
+  const long long sg64 = (long long)sg;
+  const unsigned long long m = (unsigned long long)((v ^ sg64) - sg64);
+  const unsigned mh = (unsigned)(m >> 32), ml = (unsigned)m;
+  const unsigned w = mh ? mh : ml;
+  const int up = (mh ? 157 : 189) - (__float_as_int(__uint2float_rz(w)) >> 23);  // leading bit to bit 62
+  const unsigned long long q = ((m << (up & 63)) + 0x200) >> 10;
+  const int hi = (int)(q >> 32) + ((ec + 1084 - up) << 20);  // the leading bit adds the missing 1
+  return __hiloint2double(w ? hi | (sg & (int)0x80000000) : 0, (int)q);
 }
 
 // ---------------------------------------------------------------------------

@@ -12,19 +12,31 @@
 // between conv_x, conv_y and conv_z (uy*vx serves both conv_x and conv_y).
 //
 // Tiling: a CTA owns 32 x-cells by TY y-rows and marches along z through a
-// chunk of KC planes.  Warp w (0..TY) is y-row j0-1+w; warp 0 only computes
+// chunk of planes.  Warp w (0..TY) is y-row j0-1+w; warp 0 only computes
 // products: those of the low y-halo row and, in one extra pass with lane r
 // on row r, the low x-halo position of every row.  Products are owned
 // one-sided (cell a owns SX[a], and the face products at faces a+1), so an
-// output cell needs products of its own and its lower neighbours only.  An
-// FP64 warp instruction costs its full issue slot however many lanes are
-// active, so no halo work is done by single lanes of the row warps.
-// Every FP64 operation is issued in FMA form (see ns_internal.cuh).
+// output cell needs products of its own and its lower neighbours only.
+//
+// The predictor itself (MODE 0) runs on block fixed-point integers
+// (predict_fx_planes); the convection and the diffusion alone (the routine
+// tier) and planes out of the fixed-point range run in FP64, every operation
+// in FMA form (see ns_internal.cuh).
+//
+// What bounds it: the FP64 stencils issue 62.7 FP64 instructions a cell, one
+// per 64 clocks and SM partition: 2.09 ms at 256^3, 83% of that pipe.  The
+// integer stencils take about 900 integer issue clocks a warp of cells beside
+// 10 FP64 instructions: 0.76 ms, plus 0.06 ms for the plane maxima; issue
+// slots 51% busy.  TY = 8 at three CTAs per SM (72 registers) leaves room to
+// hold the next plane's and the history's loads in flight; TY = 16 at two CTAs
+// (56 registers) waited for them at 1.9 ms.
 #include <algorithm>
+#include <cmath>
 
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
+#include "ns_fixed.cuh"
 #include "ns_internal.cuh"
 #include "ns_kernels.cuh"
 
@@ -33,8 +45,8 @@ namespace ns {
 namespace {
 
 constexpr int TX = 32;
-constexpr int TY = 16;
-constexpr int KC = 16;
+constexpr int TY = 8;
+constexpr int KC = 16;       // planes per CTA of the FP64 launches, at most of the others
 constexpr int SXW = TX + 8;  // smem row width: column c is x = i0-2+c; columns 1..34 (x in
                              // [i0-1, i0+32]) are read, 0..35 loaded (a 320-byte row)
 constexpr int SYH = TY + 2;  // smem rows: y in [j0-1, j0+TY]
@@ -46,8 +58,6 @@ constexpr int RING = 4;       // planes k-1, k, k+1 in use, k+2 in flight
 __device__ __forceinline__ int clampi(int a, int lo, int hi) { return a < lo ? lo : (a > hi ? hi : a); }
 
 struct PredSmem {
-  // u, v, w first: each ring slot (18 x 40 doubles, 5760 bytes) starts on a
-  // 128-byte boundary for the tile loader
   double u[RING][SYH][SXW];
   double v[RING][SYH][SXW];
   double w[RING][SYH][SXW];
@@ -57,11 +67,32 @@ struct PredSmem {
   double qxy[PYH][PXW];
   double qxz[2][PYH][PXW];
   double qyz[2][PYH][PXW];
-  unsigned long long bar[RING];  // tile loader: one mbarrier per ring slot
 };
-static_assert(sizeof(double) * SYH * SXW % 128 == 0, "ring slots of the tile loader stay 128-byte aligned");
 
-// ---- tile loader (TMA): one thread fills a ring slot with three 40 x 18 x 1
+// The fixed-point stencils' planes: the same ring and products as integers.
+constexpr int GRP = 16;      // cell planes of one block exponent
+constexpr int NWIN = 3;      // groups that a CTA's planes can touch
+struct FxPredSmem {
+  long long f[3][RING][SYH][SXW];
+  long long sx2[PYH][PXW];
+  long long sy2[PYH][PXW];
+  long long sz2[2][PYH][PXW];
+  long long qxy[PYH][PXW];
+  long long qxz[2][PYH][PXW];
+  long long qyz[2][PYH][PXW];
+};
+struct FxTail {  // behind the planes: the groups' exponents, and the tile loader's barriers
+  int e[NWIN][3];
+  int pad;
+  unsigned long long bar[2];
+};
+struct FxRaw {  // tile loader: two planes of doubles, each field's box on a 128-byte boundary
+  double f[2][3][SYH][SXW];
+};
+static_assert(sizeof(double) * SYH * SXW % 128 == 0, "boxes of the tile loader stay 128-byte aligned");
+static_assert(sizeof(FxPredSmem) == sizeof(PredSmem), "one shared-memory area serves both stencils");
+
+// ---- tile loader (TMA): one thread fills a staging slot with three 40 x 10 x 1
 // boxes (u, v, w) and arms the slot's mbarrier with their byte count ----
 constexpr unsigned kTileBytes = 3u * SYH * SXW * sizeof(double);
 constexpr int kWaitLimit = 1 << 20;                   // try_wait polls before a wait gives up
@@ -122,19 +153,19 @@ __global__ void wait_selftest_kernel(unsigned long long limit_ns, int* __restric
   if (!ok) asm volatile("mbarrier.complete_tx.shared::cta.b64 [%0], %1;" ::"r"(b), "r"(8u) : "memory");
   *gave_up = ok ? 0 : 1;
 }
-// Fill ring slot s with plane k (clamped into the box) of u, v, w: x from slot
+// Fill staging slot s with plane k (clamped into the box) of u, v, w: x from slot
 // i0-2 (tensor x = slot + 7: 8 (32 bx + 6) bytes, 16-byte aligned), y from
 // row j0-1.  Positions past the field read zeros or row padding; only inactive
 // positions use them.
-__device__ __forceinline__ void tma_plane(PredSmem& S, const CUtensorMap* mu, const CUtensorMap* mv,
+__device__ __forceinline__ void tma_plane(FxRaw& S, FxTail& T, const CUtensorMap* mu, const CUtensorMap* mv,
                                           const CUtensorMap* mw, int nz, int i0, int j0, int k, int s) {
   const int kk = clampi(k, 0, nz + 1);
   const int x = i0 - 2 + 7, y = j0 - 1;
-  const unsigned b = sm_addr(&S.bar[s]);
+  const unsigned b = sm_addr(&T.bar[s]);
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the slot's last readers are done (barrier)
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(kTileBytes) : "memory");
   const CUtensorMap* maps[3] = {mu, mv, mw};
-  double* dst[3] = {&S.u[s][0][0], &S.v[s][0][0], &S.w[s][0][0]};
+  double* dst[3] = {&S.f[s][0][0][0], &S.f[s][1][0][0], &S.f[s][2][0][0]};
 #pragma unroll
   for (int f = 0; f < 3; ++f)
     asm volatile(
@@ -212,57 +243,26 @@ __device__ __forceinline__ void products_zface(PredSmem& S, const FOne& c, int x
 
 // MODE: 0 predictor, 1 conv only (writes conv into us/vs/ws), 2 diffusion only.
 // One tile (bx, by) of TX x TY faces marching over the z-chunk bz.
-// TMA: planes arrive by the tile loader (maps mu, mv, mw of a.u, a.v, a.w)
-// instead of per-element cp.async.
-template <int SCHEME, bool FIRST, bool DPF, int MODE, bool TMA = false>
-__device__ __forceinline__ void predict_body(const PredictArgs& a, PredSmem& S, int bx, int by, int bz,
-                                             const CUtensorMap* mu = nullptr, const CUtensorMap* mv = nullptr,
-                                             const CUtensorMap* mw = nullptr) {
+template <int SCHEME, bool FIRST, bool DPF, int MODE>
+__device__ __forceinline__ void predict_body(const PredictArgs& a, PredSmem& S, int bx, int by, int k0, int k1) {
   const Layout L = a.L;
   const FOne c{a.one, a.mzero};
   const int lane = threadIdx.x;
   const int wy = threadIdx.y;  // 0..TY
   const int i0 = 1 + TX * bx;
   const int j0 = 1 + TY * by;
-  const int kc = a.kc > 0 ? a.kc : KC;
-  const int k0 = 1 + a.koff + kc * bz;
-  const int k1 = min(k0 + kc, a.kend > 0 ? a.kend : L.nz + 1);
   // smem coordinates of this thread's position: x = i0-1+lane+1 -> xa = lane+1; y = j0-1+wy -> yb = wy
   const int xa = lane + 1;
   const int yb = wy;
 
   // Warm-up: planes k0-1 and k0 (one copy group) and k0+1 (a second one);
   // products at z-face k0 once the first group has landed.
-  const bool producer = threadIdx.x == 0 && threadIdx.y == 0;
-  unsigned phase = 0;  // tile loader: bit s is the parity of slot s's next phase
-  bool ok = true;      // false once a wait gave up (recorded in a.err); every issued plane
-                       // is still waited for (bounded), so none is in flight at exit
-  auto wait_slot = [&](int sl) {
-    const bool r = mbar_wait(&S.bar[sl], (phase >> sl) & 1u);
-    ok = ok && r;
-    phase ^= 1u << sl;
-  };
-  if (TMA) {
-    if (producer) {
-      for (int sl = 0; sl < RING; ++sl) mbar_init(&S.bar[sl]);
-      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-    if (producer) {
-      tma_plane(S, mu, mv, mw, L.nz, i0, j0, k0 - 1, (k0 - 1) & 3);
-      tma_plane(S, mu, mv, mw, L.nz, i0, j0, k0, k0 & 3);
-      tma_plane(S, mu, mv, mw, L.nz, i0, j0, k0 + 1, (k0 + 1) & 3);
-    }
-    wait_slot((k0 - 1) & 3);
-    wait_slot(k0 & 3);
-  } else {
-    issue_plane(S, L, a.u, a.v, a.w, i0, j0, k0 - 1, (k0 - 1) & 3);
-    issue_plane(S, L, a.u, a.v, a.w, i0, j0, k0, k0 & 3);
-    cp_async_commit();
-    issue_plane(S, L, a.u, a.v, a.w, i0, j0, k0 + 1, (k0 + 1) & 3);
-    cp_async_commit();
-    cp_async_wait<1>();
-  }
+  issue_plane(S, L, a.u, a.v, a.w, i0, j0, k0 - 1, (k0 - 1) & 3);
+  issue_plane(S, L, a.u, a.v, a.w, i0, j0, k0, k0 & 3);
+  cp_async_commit();
+  issue_plane(S, L, a.u, a.v, a.w, i0, j0, k0 + 1, (k0 + 1) & 3);
+  cp_async_commit();
+  cp_async_wait<1>();
   __syncthreads();
   if (MODE != 2) {
     products_zface(S, c, xa, yb, (k0 - 1) & 3, k0 & 3, (k0 - 1) & 1);
@@ -277,39 +277,15 @@ __device__ __forceinline__ void predict_body(const PredictArgs& a, PredSmem& S, 
   const bool act_u = in_xy && (i >= a.ulo);
   const bool act_v = in_xy && (j >= a.vlo);
 
-  double hu = 0.0, hv = 0.0, hw = 0.0;  // tile loader: the AB2 history of this cell at plane k
-  if (TMA && MODE == 0 && SCHEME != 0 && !FIRST && in_xy && k0 < k1) {
-    const long long gh = L.at(i, j, k0);
-    hu = __ldg(a.hx + gh);
-    hv = __ldg(a.hy + gh);
-    hw = __ldg(a.hz + gh);
-  }
   for (int k = k0; k < k1; ++k) {
     const int s0 = k & 3, s1 = (k + 1) & 3, sm = (k + 3) & 3;  // planes k, k+1, k-1
     const int pb = k & 1, pbm = (k - 1) & 1;
-    // With the tile loader, this cell's AB2 history is read one plane
-    // ahead, so that its latency overlaps a whole iteration (each cell's
-    // history is read and then rewritten by its own thread only); read where
-    // it is used, it left the tile-loader kernel at 3.3 ms against 2.1.  The
-    // cp.async loader reads it at the combine (its copies already fill that time).
-    const double pu = hu, pv = hv, pw = hw;
-    if (TMA && MODE == 0 && SCHEME != 0 && !FIRST && in_xy && k + 1 < k1) {
-      const long long gh = L.at(i, j, k + 1);  // the next plane's, one iteration ahead
-      hu = __ldg(a.hx + gh);
-      hv = __ldg(a.hy + gh);
-      hw = __ldg(a.hz + gh);
-    }
     // plane k+1 has landed and every thread is done with plane k-2, whose
     // slot receives plane k+2 while this plane is computed
-    if (TMA) wait_slot((k + 1) & 3);
-    else cp_async_wait<0>();
+    cp_async_wait<0>();
     __syncthreads();
-    if (TMA) {
-      if (producer) tma_plane(S, mu, mv, mw, L.nz, i0, j0, k + 2, (k + 2) & 3);
-    } else {
-      issue_plane(S, L, a.u, a.v, a.w, i0, j0, k + 2, (k + 2) & 3);
-      cp_async_commit();
-    }
+    if (k + 2 <= k1) issue_plane(S, L, a.u, a.v, a.w, i0, j0, k + 2, (k + 2) & 3);
+    cp_async_commit();
     if (MODE != 2) {
       products(S, c, xa, yb, s0, s1, pb);
       if (wy == 0 && lane <= TY) products(S, c, 0, lane, s0, s1, pb);
@@ -339,7 +315,7 @@ __device__ __forceinline__ void predict_body(const PredictArgs& a, PredSmem& S, 
         } else if (MODE == 2) {
           out = fma(a.ix2, sWE, fma(a.iy2, sSN, fma(a.iz2, sBT, fmul(c, a.lap0, uc))));
         } else {
-          out = predictor_combine<SCHEME, FIRST>(a, c, uc, sWE, sSN, sBT, C, TMA ? pu : a.hx[g], a.hx, g);
+          out = predictor_combine<SCHEME, FIRST>(a, c, uc, sWE, sSN, sBT, C, a.hx[g], a.hx, g);
           if (DPF) out = fma(a.gpx, fsub(c, __ldg(a.p + g), __ldg(a.p + g - 1)), out);
         }
         a.us[g] = out;
@@ -365,7 +341,7 @@ __device__ __forceinline__ void predict_body(const PredictArgs& a, PredSmem& S, 
         } else if (MODE == 2) {
           out = fma(a.ix2, sWE, fma(a.iy2, sSN, fma(a.iz2, sBT, fmul(c, a.lap0, vc))));
         } else {
-          out = predictor_combine<SCHEME, FIRST>(a, c, vc, sWE, sSN, sBT, C, TMA ? pv : a.hy[g], a.hy, g);
+          out = predictor_combine<SCHEME, FIRST>(a, c, vc, sWE, sSN, sBT, C, a.hy[g], a.hy, g);
           if (DPF) out = fma(a.gpy, fsub(c, __ldg(a.p + g), __ldg(a.p + g - L.sy)), out);
         }
         a.vs[g] = out;
@@ -391,45 +367,345 @@ __device__ __forceinline__ void predict_body(const PredictArgs& a, PredSmem& S, 
         } else if (MODE == 2) {
           out = fma(a.ix2, sWE, fma(a.iy2, sSN, fma(a.iz2, sBT, fmul(c, a.lap0, wc))));
         } else {
-          out = predictor_combine<SCHEME, FIRST>(a, c, wc, sWE, sSN, sBT, C, TMA ? pw : a.hz[g], a.hz, g);
+          out = predictor_combine<SCHEME, FIRST>(a, c, wc, sWE, sSN, sBT, C, a.hz[g], a.hz, g);
           if (DPF) out = fma(a.gpz, fsub(c, __ldg(a.p + g), __ldg(a.p + g - L.sz)), out);
         }
         a.ws[g] = out;
       }
     }
   }
-  if (TMA) {
-    // the last plane issued (k1 + 1) is still in flight: drain it (bounded);
-    // a wait that gave up marks the step invalid
-    wait_slot((k1 + 1) & 3);
-    if (!ok && a.err) atomicExch(a.err, 1);
-  } else {
-    cp_async_wait<0>();  // nothing left in flight when the tile is done
+  cp_async_wait<0>();  // nothing left in flight when the tile is done
+}
+
+// ---------------------------------------------------------------------------
+// The predictor on block fixed-point integers (MODE 0)
+// ---------------------------------------------------------------------------
+// The cell planes 16 g + 1 .. 16 g + 16 form a group; the exponents of the
+// largest magnitudes of the planes their stencils read (16 g .. 16 g + 17),
+// one per field, are its block exponents.  They depend on the fields alone,
+// so the results do not depend on how the box is cut into launches, chunks
+// or tiles.  (Exponents of each plane's own three planes changed every few
+// planes of a turbulent field, and every change is a new warm-up: 3.0 ms at
+// 256^3.)  A velocity takes 59 bits, a two-point sum 60, a product 60 (its
+// unit is 2^-60 of four times the largest velocity squared, rounded).  Per
+// component the convection C and the viscous increment L are formed as
+// integers (the axis coefficients in units of 2^-60), brought back to
+// doubles, and combined with u itself and the AB2 history in FP64: u* is u
+// plus increments, as accurate for small u as for large.  A group that reads
+// an Inf, a NaN or a velocity beyond 2^250 takes the FP64 stencils; velocities
+// below 2^-250 count as fixed-point values of that exponent.
+constexpr int kFxB = 59;                    // bits of a velocity
+constexpr int kFxLo = 773, kFxHi = 1273;    // biased exponents of the fixed-point stencils
+struct FxPlane {
+  int e[3];  // biased block exponents of u, v, w
+};
+
+__device__ __forceinline__ void products_fx(FxPredSmem& S, int xa, int yb, int s0, int s1, int pb, bool zonly) {
+  const long long (*U0)[SXW] = S.f[0][s0], (*U1)[SXW] = S.f[0][s1];
+  const long long (*V0)[SXW] = S.f[1][s0], (*V1)[SXW] = S.f[1][s1];
+  const long long (*W0)[SXW] = S.f[2][s0], (*W1)[SXW] = S.f[2][s1];
+  const long long ue = U0[yb][xa + 2], vn = V0[yb + 1][xa + 1], wt = W1[yb][xa + 1];
+  S.sz2[pb][yb][xa] = fx_sqr(W0[yb][xa + 1] + wt);
+  S.qxz[pb][yb][xa] = fx_mulv(ue + U1[yb][xa + 2], wt + W1[yb][xa + 2]);
+  S.qyz[pb][yb][xa] = fx_mulv(vn + V1[yb + 1][xa + 1], wt + W1[yb + 1][xa + 1]);
+  if (zonly) return;
+  S.sx2[yb][xa] = fx_sqr(U0[yb][xa + 1] + ue);
+  S.sy2[yb][xa] = fx_sqr(V0[yb][xa + 1] + vn);
+  S.qxy[yb][xa] = fx_mulv(ue + U0[yb + 1][xa + 2], vn + V0[yb + 1][xa + 2]);
+}
+
+// The cell planes [k0, k1) of one tile, all with the block exponents P.
+template <int SCHEME, bool FIRST, bool DPF, bool ISO, bool TMA>
+__device__ __forceinline__ void predict_fx_planes(const PredictArgs& a, FxPredSmem& S, FxTail& T, FxRaw* raw,
+                                                  const FxPlane& P, int bx, int by, int k0, int k1, unsigned& phase,
+                                                  bool& ok, const CUtensorMap* mu, const CUtensorMap* mv,
+                                                  const CUtensorMap* mw) {
+  const Layout& L = a.L;
+  const FOne c{a.one, a.mzero};
+  const int lane = threadIdx.x, wy = threadIdx.y;
+  const int i0 = 1 + TX * bx, j0 = 1 + TY * by;
+  const int xa = lane + 1, yb = wy;
+  const int tid = lane + TX * wy;
+  const bool producer = tid == 0;
+  // this thread's two column pairs of a plane (of 3 x 10 x 18)
+  constexpr int NV = (TX + 4) / 2, NPAIR = 3 * NV * SYH, NTHR = TX * (TY + 1);
+  static_assert(NPAIR <= 2 * NTHR, "two pairs per thread cover a plane");
+  const double* src[2];
+  int dst[2], ee[2];
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const int e = min(tid + q * NTHR, NPAIR - 1);
+    const int f = e / (NV * SYH), yy = e / NV % SYH, xv = e % NV;
+    src[q] = (f == 0 ? a.u : f == 1 ? a.v : a.w) + L.at(i0 - 2 + 2 * xv, clampi(j0 - 1 + yy, 0, L.ny + 1), 0);
+    dst[q] = (f * RING * SYH + yy) * SXW + 2 * xv;
+    ee[q] = f == 0 ? P.e[0] : f == 1 ? P.e[1] : P.e[2];
   }
+  const bool two = tid + NTHR < NPAIR;
+  double2 r[2];
+  auto fetch = [&](int k) {  // plane k on its way: into registers, or (tile loader) into its staging slot
+    if (TMA) {
+      if (producer) tma_plane(*raw, T, mu, mv, mw, L.nz, i0, j0, k, k & 1);
+    } else {
+      const long long o = L.sz * (long long)clampi(k, 0, L.nz + 1);
+      r[0] = *reinterpret_cast<const double2*>(src[0] + o);
+      if (two) r[1] = *reinterpret_cast<const double2*>(src[1] + o);
+    }
+  };
+  auto convert = [&](int k) {  // and into the ring
+    if (TMA) {
+      ok = mbar_wait(&T.bar[k & 1], (phase >> (k & 1)) & 1u) && ok;
+      phase ^= 1u << (k & 1);
+    }
+    long long* ring = &S.f[0][k & 3][0][0];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      if (q == 1 && !two) break;
+      double2 d = r[q];
+      if (TMA) {
+        const int e = tid + q * NTHR;
+        d = *reinterpret_cast<const double2*>(&raw->f[k & 1][e / (NV * SYH)][e / NV % SYH][2 * (e % NV)]);
+      }
+      *reinterpret_cast<longlong2*>(ring + dst[q]) = make_longlong2(fx_from<kFxB>(d.x, ee[q]), fx_from<kFxB>(d.y, ee[q]));
+    }
+  };
+  // units: a velocity of field f is v 2^(e[f] - 1022 - kFxB), a product of fields f, g the product's
+  // 2^60 more.  The terms of C along the axes differ by the advecting field, so fields of about the
+  // same magnitude are summed as integers (at the largest one's unit); otherwise every term is
+  // brought back by itself, so that a small term keeps its digits where the large one vanishes
+  // (a shear layer u(y): du/dx = 0).
+  const int em = max(P.e[0], max(P.e[1], P.e[2]));
+  const bool apart = em - min(P.e[0], min(P.e[1], P.e[2])) > 1;
+  FxW qw[3], vw[3];
+  if (ISO) {
+    vw[0] = fxw62(a.v60[0]);
+  } else {
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      qw[q] = fxw(a.q60[q] >> (apart ? 0 : em - P.e[q]));
+      vw[q] = fxw(a.v60[q]);
+    }
+  }
+  const int kP = 60 - 2 * (1022 + kFxB), kL = a.kv + (ISO ? 1 : 0) - 1022 - kFxB;
+  // C of the differences of the products along x, y, z, and L of a component
+  auto conv = [&](long long dx, long long dy, long long dz, int e) -> double {
+    if (apart) {
+      double t = fmul(c, fx_to_int(dx, e + P.e[0] + kP), a.cx);
+      t = fma(fx_to_int(dy, e + P.e[1] + kP), a.cy, t);
+      return fma(fx_to_int(dz, e + P.e[2] + kP), a.cz, t);
+    }
+    if (ISO) {
+      auto at = [&](long long d, int n) { return n ? (d + 1) >> 1 : d; };
+      return fmul(c, fx_to_int(at(dx, em - P.e[0]) + at(dy, em - P.e[1]) + at(dz, em - P.e[2]), e + em + kP), a.cx);
+    }
+    return fx_to_int(fx_mul(dx, qw[0]) + fx_mul(dy, qw[1]) + fx_mul(dz, qw[2]), e + em + kP + a.kq);
+  };
+  auto visc = [&](long long uc, long long we, long long sn, long long bt, int e) -> double {
+    long long s;
+    if (ISO) s = fx_mul62((we + sn + bt - 6 * uc + 1) >> 1, vw[0]);
+    else s = fx_mul(we - 2 * uc, vw[0]) + fx_mul(sn - 2 * uc, vw[1]) + fx_mul(bt - 2 * uc, vw[2]);
+    return fx_to_int(s, e + kL);
+  };
+  auto combine = [&](double uc, double Lv, double C, double prev, double* __restrict__ hist, long long g) -> double {
+    if (SCHEME == 2) {  // AB2-CN explicit half (big_periodic_3D.f90:398-423)
+      double t = fma(FIRST ? a.dt : a.cC, C, fadd(c, uc, Lv));  // Euler start: nu/2 diff - conv (:400-408)
+      if (!FIRST) t = fma(a.cP, prev, t);
+      hist[g] = C;  // rhs_?_previous = -conv
+      return t;
+    }
+    const double rhs = fadd(c, Lv, C);  // nu*diff - conv
+    hist[g] = SCHEME == 0 ? 0.0 : rhs;
+    if (SCHEME == 1 && !FIRST) return fma(a.e1, rhs, fma(a.e2, prev, uc));  // AB2 (:369-396)
+    return fma(a.dt, rhs, uc);  // Euler, or the Euler start of AB2
+  };
+
+  // Warm-up: planes k0-1, k0, k0+1 in the ring, k0+2 on its way; products at z-face k0.
+  fetch(k0 - 1);
+  convert(k0 - 1);
+  fetch(k0);
+  convert(k0);
+  if (TMA) __syncthreads();  // both staging slots are read
+  fetch(k0 + 1);
+  convert(k0 + 1);
+  if (k0 + 2 <= k1) fetch(k0 + 2);
+  __syncthreads();
+  products_fx(S, xa, yb, (k0 - 1) & 3, k0 & 3, (k0 - 1) & 1, true);
+  // low x-halo position of every row, by warp 0 (one partially active pass)
+  if (wy == 0 && lane <= TY) products_fx(S, 0, lane, (k0 - 1) & 3, k0 & 3, (k0 - 1) & 1, true);
+
+  const int i = i0 + lane, j = j0 - 1 + wy;
+  const bool in_xy = (wy >= 1) && (i <= L.nx) && (j <= L.ny);
+  const bool act_u = in_xy && (i >= a.ulo), act_v = in_xy && (j >= a.vlo);
+  for (int k = k0; k < k1; ++k) {
+    const int s0 = k & 3, s1 = (k + 1) & 3, sm = (k + 3) & 3;  // planes k, k+1, k-1
+    const int pb = k & 1, pbm = (k - 1) & 1;
+    const long long g = L.at(i, j, k);
+    double uc = 0.0, vc = 0.0, wc = 0.0, hu = 0.0, hv = 0.0, hw = 0.0;  // this cell's, ahead of the products
+    if (in_xy) {
+      uc = __ldg(a.u + g);
+      vc = __ldg(a.v + g);
+      wc = __ldg(a.w + g);
+      if (SCHEME != 0 && !FIRST) {
+        hu = a.hx[g];
+        hv = a.hy[g];
+        hw = a.hz[g];
+      }
+    }
+    __syncthreads();  // plane k+1 is in the ring and every thread is done with plane k-2, whose slot takes plane k+2
+    if (TMA && k + 3 <= k1) fetch(k + 3);  // its staging slot held plane k+1
+    if (k + 2 <= k1) convert(k + 2);
+    if (!TMA && k + 3 <= k1) fetch(k + 3);
+    products_fx(S, xa, yb, s0, s1, pb, false);
+    if (wy == 0 && lane <= TY) products_fx(S, 0, lane, s0, s1, pb, false);
+    __syncthreads();
+    if (!in_xy) continue;
+    if (act_u) {  // x-component at x-face i
+      const long long (*F)[SXW] = S.f[0][s0];
+      const double C = conv(S.sx2[yb][xa] - S.sx2[yb][xa - 1], S.qxy[yb][xa - 1] - S.qxy[yb - 1][xa - 1],
+                            S.qxz[pb][yb][xa - 1] - S.qxz[pbm][yb][xa - 1], P.e[0]);
+      const double Lv = visc(F[yb][xa + 1], F[yb][xa] + F[yb][xa + 2], F[yb - 1][xa + 1] + F[yb + 1][xa + 1],
+                             S.f[0][sm][yb][xa + 1] + S.f[0][s1][yb][xa + 1], P.e[0]);
+      double out = combine(uc, Lv, C, hu, a.hx, g);
+      if (DPF) out = fma(a.gpx, fsub(c, __ldg(a.p + g), __ldg(a.p + g - 1)), out);
+      a.us[g] = out;
+    }
+    if (act_v) {  // y-component at y-face j
+      const long long (*F)[SXW] = S.f[1][s0];
+      const double C = conv(S.qxy[yb - 1][xa] - S.qxy[yb - 1][xa - 1], S.sy2[yb][xa] - S.sy2[yb - 1][xa],
+                            S.qyz[pb][yb - 1][xa] - S.qyz[pbm][yb - 1][xa], P.e[1]);
+      const double Lv = visc(F[yb][xa + 1], F[yb][xa] + F[yb][xa + 2], F[yb - 1][xa + 1] + F[yb + 1][xa + 1],
+                             S.f[1][sm][yb][xa + 1] + S.f[1][s1][yb][xa + 1], P.e[1]);
+      double out = combine(vc, Lv, C, hv, a.hy, g);
+      if (DPF) out = fma(a.gpy, fsub(c, __ldg(a.p + g), __ldg(a.p + g - L.sy)), out);
+      a.vs[g] = out;
+    }
+    if (k >= a.wlo) {  // z-component at z-face k
+      const long long (*F)[SXW] = S.f[2][s0];
+      const double C = conv(S.qxz[pbm][yb][xa] - S.qxz[pbm][yb][xa - 1], S.qyz[pbm][yb][xa] - S.qyz[pbm][yb - 1][xa],
+                            S.sz2[pb][yb][xa] - S.sz2[pbm][yb][xa], P.e[2]);
+      const double Lv = visc(F[yb][xa + 1], F[yb][xa] + F[yb][xa + 2], F[yb - 1][xa + 1] + F[yb + 1][xa + 1],
+                             S.f[2][sm][yb][xa + 1] + S.f[2][s1][yb][xa + 1], P.e[2]);
+      double out = combine(wc, Lv, C, hw, a.hz, g);
+      if (DPF) out = fma(a.gpz, fsub(c, __ldg(a.p + g), __ldg(a.p + g - L.sz)), out);
+      a.ws[g] = out;
+    }
+  }
+}
+
+// One tile (bx, by) over the cell planes [k0, k1), group by group.
+template <int SCHEME, bool FIRST, bool DPF, bool ISO, bool TMA>
+__device__ __forceinline__ void predict_fx_body(const PredictArgs& a, unsigned char* smem, int bx, int by, int k0,
+                                                int k1, const CUtensorMap* mu = nullptr,
+                                                const CUtensorMap* mv = nullptr, const CUtensorMap* mw = nullptr) {
+  FxRaw* raw = reinterpret_cast<FxRaw*>(smem);
+  FxPredSmem& S = *reinterpret_cast<FxPredSmem*>(smem + (TMA ? sizeof(FxRaw) : 0));
+  FxTail& T = *reinterpret_cast<FxTail*>(reinterpret_cast<unsigned char*>(&S) + sizeof(FxPredSmem));
+  const int tid = threadIdx.x + TX * threadIdx.y;
+  const int g0 = (k0 - 1) / GRP, ng = (k1 - 2) / GRP - g0 + 1;
+  if (a.pmax && (int)threadIdx.y < 3 * ng) {  // a warp per group and field
+    const int f = threadIdx.y % 3, gi = threadIdx.y / 3, lane = threadIdx.x;
+    const int k = GRP * (g0 + gi) + lane;
+    const unsigned m = lane < GRP + 2 && k <= a.L.nz + 1 ? __ldg(a.pmax + f * (a.L.nz + 2) + k) : 0u;
+    const unsigned r = __reduce_max_sync(0xffffffffu, m);
+    if (lane == 0) T.e[gi][f] = (int)(r >> 20);
+  }
+  unsigned phase = 0;  // tile loader: bit s is the parity of slot s's next phase
+  bool ok = true;      // false once a wait gave up (recorded in a.err); every issued plane
+                       // is still waited for (bounded), so none is in flight at exit
+  if (TMA) {
+    if (tid == 0) {
+      mbar_init(&T.bar[0]);
+      mbar_init(&T.bar[1]);
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+  }
+  __syncthreads();
+  for (int gi = 0; gi < ng; ++gi) {
+    const int ks = max(k0, GRP * (g0 + gi) + 1), ke = min(k1, GRP * (g0 + gi + 1) + 1);
+    FxPlane P;
+    bool bad = !a.pmax;  // coefficients outside the fixed-point range: FP64 stencils everywhere
+#pragma unroll
+    for (int f = 0; f < 3; ++f) {
+      P.e[f] = T.e[gi][f];
+      bad = bad || P.e[f] > kFxHi;
+      P.e[f] = max(P.e[f], kFxLo);
+    }
+    if (bad) predict_body<SCHEME, FIRST, DPF, 0>(a, reinterpret_cast<PredSmem&>(S), bx, by, ks, ke);
+    else predict_fx_planes<SCHEME, FIRST, DPF, ISO, TMA>(a, S, T, raw, P, bx, by, ks, ke, phase, ok, mu, mv, mw);
+    __syncthreads();
+  }
+  if (TMA && !ok && a.err) atomicExch(a.err, 1);
+}
+
+// The planes of chunk bz.
+__device__ __forceinline__ void chunk_planes(const PredictArgs& a, int bz, int& k0, int& k1) {
+  const int kc = a.kc > 0 ? a.kc : KC;
+  k0 = 1 + a.koff + kc * bz;
+  k1 = min(k0 + kc, a.kend > 0 ? a.kend : a.L.nz + 1);
 }
 
 template <int SCHEME, bool FIRST, bool DPF, int MODE>
 __global__ void __launch_bounds__(TX*(TY + 1)) predict_kernel(PredictArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  predict_body<SCHEME, FIRST, DPF, MODE>(a, *reinterpret_cast<PredSmem*>(smem_raw), blockIdx.x, blockIdx.y,
-                                         blockIdx.z);
+  int k0, k1;
+  chunk_planes(a, blockIdx.z, k0, k1);
+  predict_body<SCHEME, FIRST, DPF, MODE>(a, *reinterpret_cast<PredSmem*>(smem_raw), blockIdx.x, blockIdx.y, k0, k1);
+}
+
+template <int SCHEME, bool FIRST, bool DPF, bool ISO>
+__global__ void __launch_bounds__(TX*(TY + 1), 3) predict_fx_kernel(PredictArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  int k0, k1;
+  chunk_planes(a, blockIdx.z, k0, k1);
+  predict_fx_body<SCHEME, FIRST, DPF, ISO, false>(a, smem_raw, blockIdx.x, blockIdx.y, k0, k1);
 }
 
 // The same with the tile loader: the maps of a.u, a.v, a.w as kernel
-// parameters, the ring slots 128-byte aligned in dynamic shared memory.
-template <int SCHEME, bool FIRST, bool DPF>
+// parameters, the staging slots 128-byte aligned in dynamic shared memory.
+template <int SCHEME, bool FIRST, bool DPF, bool ISO>
 __global__ void __launch_bounds__(TX*(TY + 1)) predict_tma_kernel(PredictArgs a, const __grid_constant__ CUtensorMap mu,
                                                                   const __grid_constant__ CUtensorMap mv,
                                                                   const __grid_constant__ CUtensorMap mw) {
   extern __shared__ __align__(16) unsigned char smem_tma[];  // base rounded up to 128 B below
-  unsigned char* p = smem_tma + ((128u - (sm_addr(smem_tma) & 127u)) & 127u);
-  predict_body<SCHEME, FIRST, DPF, 0, true>(a, *reinterpret_cast<PredSmem*>(p), blockIdx.x, blockIdx.y, blockIdx.z,
-                                            &mu, &mv, &mw);
+  int k0, k1;
+  chunk_planes(a, blockIdx.z, k0, k1);
+  predict_fx_body<SCHEME, FIRST, DPF, ISO, true>(a, smem_tma + ((128u - (sm_addr(smem_tma) & 127u)) & 127u), blockIdx.x,
+                                                 blockIdx.y, k0, k1, &mu, &mv, &mw);
+}
+
+// Largest magnitude (high word) of each z plane of u, v, w: CTA (plane, field), a warp per row.
+constexpr int kMaxThreads = 512;
+__device__ __forceinline__ void plane_max_body(const PredictArgs& a, int k, int f) {
+  const Layout& L = a.L;
+  if (!a.pmax) return;
+  const double* p = (f == 0 ? a.u : f == 1 ? a.v : a.w) + L.at(0, 0, k);
+  const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+  unsigned m = 0;
+  for (int j = warp; j < L.ny + 2; j += kMaxThreads / 32) {
+    const double* row = p + L.sy * (long long)j;
+#pragma unroll 4
+    for (int i = lane; i < L.nx + 2; i += 32) m = max(m, (unsigned)__double2hiint(__ldg(row + i)) & 0x7fffffffu);
+  }
+  m = __reduce_max_sync(0xffffffffu, m);
+  __shared__ unsigned w[kMaxThreads / 32];
+  if (lane == 0) w[warp] = m;
+  __syncthreads();
+  if (warp == 0) {
+    m = __reduce_max_sync(0xffffffffu, lane < kMaxThreads / 32 ? w[lane] : 0u);
+    if (lane == 0) a.pmax[f * (L.nz + 2) + k] = m;
+  }
+}
+__global__ void __launch_bounds__(kMaxThreads) plane_max_kernel(PredictArgs a, int p0) {
+  plane_max_body(a, p0 + blockIdx.x, blockIdx.y);
+}
+__global__ void __launch_bounds__(kMaxThreads) plane_max_batch_kernel(const PredictArgs* __restrict__ tab,
+                                                                      const BatchItem* __restrict__ items) {
+  const BatchItem w = items[blockIdx.x];
+  plane_max_body(tab[w.sub], w.bx, blockIdx.y);
 }
 
 // Batched: persistent CTAs walk the work items (subdomain, tile) of a batch.
-template <int SCHEME, bool FIRST, bool DPF>
-__global__ void __launch_bounds__(TX*(TY + 1), 2) predict_batch_kernel(const PredictArgs* __restrict__ tab,
+template <int SCHEME, bool FIRST, bool DPF, bool ISO>
+__global__ void __launch_bounds__(TX*(TY + 1), 3) predict_batch_kernel(const PredictArgs* __restrict__ tab,
                                                                        const BatchItem* __restrict__ items,
                                                                        int n_items) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -438,45 +714,109 @@ __global__ void __launch_bounds__(TX*(TY + 1), 2) predict_batch_kernel(const Pre
     // the subdomain's arguments in registers: a reference into shared memory
     // would be reloaded after every barrier of the plane loop
     const PredictArgs a = tab[w.sub];
-    predict_body<SCHEME, FIRST, DPF, 0>(a, *reinterpret_cast<PredSmem*>(smem_raw), w.bx, w.by, w.bz);
+    int k0, k1;
+    chunk_planes(a, w.bz, k0, k1);
+    predict_fx_body<SCHEME, FIRST, DPF, ISO, false>(a, smem_raw, w.bx, w.by, k0, k1);
     __syncthreads();
   }
 }
 
-size_t predict_smem_bytes() { return sizeof(PredSmem); }
+constexpr size_t kFxSmem = sizeof(FxPredSmem) + sizeof(FxTail);
+size_t predict_smem_bytes() { return kFxSmem; }
 
 // The tile loader serves a launch whose u, v, w are the mapped fields.
 static bool tma_serves(const PredTma* t, const PredictArgs& a) {
   return t && t->ready && a.u == t->pu && a.v == t->pv && a.w == t->pw;
 }
 
-template <int SCHEME, bool FIRST, bool DPF, int MODE>
-static cudaError_t launch_grid(const PredictArgs& b, dim3 grid, cudaStream_t st, const PredTma* tma) {
-  const dim3 block(TX, TY + 1);
-  if constexpr (MODE == 0) {
-    if (tma_serves(tma, b)) {
-      auto kern = predict_tma_kernel<SCHEME, FIRST, DPF>;
-      const size_t sm = sizeof(PredSmem) + 128;
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-      if (e != cudaSuccess) return e;
-      kern<<<grid, block, sm, st>>>(b, tma->u, tma->v, tma->w);
-      return cudaGetLastError();
+void set_predict_fixed(PredictArgs& a, int scheme, unsigned* pmax) {
+  const double c[3] = {a.cx, a.cy, a.cz};
+  const double v[3] = {scheme == 2 ? a.ca : a.kx, scheme == 2 ? a.cb : a.ky, scheme == 2 ? a.cc : a.kz};
+  auto scale = [](const double (&x)[3], long long (&q)[3], int& k, int below) {  // largest in [2^-below-1, 2^-below)
+    const double m = std::max(std::fabs(x[0]), std::max(std::fabs(x[1]), std::fabs(x[2])));
+    k = 0;
+    for (int i = 0; i < 3; ++i) q[i] = 0;
+    if (!(m > 0.0)) return m == 0.0;
+    if (!std::isfinite(x[0]) || !std::isfinite(x[1]) || !std::isfinite(x[2])) return false;
+    k = std::ilogb(m) + 1 + below;
+    for (int i = 0; i < 3; ++i) q[i] = std::llrint(std::ldexp(x[i], 60 - k));
+    return std::abs(k) <= 200;
+  };
+  const bool okc = scale(c, a.q60, a.kq, 0), okv = scale(v, a.v60, a.kv, 1);
+  a.pmax = okc && okv ? pmax : nullptr;
+  a.iso = c[0] == c[1] && c[0] == c[2] && v[0] == v[1] && v[0] == v[2];
+}
+
+// Planes per CTA: a chunk's cost is its planes plus about two (its first
+// planes and the products of its first face), and two CTAs share an SM, so
+// the depth with the fewest waves x (depth + 2) is taken, of those that
+// divide a group.  At 256^3 that is 16 (4096 CTAs), at 64^3 4 (256 CTAs), at
+// 32^3 1 (128 CTAs).  With 16 planes a CTA at every size the 64^3 predictor
+// took 0.180 ms (now 0.035), the 32^3 one 0.165 (0.017).
+int predict_chunk(const std::vector<std::pair<long long, int>>& boxes) {
+  int dev = 0, nsm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return KC;
+  const long long slots = 3LL * std::max(1, nsm);
+  int best = KC;
+  long long cost = -1;
+  for (int kc = 1; kc <= GRP; kc *= 2) {
+    long long ctas = 0;
+    for (const auto& b : boxes) ctas += b.first * ((b.second + kc - 1) / kc);
+    const long long t = (ctas + slots - 1) / slots * (kc + 2);
+    if (cost < 0 || t <= cost) {
+      cost = t;
+      best = kc;
     }
   }
-  auto kern = predict_kernel<SCHEME, FIRST, DPF, MODE>;
-  const size_t sm = sizeof(PredSmem);
+  return best;
+}
+
+template <typename K, typename... A>
+static cudaError_t launch_smem(K kern, dim3 grid, size_t sm, cudaStream_t st, const A&... args) {
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
-  kern<<<grid, block, sm, st>>>(b);
+  kern<<<grid, dim3(TX, TY + 1), sm, st>>>(args...);
   return cudaGetLastError();
 }
 
-template <int SCHEME, bool FIRST, bool DPF, int MODE>
+// The largest magnitudes of the planes [p0, p1) that the launch reads, then the predictor.
+template <int SCHEME, bool FIRST, bool DPF>
+static cudaError_t launch_grid(const PredictArgs& b, dim3 grid, int p0, int p1, cudaStream_t st, const PredTma* tma) {
+  if (b.pmax) {
+    plane_max_kernel<<<dim3(p1 - p0, 3), kMaxThreads, 0, st>>>(b, p0);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  if (tma_serves(tma, b)) {
+    const size_t sm = kFxSmem + sizeof(FxRaw) + 128;
+    if (b.iso) return launch_smem(predict_tma_kernel<SCHEME, FIRST, DPF, true>, grid, sm, st, b, tma->u, tma->v, tma->w);
+    return launch_smem(predict_tma_kernel<SCHEME, FIRST, DPF, false>, grid, sm, st, b, tma->u, tma->v, tma->w);
+  }
+  if (b.iso) return launch_smem(predict_fx_kernel<SCHEME, FIRST, DPF, true>, grid, kFxSmem, st, b);
+  return launch_smem(predict_fx_kernel<SCHEME, FIRST, DPF, false>, grid, kFxSmem, st, b);
+}
+
+static dim3 tile_grid(const Layout& L, int planes, int kc) {
+  return dim3((L.nx + TX - 1) / TX, (L.ny + TY - 1) / TY, (planes + kc - 1) / kc);
+}
+
+template <int SCHEME, bool FIRST, bool DPF>
 static cudaError_t launch_t(const PredictArgs& a, cudaStream_t st, const PredTma* tma) {
   PredictArgs b = a;
+  const dim3 t = tile_grid(a.L, a.L.nz, 1);
+  b.kc = predict_chunk({{(long long)t.x * t.y, a.L.nz}});
+  b.koff = b.kend = 0;
+  return launch_grid<SCHEME, FIRST, DPF>(b, tile_grid(a.L, a.L.nz, b.kc), 0, a.L.nz + 2, st, tma);
+}
+
+// Convection (mode 1) or diffusion (mode 2) alone, in FP64.
+template <int MODE>
+static cudaError_t launch_mode(const PredictArgs& a, cudaStream_t st) {
+  PredictArgs b = a;
   b.kc = b.koff = b.kend = 0;
-  const dim3 grid((a.L.nx + TX - 1) / TX, (a.L.ny + TY - 1) / TY, (a.L.nz + KC - 1) / KC);
-  return launch_grid<SCHEME, FIRST, DPF, MODE>(b, grid, st, tma);
+  return launch_smem(predict_kernel<0, false, false, MODE>, tile_grid(a.L, a.L.nz, KC), sizeof(PredSmem), st, b);
 }
 
 int predict_chunk_planes() { return KC; }
@@ -492,13 +832,12 @@ static cudaError_t launch_planes_t(PredictArgs b, cudaStream_t st, int p0, int p
   b.kc = kc;
   b.koff = p0 - 1;
   b.kend = p1;
-  const dim3 grid((b.L.nx + TX - 1) / TX, (b.L.ny + TY - 1) / TY, (p1 - p0 + kc - 1) / kc);
-  return launch_grid<SCHEME, FIRST, DPF, 0>(b, grid, st, tma);
+  return launch_grid<SCHEME, FIRST, DPF>(b, tile_grid(b.L, p1 - p0, kc), p0 - 1, p1 + 1, st, tma);
 }
 
 cudaError_t launch_predict_planes(PredictArgs a, int scheme, bool first, bool dpf, int p0, int p1, int kc,
                                   cudaStream_t st, const PredTma* tma) {
-  if (p0 < 1 || p1 > a.L.nz + 1 || p0 > p1 || kc < 1) return cudaErrorInvalidValue;
+  if (p0 < 1 || p1 > a.L.nz + 1 || p0 > p1 || kc < 1 || kc > GRP * (NWIN - 1)) return cudaErrorInvalidValue;
   if (p0 == p1) return cudaSuccess;
 #define NS_PRED_PCASE(S, F, D) \
   if (scheme == S && first == F && dpf == D) return launch_planes_t<S, F, D>(a, st, p0, p1, kc, tma);
@@ -511,10 +850,10 @@ cudaError_t launch_predict_planes(PredictArgs a, int scheme, bool first, bool dp
 
 cudaError_t launch_predict(const PredictArgs& a, int scheme, bool first, bool dpf, int mode, cudaStream_t st,
                            const PredTma* tma) {
-  if (mode == 1) return launch_t<0, false, false, 1>(a, st, nullptr);
-  if (mode == 2) return launch_t<0, false, false, 2>(a, st, nullptr);
+  if (mode == 1) return launch_mode<1>(a, st);
+  if (mode == 2) return launch_mode<2>(a, st);
 #define NS_PRED_CASE(S, F, D) \
-  if (scheme == S && first == F && dpf == D) return launch_t<S, F, D, 0>(a, st, tma);
+  if (scheme == S && first == F && dpf == D) return launch_t<S, F, D>(a, st, tma);
   NS_PRED_CASE(0, false, false) NS_PRED_CASE(0, false, true) NS_PRED_CASE(0, true, false) NS_PRED_CASE(0, true, true)
   NS_PRED_CASE(1, false, false) NS_PRED_CASE(1, false, true) NS_PRED_CASE(1, true, false) NS_PRED_CASE(1, true, true)
   NS_PRED_CASE(2, false, false) NS_PRED_CASE(2, false, true) NS_PRED_CASE(2, true, false) NS_PRED_CASE(2, true, true)
@@ -549,35 +888,42 @@ bool make_pred_tma(PredTma& t, const Layout& L, const double* u, const double* v
   return true;
 }
 
-void predict_tiles(const Layout& L, int& gx, int& gy, int& gz) {
-  gx = (L.nx + TX - 1) / TX;
-  gy = (L.ny + TY - 1) / TY;
-  gz = (L.nz + KC - 1) / KC;
+void predict_tiles(const Layout& L, int kc, int& gx, int& gy, int& gz) {
+  const dim3 g = tile_grid(L, L.nz, kc);
+  gx = (int)g.x;
+  gy = (int)g.y;
+  gz = (int)g.z;
 }
 
-template <int SCHEME, bool FIRST, bool DPF>
+template <int SCHEME, bool FIRST, bool DPF, bool ISO>
 static cudaError_t launch_bt(const PredictArgs* tab, const BatchItem* items, int n_items, int grid, cudaStream_t st) {
-  auto kern = predict_batch_kernel<SCHEME, FIRST, DPF>;
-  const size_t sm = sizeof(PredSmem);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  auto kern = predict_batch_kernel<SCHEME, FIRST, DPF, ISO>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFxSmem);
   if (e != cudaSuccess) return e;
   if (grid <= 0) {
     int per_sm = 0, dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TX * (TY + 1), sm);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TX * (TY + 1), kFxSmem);
     grid = std::max(1, per_sm) * nsm;
   }
   grid = std::min(grid, n_items);
   if (grid <= 0) return cudaSuccess;
-  kern<<<grid, dim3(TX, TY + 1), sm, st>>>(tab, items, n_items);
+  kern<<<grid, dim3(TX, TY + 1), kFxSmem, st>>>(tab, items, n_items);
   return cudaGetLastError();
 }
 
-cudaError_t launch_predict_batch(const PredictArgs* tab, const BatchItem* items, int n_items, int scheme, bool first,
-                                 bool dpf, int grid, cudaStream_t st) {
-#define NS_PRED_CASE(S, F, D) \
-  if (scheme == S && first == F && dpf == D) return launch_bt<S, F, D>(tab, items, n_items, grid, st);
+cudaError_t launch_predict_batch(const PredictArgs* tab, const BatchItem* items, int n_items, const BatchItem* planes,
+                                 int n_planes, bool iso, int scheme, bool first, bool dpf, int grid, cudaStream_t st) {
+  if (n_planes > 0) {
+    plane_max_batch_kernel<<<dim3(n_planes, 3), kMaxThreads, 0, st>>>(tab, planes);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+#define NS_PRED_CASE(S, F, D)                                                         \
+  if (scheme == S && first == F && dpf == D)                                          \
+    return iso ? launch_bt<S, F, D, true>(tab, items, n_items, grid, st)              \
+               : launch_bt<S, F, D, false>(tab, items, n_items, grid, st);
   NS_PRED_CASE(0, false, false) NS_PRED_CASE(0, false, true) NS_PRED_CASE(0, true, false) NS_PRED_CASE(0, true, true)
   NS_PRED_CASE(1, false, false) NS_PRED_CASE(1, false, true) NS_PRED_CASE(1, true, false) NS_PRED_CASE(1, true, true)
   NS_PRED_CASE(2, false, false) NS_PRED_CASE(2, false, true) NS_PRED_CASE(2, true, false) NS_PRED_CASE(2, true, true)

@@ -68,3 +68,92 @@ def test_nonfinite_right_hand_side(pbc, bad):
     rhs = np.random.default_rng(3).standard_normal(n)
     rhs[7, 11, 5] = bad
     assert not np.isfinite(_solve(n, pbc, rhs)).any()
+
+
+# --- the predictor's fixed-point stencils -------------------------------------------------------
+def _layered(cfg, seed, mags=(1.0, 1.0, 1.0), zamp=0.0):
+    """Random state with one magnitude per component, changing along z by 10^zamp over the box (the
+    16-plane groups then have different exponents)."""
+    from tests.helpers import random_state
+
+    st = random_state(cfg, seed, history=True)
+    for f, h, m in (("u", "px", mags[0]), ("v", "py", mags[1]), ("w", "pz", mags[2])):
+        for name in (f, h):
+            a = getattr(st, name)
+            a *= m * 10.0 ** (zamp * np.cos(np.pi * np.arange(a.shape[2]) / cfg.nz))
+    O.vel_bc_staggered(st.u, st.v, st.w, O.Faces.zeros(cfg.nx, cfg.ny, cfg.nz), *cfg.bc)
+    return st
+
+
+def _gpu_step(cfg, st, stage=False):
+    from ns_3d_staggered_dp_gb300 import Session, make_config
+
+    with Session(make_config(cfg.nx, cfg.ny, cfg.nz, lx=cfg.lx, ly=cfg.ly, lz=cfg.lz, nu=cfg.nu, dt=cfg.dt,
+                             scheme=cfg.scheme, bc=cfg.bc, pbc=cfg.pbc, dp_flag=cfg.dp_flag)) as s:
+        s.set_state(st.u, st.v, st.w, st.p, (st.px, st.py, st.pz))
+        s.step(1)
+        return s.get_state()
+
+
+WALLS = dict(bc=(2, 2, 2), pbc=(3, 3, 3))
+STENCILS = [((16, 16, 16), {}), ((32, 16, 64), dict(lz=3.0)), ((64, 32, 32), {})]
+STENCILS += [((34, ny, nz), WALLS) for ny, nz in ((7, 15), (8, 16), (9, 17), (17, 33))]
+
+
+@pytest.mark.parametrize("n,kw", STENCILS)
+@pytest.mark.parametrize("scheme,dpf", [(O.EULER, 0), (O.AB2, 1), (O.AB2_CN, 0)])
+@pytest.mark.parametrize("mags,zamp", [((1, 1, 1), 0.0), ((1, 1e-3, 1e-6), 0.0), ((1e-5, 1, 0), 2.0)])
+def test_predictor_shapes_and_magnitudes(n, kw, scheme, dpf, mags, zamp):
+    """Tile and group edges, unequal axes, components of very different size; the step's tolerance."""
+    cfg = O.Config(*n, nu=0.01, dt=0.003, scheme=scheme, dp_flag=dpf, **kw)
+    st = _layered(cfg, sum(n), mags, zamp)
+    got, ref = _gpu_step(cfg, st), O.step(st.copy(), cfg)
+    for k, a in (("u", "u"), ("v", "v"), ("w", "w"), ("p", "p"), ("hx", "px"), ("hy", "py"), ("hz", "pz")):
+        assert rel_l2(got[k], getattr(ref, a)) < 1e-10, k
+
+
+@pytest.mark.parametrize("amp", [1e-150, 1e-60, 1e60, 1e100])
+def test_predictor_extreme_velocities(amp):
+    """Velocities outside the fixed-point range take the FP64 stencils (large) or vanish against none
+    (small); dt scaled so that the convection stays an increment."""
+    cfg = O.Config(32, 16, 32, nu=0.01 * amp, dt=0.003 / amp, scheme=O.AB2)
+    st = _layered(cfg, 5, (amp, amp, amp))
+    for h in (st.px, st.py, st.pz):
+        h *= amp  # a history of the size of u^2
+    got, ref = _gpu_step(cfg, st), O.step(st.copy(), cfg)
+    for k, a in (("u", "u"), ("v", "v"), ("w", "w")):
+        assert rel_l2(got[k] / amp, getattr(ref, a) / amp) < 1e-10, k
+
+
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+def test_predictor_nonfinite_velocity(bad):
+    """A non-finite velocity spoils exactly the history entries that the reference's stencils spoil."""
+    cfg = O.Config(32, 16, 64, nu=0.01, dt=0.003, scheme=O.AB2)
+    st = _layered(cfg, 6)
+    st.v[9, 7, 30] = bad
+    with np.errstate(invalid="ignore", over="ignore"):
+        got, ref = _gpu_step(cfg, st), O.step(st.copy(), cfg)
+    for k, a in (("hx", "px"), ("hy", "py"), ("hz", "pz")):
+        r = getattr(ref, a)
+        fin = np.isfinite(r)
+        assert np.array_equal(np.isfinite(got[k]), fin) and not fin.all(), k
+        assert rel_l2(got[k][fin], r[fin]) < 1e-12, k
+
+
+@pytest.mark.parametrize("n,kw", [((32, 16, 64), {}), ((34, 18, 49), WALLS)])
+@pytest.mark.parametrize("scheme", [O.AB2, O.AB2_CN])
+def test_slabs_of_different_exponents(n, kw, scheme):
+    """ns_step_host predicts in z-slabs: the same bits as the whole-box step, with exponents that
+    change from group to group."""
+    from ns_3d_staggered_dp_gb300 import Session, make_config
+
+    cfg = O.Config(*n, nu=0.01, dt=0.003, scheme=scheme, **kw)
+    st = _layered(cfg, 11, (1, 1e-2, 1), 3.0)
+    hist = (st.px, st.py, st.pz)
+    with Session(make_config(*n, nu=0.01, dt=0.003, scheme=scheme, **kw)) as s:
+        s.set_state(st.u, st.v, st.w, st.p, hist)
+        s.step(1)
+        dev = s.get_state()
+        host = s.step_host(st.u, st.v, st.w, st.p, hist)
+    for k in dev:
+        assert np.array_equal(dev[k], host[k]), k
