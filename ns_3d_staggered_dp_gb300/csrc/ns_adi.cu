@@ -430,11 +430,236 @@ cudaError_t launch_adi_batch(int axis, const BatchAdiArgs* tab, const BatchItem*
   return cudaGetLastError();
 }
 
+// ---------------------------------------------------------------------------
+// Chunked sweeps
+// ---------------------------------------------------------------------------
+// With a small viscous number every factor of the LU is small (nu dt / 2 h^2 =
+// 0.002: 0.002), so a row hears nothing, to the last bit, of rows `halo` (6 to
+// 16) away.  A thread solves CH unknowns of a line from CH + 2 halo right-hand
+// sides held in registers: one read and one write of the fields, no
+// intermediate in memory, and CH-fold parallelism along the line.  The
+// right-hand sides come scaled by the pivots (ChunkSys), one FMA each way:
+// 2.75 FP64 instructions an unknown at CH 32, halo 8, against 3 and 1.9 times
+// the traffic of the whole-line kernels.  At 256^3 (whole lines before, in
+// parentheses): x 0.36 ms (0.51), y 0.29 (0.38), z 0.29 (0.37), the FP64 pipe
+// at 61-78%; at 32^3 10 us a sweep (20).
+// Rows q of [T0, T1) take their factors from the tables, the others the converged ones.
+template <int R, int W, int T0, int T1>
+__device__ __forceinline__ void chunk_rows(double (&r)[R], const ChunkSys& S, int e0) {
+  const double* l = S.l + kAdiExt + e0;
+  const double* dm = S.dm + kAdiExt + e0;
+  const double* cu = S.cu + kAdiExt + e0;
+  const double nl = -S.lc, nc = -S.cc;
+#pragma unroll
+  for (int q = 1; q < R; ++q) r[q] = fma(q >= T0 && q < T1 ? -__ldg(l + q) : nl, r[q - 1], r[q]);
+  if (R - 1 >= T0 && R - 1 < T1) r[R - 1] *= __ldg(dm + R - 1);
+#pragma unroll
+  for (int q = R - 2; q >= W; --q)
+    r[q] = q >= T0 && q < T1 ? fma(-__ldg(cu + q), r[q + 1], r[q] * __ldg(dm + q)) : fma(nc, r[q + 1], r[q]);
+}
+// The factors differ from the converged ones on a few rows at a line's first
+// end and on its last row (and where a periodic line goes on with row 0).
+template <int CH, int W>
+__device__ __forceinline__ void chunk_solve(double (&r)[CH + 2 * W], const ChunkSys& S, int e0) {
+  constexpr int R = CH + 2 * W, LOW = 2 * W + 2, HIGH = W + CH - 2;
+  if (e0 >= S.c0 && e0 + R <= S.c1) chunk_rows<R, W, 0, 0>(r, S, e0);
+  else if (e0 + LOW >= S.c0 && e0 + R <= S.c1) chunk_rows<R, W, 0, LOW>(r, S, e0);
+  else if (e0 >= S.c0 && e0 + HIGH <= S.c1) chunk_rows<R, W, HIGH, R>(r, S, e0);
+  else chunk_rows<R, W, 0, R>(r, S, e0);
+}
+// First unknown that chunk c works out: the last chunk ends at the line's end
+// (and writes only the unknowns past the chunk before it).
+template <int CH>
+__device__ __forceinline__ int chunk_first(const ChunkSys& S, int s) { return min(s, max(S.m - CH, 0)); }
+// Unknown index e continued past an end: where its right-hand side is (within
+// [0, m)), or -1 past an end that does not wrap.
+__device__ __forceinline__ int chunk_row(const ChunkSys& S, int e) {
+  if (e < 0 ? !S.wrap_lo : e >= S.m && !S.wrap_hi) return -1;
+  while (e < 0) e += S.m;
+  while (e >= S.m) e -= S.m;
+  return e;
+}
+
+// y and z sweeps: a thread per (field, chunk, line), lanes over x.
+template <int AXIS, int CH, int W>
+__global__ void __launch_bounds__(128, CH + 2 * W <= 50 ? 4 : 3) adi_chunk_kernel(const __grid_constant__ AdiArgs a) {
+  constexpr int R = CH + 2 * W;
+  const Layout& L = a.L;
+  const int fld = blockIdx.z, s = blockIdx.y * CH;
+  const ChunkSys& S = a.ch[fld];
+  if (s >= S.m) return;
+  const int n1 = L.nx + 2;
+  const int zlo = (AXIS == 1 && a.z1 > 0) ? a.z0 : 0;
+  const int n2 = AXIS == 2 ? L.ny + 2 : ((AXIS == 1 && a.z1 > 0) ? a.z1 - a.z0 : L.nz + 2);
+  const int tl = blockIdx.x * 128 + threadIdx.x;
+  if (tl >= n1 * n2) return;
+  long long base, st;
+  line_of<AXIS>(L, tl % n1, zlo + tl / n1, base, st);
+  const double* __restrict__ src = a.src[fld] + base;
+  double* __restrict__ dst = a.dst[fld] + base;
+  const double* sl = src + S.lo * st;
+  const bool walls = !S.periodic;
+  const int f = chunk_first<CH>(S, s), e0 = f - W, skip = s - f;
+  double r[R];
+  int er = chunk_row(S, e0 < 0 && !S.wrap_lo ? 0 : e0);
+#pragma unroll
+  for (int q = 0; q < R; ++q) {
+    const int e = e0 + q;
+    const bool in = (e >= 0 || S.wrap_lo) && (e < S.m || S.wrap_hi);
+    r[q] = in ? sl[er * st] : 0.0;
+    if (in) er = er + 1 == S.m ? 0 : er + 1;
+  }
+  if (walls && (f == 0 || f + CH + W >= S.m)) {  // the BC rows take the sweep's face values
+    const int pl = tl + zlo * n1;                // index in the full face plane
+    const double lo = a.face_lo[fld] ? a.face_scale * __ldg(a.face_lo[fld] + pl) : 0.0;
+    const double hi = a.face_hi[fld] ? a.face_scale * __ldg(a.face_hi[fld] + pl) : 0.0;
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      if (e0 + q == 0) r[q] = lo;
+      if (e0 + q == S.m - 1) r[q] = hi;
+    }
+  }
+  chunk_solve<CH, W>(r, S, e0);
+  double* xl = dst + S.lo * st;
+  const int n = S.m - s;  // unknowns from this chunk's first on
+#pragma unroll
+  for (int q = 0; q < CH; ++q)
+    if (q >= skip && f + q < S.m) xl[(f + q) * st] = r[W + q];
+  const int nax = axis_n(L, AXIS);
+  if (walls) {  // the carried slots
+    if (s == 0)
+      for (int i = 0; i < S.lo; ++i) dst[i * st] = src[i * st];
+    if (n <= CH)
+      for (int i = S.lo + S.m; i <= nax + 1; ++i) dst[i * st] = src[i * st];
+  } else {
+    if (s == 0) dst[(nax + 1) * st] = xl[0];  // slot n+1 <- slot 1
+    if (n <= CH) dst[0] = xl[(S.m - 1) * st];  // slot 0 <- slot n (written above; a register picked by n
+  }                                            // would put the array on the stack)
+}
+
+// x sweep: a warp takes one chunk of 32 consecutive lines; its rows pass
+// through shared memory (stride 33), so that every global access is a row
+// segment.
+template <int CH, int W>
+__global__ void __launch_bounds__(32 * XW, CH + 2 * W <= 50 ? 4 : 3) adi_chunk_x_kernel(const __grid_constant__ AdiArgs a) {
+  constexpr int R = CH + 2 * W;
+  extern __shared__ double sh_x[];
+  const Layout& L = a.L;
+  const int fld = blockIdx.z, s = blockIdx.y * CH;
+  const ChunkSys& S = a.ch[fld];
+  if (s >= S.m) return;
+  const int n1 = L.ny + 2;
+  const int nlines = n1 * (a.z1 > 0 ? a.z1 - a.z0 : L.nz + 2);
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int t0 = (blockIdx.x * XW + warp) * 32;
+  if (t0 >= nlines) return;
+  const int nl = min(32, nlines - t0);
+  const int t = t0 + min(lane, nl - 1);  // lanes past the end repeat the last line (never stored)
+  const int j = t % n1, k = a.z0 + t / n1;
+  const int my_off = (int)L.at(S.lo, j, k);  // unknown 0 of this lane's line
+  double* sb = sh_x + warp * (R * XS);
+  const double* __restrict__ src = a.src[fld];
+  double* __restrict__ dst = a.dst[fld];
+  const bool walls = !S.periodic;
+  const int f = chunk_first<CH>(S, s), e0 = f - W, skip = s - f;
+  int er[(R + 31) / 32];
+#pragma unroll
+  for (int p = 0; p < (R + 31) / 32; ++p) er[p] = chunk_row(S, e0 + lane + 32 * p);
+#pragma unroll 4
+  for (int l = 0; l < 32; ++l) {
+    const int off = __shfl_sync(0xffffffffu, my_off, l);
+#pragma unroll
+    for (int p = 0; p < (R + 31) / 32; ++p) {
+      const int q = lane + 32 * p;
+      if (q < R) {
+        if (er[p] >= 0) cp_async8(&sb[q * XS + l], src + off + er[p]);
+        else sb[q * XS + l] = 0.0;
+      }
+    }
+  }
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncwarp();
+  double r[R];
+#pragma unroll
+  for (int q = 0; q < R; ++q) r[q] = sb[q * XS + lane];
+  if (walls && (f == 0 || f + CH + W >= S.m)) {  // the BC rows take the sweep's face values
+    const int pl = j + n1 * k;
+    const double lo = a.face_lo[fld] ? a.face_scale * __ldg(a.face_lo[fld] + pl) : 0.0;
+    const double hi = a.face_hi[fld] ? a.face_scale * __ldg(a.face_hi[fld] + pl) : 0.0;
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      if (e0 + q == 0) r[q] = lo;
+      if (e0 + q == S.m - 1) r[q] = hi;
+    }
+  }
+  chunk_solve<CH, W>(r, S, e0);
+#pragma unroll
+  for (int q = W; q < W + CH; ++q) sb[q * XS + lane] = r[q];
+  __syncwarp();
+  const int n = S.m - s, nc = min(n, CH);
+#pragma unroll 4
+  for (int l = 0; l < 32; ++l) {
+    const int off = __shfl_sync(0xffffffffu, my_off, l);
+    if (l < nl)
+      for (int q = lane; q < nc; q += 32) dst[off + s + q] = sb[(W + skip + q) * XS + l];
+  }
+  if (lane < nl) {
+    const double* xs = src + L.at(0, j, k);
+    double* xd = dst + L.at(0, j, k);
+    if (walls) {  // the carried slots
+      if (s == 0)
+        for (int i = 0; i < S.lo; ++i) xd[i] = xs[i];
+      if (n <= CH)
+        for (int i = S.lo + S.m; i <= L.nx + 1; ++i) xd[i] = xs[i];
+    } else {
+      if (s == 0) xd[L.nx + 1] = sb[W * XS + lane];             // slot n+1 <- slot 1
+      if (n <= CH) xd[0] = sb[(W + skip + n - 1) * XS + lane];  // slot 0 <- slot n
+    }
+  }
+}
+
+template <int CH, int W>
+cudaError_t launch_adi_chunk(int axis, const AdiArgs& a, cudaStream_t st) {
+  const int n1 = axis == 0 ? a.L.ny + 2 : a.L.nx + 2;
+  const int n2 = axis == 2 ? a.L.ny + 2 : (a.z1 > 0 ? a.z1 - a.z0 : a.L.nz + 2);
+  if (n2 <= 0) return cudaSuccess;
+  const int m = std::max(a.ch[0].m, std::max(a.ch[1].m, a.ch[2].m));
+  const dim3 grid((unsigned)((n1 * n2 + 127) / 128), (unsigned)((m + CH - 1) / CH), 3);
+  if (axis == 0) {
+    const size_t sm = (size_t)XW * (CH + 2 * W) * XS * sizeof(double);
+    cudaError_t e = cudaFuncSetAttribute(adi_chunk_x_kernel<CH, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+    adi_chunk_x_kernel<CH, W><<<grid, 32 * XW, sm, st>>>(a);
+  } else if (axis == 1) {
+    adi_chunk_kernel<1, CH, W><<<grid, 128, 0, st>>>(a);
+  } else {
+    adi_chunk_kernel<2, CH, W><<<grid, 128, 0, st>>>(a);
+  }
+  return cudaGetLastError();
+}
+
+// Unknowns per chunk: 32, or 34 where that saves a chunk (the n + 2 unknowns
+// of a wall line), and 16 on boxes whose 32-unknown chunks leave SMs idle.
+cudaError_t launch_adi_chunks(int axis, const AdiArgs& a, cudaStream_t st) {
+  const int m = std::max(a.ch[0].m, std::max(a.ch[1].m, a.ch[2].m));
+  const long long cells = 3LL * (a.L.nx + 2) * (a.L.ny + 2) * (a.L.nz + 2);
+  const int ch = cells / 32 < 40000 ? 16 : ((m + 33) / 34 < (m + 31) / 32 ? 34 : 32);
+#define NS_ADI_HALO(W)                                                             \
+  if (a.halo == W)                                                                 \
+    return ch == 16 ? launch_adi_chunk<16, W>(axis, a, st)                         \
+                    : (ch == 34 ? launch_adi_chunk<34, W>(axis, a, st) : launch_adi_chunk<32, W>(axis, a, st));
+  NS_ADI_HALO(6) NS_ADI_HALO(8) NS_ADI_HALO(10) NS_ADI_HALO(12) NS_ADI_HALO(16)
+#undef NS_ADI_HALO
+  return cudaErrorInvalidValue;
+}
+
 // y and z sweeps: the persistent line kernel, 8 CTAs of 128 threads per SM
 // (measured at 256^3: 0.38 / 0.37 ms against 0.44 / 0.41 ms for one thread
 // per line without prefetch); the x sweep keeps the shared-memory blocked
 // kernel, whose row loads are coalesced.
 cudaError_t launch_adi(int axis, const AdiArgs& a, cudaStream_t st) {
+  if (a.halo) return launch_adi_chunks(axis, a, st);
   if (axis != 0) {
     int dev = 0, nsm = 0;
     cudaError_t e = cudaGetDevice(&dev);

@@ -49,6 +49,85 @@ namespace ns {
 // unknowns); otherwise tangential (B matrix, n+2 unknowns).
 // transposed (periodic only): the system M^T of the adjoint sweep, whose
 // corner entries are those of M exchanged.
+HostChunkSys build_chunk_system(int n, int bc, double h, double dt, double nu, bool normal, int closure) {
+  typedef long double ld;
+  const double idx2 = 1.0 / (h * h);
+  const double dg = 1.0 + 0.5 * dt * nu * 2.0 * idx2, of = -0.5 * dt * nu * 1.0 * idx2;  // as build_cn_system
+  HostChunkSys S;
+  const int m = S.m = bc == 1 ? n : (normal ? n + 1 : n + 2);
+  S.lo = bc == 1 || normal ? 1 : 0;
+  std::vector<ld> a(m, of), b(m, dg), c(m, of);  // a[0], c[m-1]: the couplings past the ends
+  if (bc == 1) {
+    if (normal && closure == 0) {  // A(1,n+1) ties face 1 to itself (build_cn_system)
+      b[0] = (ld)dg + of;
+      a[0] = 0;
+    }
+    S.wrap_lo = !(normal && closure == 0);
+    S.wrap_hi = S.periodic = 1;
+  } else {
+    const ld e = !normal && bc == 2 ? 0.5L : 1.0L, f = !normal && bc == 2 ? 0.5L : 0.0L;
+    b[0] = b[m - 1] = e;
+    c[0] = a[m - 1] = f;
+    a[0] = c[m - 1] = 0;
+  }
+  // elimination, around the cycle until it no longer depends on its start
+  std::vector<ld> l(m), d(m);
+  ld dp = ((ld)dg + sqrtl((ld)dg * dg - 4 * (ld)of * of)) / 2;  // the converged pivot
+  const ld dc = dp;
+  for (int turn = 0; turn < (S.wrap_lo ? 1 + 64 / m : 1); ++turn)
+    for (int e = 0; e < m; ++e) {
+      l[e] = a[e] / dp;
+      d[e] = b[e] - l[e] * c[e ? e - 1 : m - 1];
+      dp = d[e];
+    }
+  S.d = (double)(1 / dc);
+  S.lc = (double)(of / dc);
+  S.cc = (double)(of / dc);
+  const int ext = kAdiExt, len = m + 3 * ext;
+  S.l.assign(len, 0.0);
+  S.dm.assign(len, 0.0);
+  S.cu.assign(len, 0.0);
+  std::vector<char> conv(len, 0);
+  std::vector<double> dm(m), cu(m);
+  for (int e = 0; e < m; ++e) {
+    dm[e] = (double)(1 / (d[e] * (ld)S.d));
+    cu[e] = (double)(c[e] / d[e]);
+  }
+  for (int q = 0; q < len; ++q) {
+    const int e = q - ext;
+    if ((e < 0 && !S.wrap_lo) || (e >= m && !S.wrap_hi)) continue;
+    const int r = ((e % m) + m) % m;
+    S.l[q] = (double)l[r];
+    S.dm[q] = dm[r];
+    S.cu[q] = cu[r];
+    auto same = [](double x, double y) { return std::fabs(x - y) <= 4.5e-16 * std::fabs(y); };
+    conv[q] = same(S.l[q], S.lc) && same(S.cu[q], S.cc) && same(S.dm[q], 1.0);
+  }
+  int q0 = ext + m / 2, q1 = q0;
+  if (conv[q0]) {
+    while (q0 > 0 && conv[q0 - 1]) --q0;
+    while (q1 < len && conv[q1]) ++q1;
+  }
+  S.c0 = q0 - ext;
+  S.c1 = q1 - ext;
+  for (int w : {6, 8, 10, 12, 16}) {  // the weight of what lies w unknowns away
+    bool ok = true;
+    for (int q = 0; q + w <= len && ok; ++q) {
+      double pl = 1, pc = 1;
+      for (int i = 0; i < w; ++i) {
+        pl *= std::fabs(S.l[q + i]);
+        pc *= std::fabs(S.cu[q + i]);
+      }
+      ok = pl <= 0x1p-57 && pc <= 0x1p-57;
+    }
+    if (ok) {
+      S.halo = w;
+      break;
+    }
+  }
+  return S;
+}
+
 HostLineSys build_cn_system(int n, int bc, double h, double dt, double nu, bool normal, int closure,
                             bool transposed) {
   const double idx2 = 1.0 / (h * h);
@@ -525,6 +604,10 @@ PredictArgs predict_args(ns_handle* h) {
   a.hx = h->hx; a.hy = h->hy; a.hz = h->hz;
   a.err = h->dev_err;
   set_predict_coeffs(a, c.bc, h->dx, h->dy, h->dz, c.dt, c.nu);
+  if (h->adi_halo[0]) {  // the sweeps' right-hand sides come scaled (ChunkSys)
+    const double d = h->adi_d[0] * h->adi_d[1] * h->adi_d[2];
+    for (double* q : {&a.c0, &a.ca, &a.cb, &a.cc, &a.cu, &a.cC, &a.cP, &a.dt, &a.gpx, &a.gpy, &a.gpz}) *q *= d;
+  }
   set_predict_fixed(a, c.scheme, h->pmax);
   return a;
 }
@@ -545,7 +628,7 @@ void set_predict_coeffs(PredictArgs& a, const int bc[3], double dx, double dy, d
   const double hnd = 0.5 * nu * dt;
   a.ca = hnd * ix2; a.cb = hnd * iy2; a.cc = hnd * iz2;
   a.c0 = 1.0 - 2.0 * hnd * (ix2 + iy2 + iz2);
-  a.cC = 1.5 * dt; a.cP = -0.5 * dt;
+  a.cC = 1.5 * dt; a.cP = -0.5 * dt; a.cu = 1.0;
   a.dt = dt; a.e1 = 1.5 * dt; a.e2 = -0.5 * dt;
   a.gpx = -dt / dx; a.gpy = -dt / dy; a.gpz = -dt / dz;
   a.ix2 = ix2; a.iy2 = iy2; a.iz2 = iz2; a.lap0 = -2.0 * (ix2 + iy2 + iz2);
@@ -560,7 +643,9 @@ namespace {
 // the final u*, v*, w* are in B on every step (and in every captured graph).
 // With keep_sweeps the x sweep writes C instead (and y reads C), so after a
 // step C holds u* after the x sweep, A after the y sweep, B after the z sweep.
-AdiArgs adi_args(ns_handle* h, int ax) {
+// chunked: the step's sweeps, whose right-hand sides the predictor scales
+// (predict_args); not ns_adi's.
+AdiArgs adi_args(ns_handle* h, int ax, bool chunked = true) {
   double* A[3] = {h->us, h->vs, h->ws};
   double* B[3] = {h->us2, h->vs2, h->ws2};
   double* X[3] = {h->us3 ? h->us3 : h->us2, h->vs3 ? h->vs3 : h->vs2, h->ws3 ? h->ws3 : h->ws2};
@@ -572,13 +657,17 @@ AdiArgs adi_args(ns_handle* h, int ax) {
     a.sys[f] = h->sys[ax][f];
     a.face_lo[f] = h->face_set_nonzero[1 + ax] ? h->faces[1 + ax].ax[ax].f[f][0] : nullptr;
     a.face_hi[f] = h->face_set_nonzero[1 + ax] ? h->faces[1 + ax].ax[ax].f[f][1] : nullptr;
+    a.ch[f] = h->csys[ax][f];
   }
+  a.halo = chunked ? h->adi_halo[ax] : 0;
+  a.face_scale = 1.0;
+  for (int q = ax; q < 3; ++q) a.face_scale *= h->adi_d[q];
   return a;
 }
 
 int enqueue_adi(ns_handle* h) {
   for (int ax = 0; ax < 3; ++ax) {
-    NS_CUDA(h, launch_adi(ax, adi_args(h, ax), h->stream));
+    NS_CUDA(h, launch_adi(ax, adi_args(h, ax, false), h->stream));
     mark(h, ax == 0 ? "adi_x" : (ax == 1 ? "adi_y" : "adi_z"));
   }
   return NS_OK;
@@ -1015,9 +1104,50 @@ int build_line_tables(ns_handle* h, bool transposed, LineSys sys[3][3], double**
   return NS_OK;
 }
 
+// The chunked sweeps' tables, when every system's halo is at most 16.  Their
+// right-hand sides are scaled by the product of the pivots still to come, so
+// a session that hands out u* between the sweeps (keep_sweeps) keeps the
+// whole-line kernels.
+int build_adi_chunks(ns_handle* h) {
+  const ns_config& c = h->cfg;
+  const int ns_[3] = {c.nx, c.ny, c.nz};
+  const double hs[3] = {h->dx, h->dy, h->dz};
+  if (c.keep_sweeps) return NS_OK;
+  HostChunkSys S[3][3];
+  size_t total = 0;
+  for (int ax = 0; ax < 3; ++ax)
+    for (int f = 0; f < 3; ++f) {
+      // the two tangential fields share a system
+      const int first = ax == 0 ? 1 : 0;
+      if (f != ax && f != first) S[ax][f] = S[ax][first];
+      else S[ax][f] = build_chunk_system(ns_[ax], c.bc[ax], hs[ax], c.dt, c.nu, f == ax, c.cn_periodic_closure);
+      if (!S[ax][f].halo) return NS_OK;
+      total += 3 * S[ax][f].l.size();
+    }
+  NS_CUDA(h, cudaMalloc(&h->adi_chunk_buf, total * sizeof(double)));
+  std::vector<double> host;
+  host.reserve(total);
+  for (int ax = 0; ax < 3; ++ax)
+    for (int f = 0; f < 3; ++f) {
+      const HostChunkSys& q = S[ax][f];
+      ChunkSys& D = h->csys[ax][f];
+      D.l = h->adi_chunk_buf + host.size(); host.insert(host.end(), q.l.begin(), q.l.end());
+      D.dm = h->adi_chunk_buf + host.size(); host.insert(host.end(), q.dm.begin(), q.dm.end());
+      D.cu = h->adi_chunk_buf + host.size(); host.insert(host.end(), q.cu.begin(), q.cu.end());
+      D.lc = q.lc; D.cc = q.cc; D.c0 = q.c0; D.c1 = q.c1; D.lo = q.lo; D.m = q.m;
+      D.wrap_lo = q.wrap_lo; D.wrap_hi = q.wrap_hi; D.periodic = q.periodic;
+      h->adi_d[ax] = q.d;  // the converged pivot is the same for the three fields
+      h->adi_halo[ax] = std::max(h->adi_halo[ax], q.halo);
+    }
+  NS_CUDA(h, cudaMemcpyAsync(h->adi_chunk_buf, host.data(), total * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+  NS_CUDA(h, cudaStreamSynchronize(h->stream));
+  return NS_OK;
+}
+
 int build_adi(ns_handle* h) {
   if (h->cfg.scheme != NS_AB2_CN) return NS_OK;
-  return build_line_tables(h, false, h->sys, &h->adi_buf);
+  const int s = build_line_tables(h, false, h->sys, &h->adi_buf);
+  return s ? s : build_adi_chunks(h);
 }
 
 void free_all(ns_handle* h) {
@@ -1049,6 +1179,7 @@ void free_all(ns_handle* h) {
   for (cudaEvent_t e : h->trace_pool) cudaEventDestroy(e);
   if (h->tw) cudaFree(h->tw);
   if (h->pmax) cudaFree(h->pmax);
+  if (h->adi_chunk_buf) cudaFree(h->adi_chunk_buf);
   if (h->diag_bits) cudaFree(h->diag_bits);
   if (h->dev_err) cudaFree(h->dev_err);
   if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);

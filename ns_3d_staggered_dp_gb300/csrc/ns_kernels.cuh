@@ -48,6 +48,7 @@ struct PredictArgs {
   double k0, kx, ky, kz;
   // AB2-CN: u* = c0*u + ca*sWE + cb*sSN + cc*sBT + cC*C + cP*prev
   double c0, ca, cb, cc, cC, cP;
+  double cu;          // AB2-CN: u* = cu*u + viscous increment + ... (the scale of the sweeps' right-hand sides)
   double dt, e1, e2;  // AB2: u* = u + e1*rhs + e2*prev
   double gpx, gpy, gpz;  // -dt/dx etc. (dp_flag)
   double ix2, iy2, iz2, lap0;  // diffusion-only mode
@@ -192,6 +193,22 @@ struct LineSys {
   int n;               // cells along the axis
   int pad;             // zero padding on each side of the factor tables
 };
+// The same system for the chunked sweeps: every chunk of a line is solved by
+// itself, from `halo` unknowns before it to `halo` after it, because what lies
+// further away enters with a weight below 2^-57.  The rows' right-hand sides
+// come scaled by 1 / (converged pivot), so that a row with the converged
+// factors takes one FMA each way: y' = r - lc y', x = y' - cc x.
+struct ChunkSys {
+  const double* l;   // forward multipliers, index kAdiExt + e, e in [-kAdiExt, m + 2 kAdiExt): continued
+  const double* dm;  // past an end where the system is cyclic there, else zero; dm: pivot ratio
+  const double* cu;  // super-diagonal / pivot
+  double lc, cc;     // their values on the rows [c0, c1), where dm is 1
+  int c0, c1;
+  int lo, m;         // slot of unknown 0, unknowns
+  int wrap_lo, wrap_hi;  // rows before the first / after the last continue at the other end
+  int periodic;
+};
+constexpr int kAdiExt = 64;
 struct AdiArgs {
   Layout L;
   const double* src[3];  // u*, v*, w* before the sweep
@@ -200,6 +217,9 @@ struct AdiArgs {
   const double* face_lo[3];  // BC row values per field (internal-slot planes), NULL -> 0
   const double* face_hi[3];
   int z0, z1;                // x and y sweeps: only the lines of z slots [z0, z1) (z1 = 0: all)
+  int halo;                  // chunked sweeps: unknowns beyond a chunk (6, 8, 10, 12 or 16; 0: the whole-line kernels)
+  ChunkSys ch[3];
+  double face_scale;         // chunked sweeps: the scale of this sweep's right-hand sides
 };
 cudaError_t launch_adi(int axis, const AdiArgs& a, cudaStream_t st);
 // The tile loader's bounded mbarrier wait on a barrier that no copy fills (ns_predict.cu).

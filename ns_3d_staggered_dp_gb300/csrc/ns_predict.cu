@@ -507,7 +507,7 @@ __device__ __forceinline__ void predict_fx_planes(const PredictArgs& a, FxPredSm
   };
   auto combine = [&](double uc, double Lv, double C, double prev, double* __restrict__ hist, long long g) -> double {
     if (SCHEME == 2) {  // AB2-CN explicit half (big_periodic_3D.f90:398-423)
-      double t = fma(FIRST ? a.dt : a.cC, C, fadd(c, uc, Lv));  // Euler start: nu/2 diff - conv (:400-408)
+      double t = fma(FIRST ? a.dt : a.cC, C, fma(a.cu, uc, Lv));  // Euler start: nu/2 diff - conv (:400-408)
       if (!FIRST) t = fma(a.cP, prev, t);
       hist[g] = C;  // rhs_?_previous = -conv
       return t;

@@ -46,6 +46,11 @@ struct ns_handle {
   // ADI factors
   double* adi_buf = nullptr;
   ns::LineSys sys[3][3];  // [axis][field]
+  // the chunked sweeps (adi_halo 0 on every axis: not used): tables, systems, 1 / converged pivot per axis
+  double* adi_chunk_buf = nullptr;
+  ns::ChunkSys csys[3][3];
+  double adi_d[3] = {1.0, 1.0, 1.0};
+  int adi_halo[3] = {0, 0, 0};
   // faces: [set 0..3][axis][field 0..3][side] -> device planes
   double* face_buf = nullptr;
   std::vector<double> face_host;  // host staging of one face set (ns_set_faces)
@@ -105,6 +110,14 @@ struct HostLineSys {
   double s0 = 0, s1 = 0;
   int zA = 0, zB = 0, lo = 0, hi = 0, periodic = 0, n = 0;
 };
+// The same system for the chunked sweeps, tables on the extended index
+// [-kAdiExt, m + 2 kAdiExt); halo is 0 when 16 unknowns do not suffice.
+struct HostChunkSys {
+  std::vector<double> l, dm, cu;
+  double lc = 0, cc = 0, d = 1;  // d: 1 / converged pivot (the right-hand sides' scale)
+  int c0 = 0, c1 = 0, lo = 0, m = 0, wrap_lo = 0, wrap_hi = 0, periodic = 0, halo = 0;
+};
+HostChunkSys build_chunk_system(int n, int bc, double h, double dt, double nu, bool normal, int closure);
 // The CN system of one sweep axis (mat_CN / mat_CN_tridiagonal,
 // NS_functions.f90:1245-1342) for n cells with velocity code bc; normal: the
 // swept field is staggered along the axis (ns_api.cu).

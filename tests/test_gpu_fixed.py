@@ -157,3 +157,49 @@ def test_slabs_of_different_exponents(n, kw, scheme):
         host = s.step_host(st.u, st.v, st.w, st.p, hist)
     for k in dev:
         assert np.array_equal(dev[k], host[k]), k
+
+
+# --- the chunked ADI sweeps ---------------------------------------------------------------------
+SWEEPS = [((16, 16, 16), (1, 1, 1)), ((64, 32, 128), (1, 1, 1)), ((32, 67, 16), (1, 2, 1)), ((64, 32, 34), (1, 1, 2)),
+          ((38, 21, 35), (2, 2, 2)), ((66, 64, 17), (4, 2, 4))]
+
+
+@pytest.mark.parametrize("n,bc", SWEEPS)
+@pytest.mark.parametrize("alpha", [0.0, 1e-4, 0.004, 0.012, 0.03, 0.07, 0.3])
+@pytest.mark.parametrize("closure", [0, 1])
+def test_sweeps_for_every_halo(n, bc, alpha, closure):
+    """u*, v*, w* after the sweeps, with viscous numbers on both sides of every halo's limit (and
+    beyond the last, where the whole-line kernels run): a few roundings of values of order one."""
+    from ns_3d_staggered_dp_gb300 import Session, make_config
+    from tests.helpers import random_state
+
+    if closure and 1 not in bc:
+        pytest.skip("no periodic axis")
+    wall = {1: 1, 2: 3, 4: 4}
+    dt, L = 0.003, [2.0 * np.pi] * 3
+    # the same viscous number on every axis: lengths in proportion to the cells
+    L = [2.0 * np.pi * m / n[0] for m in n]
+    nu = 2.0 * alpha * (L[0] / n[0]) ** 2 / dt
+    cfg = O.Config(*n, *L, nu=nu, dt=dt, scheme=O.AB2_CN, bc=bc, pbc=tuple(wall[b] for b in bc))
+    st = random_state(cfg, 3, amp=0.1, history=True)
+    cnf = None
+    if closure:  # the cyclic closure of the periodic normal component
+        cnf = O.CNFactors(*n, cfg.bc, *(h * h for h in cfg.h), dt, nu)
+        for ax, b in enumerate(bc):
+            if b == 1:
+                A = O.mat_cn(n[ax], 1, cfg.h[ax] ** 2, dt, nu)[0]
+                A[0, n[ax] - 1], A[0, n[ax]] = A[0, n[ax]], 0.0
+                cnf.lu[ax] = (O._lu(A), cnf.lu[ax][1])
+    ref, parts = O.step(st.copy(), cfg, cnf=cnf, return_parts=True)
+    with Session(make_config(*n, lx=L[0], ly=L[1], lz=L[2], nu=nu, dt=dt, scheme=2, bc=cfg.bc, pbc=cfg.pbc,
+                             cn_periodic_closure=closure)) as s:
+        s.set_state(st.u, st.v, st.w, st.p, (st.px, st.py, st.pz))
+        s.step(1)
+        g = s.get_stage()
+        out = s.get_state()
+    inner = {"us": (slice(None), slice(1, -1), slice(1, -1)), "vs": (slice(1, -1), slice(None), slice(1, -1)),
+             "ws": (slice(1, -1), slice(1, -1), slice(None))}
+    for k, sl in inner.items():
+        assert rel_l2(g[k][sl], parts[k][sl]) < 1e-13, k
+    for k in "uvw":
+        assert rel_l2(out[k], getattr(ref, k)) < 1e-10, k
