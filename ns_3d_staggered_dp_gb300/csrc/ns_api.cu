@@ -950,7 +950,9 @@ int build_plans(ns_handle* h) {
     std::vector<double> F, G;
     dense_pair(n3[a], c.pbc[a], F, G);
     const int n = n3[a];
-    P.sym[a] = dense_symmetry(n, F, G);
+    const int fe = q54_table(F);
+    P.gexp[a] = q54_table(G);
+    if (fe != 0) return fail(h, NS_ERR_ARG, "internal: a forward transform entry exceeds 1");
     if (a == 0) {
       std::vector<double> Ft((size_t)n * n), Gt((size_t)n * n);
       for (int r = 0; r < n; ++r)
@@ -1026,8 +1028,8 @@ int build_plans(ns_handle* h) {
   P.eig_x = (sax || zcyc) ? t0 + o_ex : nullptr;
   P.eig_o = (sax || zcyc) ? t0 + o_eo : nullptr;
   for (int a = 0; a < 3; ++a) {
-    P.fwd[a] = P.kind[a] == 1 ? t0 + o_f[a] : nullptr;
-    P.inv[a] = P.kind[a] == 1 ? t0 + o_g[a] : nullptr;
+    P.fwd[a] = P.kind[a] == 1 ? reinterpret_cast<const int2*>(t0 + o_f[a]) : nullptr;
+    P.inv[a] = P.kind[a] == 1 ? reinterpret_cast<const int2*>(t0 + o_g[a]) : nullptr;
   }
   // pr_bc_staggered_modify_rhs coefficients (NS_functions.f90:1345-1400) and
   // the set-0 pressure face planes they read.

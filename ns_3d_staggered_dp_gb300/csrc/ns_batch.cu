@@ -784,7 +784,7 @@ int ns_batch_create(const ns_batch_config* cfg, const ns_subdomain* subs, int n,
   // ---- size-class tables: dense x (transposed) and y pairs, x and y eigenvalues ----
   std::vector<double> tab;
   std::map<int, size_t> xF, xG, yF, yG, ex, ey;
-  std::map<int, int> ysym, xsym;  // symmetry bits of the y and x pairs per size
+  std::map<int, int> yg, xg;  // exponents of the y and x inverse matrices per size
   // FFT-based DCT tables of the axes of 24, 32, 48 and 64 points (pressure
   // codes 2 and 3; NS_DENSE_X / NS_DENSE_Y keep the dense products): the
   // N-point twiddles exp(-2 pi i m / N), m < N, then exp(-i pi k / (2N)) / 2,
@@ -808,7 +808,8 @@ int ns_batch_create(const ns_batch_config* cfg, const ns_subdomain* subs, int n,
     if (!xF.count(nx)) {
       std::vector<double> F, G;
       dense_pair(nx, c.pbc, F, G);
-      xsym[nx] = dense_symmetry(nx, F, G);
+      if (q54_table(F) != 0) return bail(NS_ERR_ARG);
+      xg[nx] = q54_table(G);
       std::vector<double> Ft((size_t)nx * nx), Gt((size_t)nx * nx);
       for (int r = 0; r < nx; ++r)
         for (int q = 0; q < nx; ++q) { Ft[(size_t)q * nx + r] = F[(size_t)r * nx + q]; Gt[(size_t)q * nx + r] = G[(size_t)r * nx + q]; }
@@ -821,7 +822,8 @@ int ns_batch_create(const ns_batch_config* cfg, const ns_subdomain* subs, int n,
     if (!yF.count(ny)) {
       std::vector<double> F, G;
       dense_pair(ny, c.pbc, F, G);
-      ysym[ny] = dense_symmetry(ny, F, G);
+      if (q54_table(F) != 0) return bail(NS_ERR_ARG);
+      yg[ny] = q54_table(G);
       yF[ny] = tab.size(); tab.insert(tab.end(), F.begin(), F.end()); tab.resize(align32(tab.size()));
       yG[ny] = tab.size(); tab.insert(tab.end(), G.begin(), G.end()); tab.resize(align32(tab.size()));
       ey[ny] = tab.size();
@@ -932,10 +934,9 @@ int ns_batch_create(const ns_batch_config* cfg, const ns_subdomain* subs, int n,
     S = SpecPlan{};
     S.nx = d.nx; S.ny = d.ny; S.nz = d.nz; S.nxh = d.nx / 2 + 1; S.nxs = d.nx / 2;
     S.kind[0] = 1; S.kind[1] = 1; S.kind[2] = 2;
-    S.fwd[0] = b->tables + xF[d.nx]; S.inv[0] = b->tables + xG[d.nx];
-    S.fwd[1] = b->tables + yF[d.ny]; S.inv[1] = b->tables + yG[d.ny];
-    S.sym[1] = ysym[d.ny];
-    S.sym[0] = xsym[d.nx];
+    auto q54 = [&](size_t off) { return reinterpret_cast<const int2*>(b->tables + off); };
+    S.fwd[0] = q54(xF[d.nx]); S.inv[0] = q54(xG[d.nx]); S.gexp[0] = xg[d.nx];
+    S.fwd[1] = q54(yF[d.ny]); S.inv[1] = q54(yG[d.ny]); S.gexp[1] = yg[d.ny];
     S.eig_x = b->tables + ex[d.nx];
     S.eig_o = b->tables + ey[d.ny];
     if (dct_x_on && dct_size(d.nx)) {

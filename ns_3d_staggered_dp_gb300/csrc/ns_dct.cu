@@ -9,7 +9,7 @@
 //   pbc 2 (Dirichlet on the wall)  : flip the sign of every other input,
 //                                    DCT-II, reverse the output (= DST-II)
 //   pbc 4 (Dirichlet on the ghost) : F = DST-I of N points
-// and applied to a line held in shared memory (2N FMAs per complex output).
+// and applied to a line held in shared memory, on fixed-point integers.
 // Any N works (the subdomain edges 24 and 48 included).
 //
 // Data flow: with x periodic the x pass is the r2c FFT of ns_fft.cu and the
@@ -25,6 +25,7 @@
 // pr_bc_staggered_modify_rhs (NS_functions.f90:1345-1400) on the first and
 // last cells of every non-periodic axis.
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "ns_fft_core.cuh"
@@ -50,178 +51,186 @@ __device__ __forceinline__ double rhs_cell(const DivArgs& d, const SpecPlan& S, 
 
 }  // namespace
 
-// x pass for a non-periodic x axis: real line -> F_x -> packed modes.
-// One warp per line (j, k); lane q computes the modes 2q' and 2q'+1.
+// ---------------------------------------------------------------------------
+// Dense transforms on block fixed-point integers (ns_fixed.cuh): a line
+// becomes integers of one exponent, a matrix entry an integer in units of
+// 2^-54 (times 2^-gexp for the inverse), both split at bit 27, so that a
+// product and sum is three 32-bit multiply-adds into two 64-bit sums: 14
+// integer issue clocks against the 64 of an FP64 FMA.  The entries' low parts
+// are signed, so the dropped products of the low parts have mean 0.
+// For codes 2, 3 and 4 and any N, F[k][N-1-n] = (-1)^k F[k][n] and
+// G[N-1-n][k] = (-1)^k G[n][k], so each pass sums half the products: forward,
+// an even mode takes s[n] = x[n] + x[N-1-n], an odd one d[n] = x[n] - x[N-1-n]
+// (s kept at n, the middle sample of an odd N with it, d at N-1-n); inverse,
+// the even and odd modes' sums E and O give E + O at n and E - O at N-1-n.
+// ---------------------------------------------------------------------------
+constexpr int DX_SEG = 128;  // terms per 64-bit partial sum
+
+struct DxSum {
+  long long hi = 0, mid = 0;
+  __device__ __forceinline__ void add(int vh, int vl, int2 w) {
+    hi = fx_wide(vh, w.x, hi);
+    mid = fx_wide(vl, w.x, fx_wide(vh, w.y, mid));
+  }
+  __device__ __forceinline__ void fold() {
+    hi += (mid + (1ll << 26)) >> 27;
+    mid = 0;
+  }
+};
+// A line whose largest biased exponent is E and whose magnitudes sum to less
+// than 2^lb of its unit 2^(E+1): the exponent to convert at, so that a value
+// takes at most `most` bits and any sum of products at most 62, the unit's
+// exponent eb, and the power of two that brings extreme lines into range
+// first (scaled).  (The sum of the magnitudes, not their number times the
+// largest: a line with few large values keeps more bits.)
+struct DxExp {
+  int ec, eb;
+  bool scaled, up;
+};
+__device__ __forceinline__ DxExp dx_exp(int E, int lb, int most) {
+  DxExp x;
+  x.scaled = E < 128 || E > 1900;
+  x.up = E < 128;
+  const int adj = x.scaled ? (x.up ? 512 : -512) : 0;
+  x.ec = max(E + adj + (E == 0 ? 1 : 0), 64) + (58 - min(most, 62 - lb));
+  x.eb = E == 0x7ff ? kFxNonfinite : x.ec - 1022 - 58 - adj;
+  return x;
+}
+// A value's share of the sum, in units of 2^(E+1-20), rounded up; its lb.
+__device__ __forceinline__ unsigned dx_share(int E, unsigned hi2) {
+  return ((1u << 20) >> min(E - (int)(hi2 >> 21), 31)) + 1u;
+}
+__device__ __forceinline__ int dx_sum_bits(unsigned sum) { return 32 - __clz((int)sum) - 20; }
+__device__ __forceinline__ long long dx_from(double d, const DxExp& x) {
+  if (x.scaled) d *= x.up ? 0x1p512 : 0x1p-512;
+  return fx_round<58>(d, x.ec);
+}
+__device__ __forceinline__ int2 dx_split(long long v) { return make_int2((int)(v >> 27), (int)v & ((1 << 27) - 1)); }
+__device__ __forceinline__ int dx_biased(unsigned hi2) { return (int)(hi2 >> 21); }  // of 2 |high word|
+
+// x pass for a non-periodic x axis: real line -> F_x -> packed modes.  A
+// group of G lanes takes a line (128/G lines per CTA, several short lines
+// share a warp); lane q computes the modes 2q and 2q+1.
 __device__ __forceinline__ void dense_x_fwd_body(const SpecPlan& S, const DivArgs& d, double2* __restrict__ spec,
                                                  double* xs, int bx) {
-  // a group of G lanes per line, 128/G lines per CTA (several short lines share a warp)
   const int G = dense_x_group(S.nx);
   const int grp = threadIdx.x / G, gl = threadIdx.x % G;
   const int line = bx * (128 / G) + grp;
-  const int nx = S.nx, ny = S.ny, nz = S.nz;
+  const int nx = S.nx, ny = S.ny, nz = S.nz, H = nx / 2;
   const bool valid = line < ny * nz;
   const int j = valid ? 1 + line % ny : 1, k = valid ? 1 + line / ny : 1;
   double* r = xs + grp * nx;
+  int2* v = reinterpret_cast<int2*>(r);
   const FOne c{d.one, d.mzero};
-  if (valid)
-    for (int i = gl; i < nx; i += G) r[i] = rhs_cell(d, S, c, i + 1, j, k);
-  __syncwarp();
-  const double* __restrict__ FT = S.fwd[0];  // F^T: FT[n * N + kk] = F[kk][n]
-  double2* out = spec + (long long)S.nxs * ((j - 1) + (long long)ny * (k - 1));
-  if (S.sym[0] & 1) {
-    // F[k][N-1-n] = (-1)^k F[k][n]: fold the line (s[n] = r[n] + r[N-1-n] at n,
-    // d[n] = r[n] - r[N-1-n] at N-1-n); mode 2q sums F s, mode 2q+1 sums F d
-    const int H = nx / 2;
-    if (valid)
-      for (int n = gl; n < H; n += G) {
-        const double a0 = r[n], b0 = r[nx - 1 - n];
-        r[n] = a0 + b0;
-        r[nx - 1 - n] = a0 - b0;
-      }
-    __syncwarp();
-    const int lv1 = (S.sym[0] >> 2) & 3;  // bit p: the modes of parity p fold once more
-    if (lv1 == 1 || lv1 == 2) {
-      // Second fold of one branch over its H points (sign (-1)^((k >> 1) & 1)):
-      // the even branch s (at 0..H-1) into s2 at n and d2 at H-1-n, the odd
-      // branch d (d[n] at N-1-n) into s2 at N-1-n and d2 at H+n, n < H/2.
-      // The folded mode of a pair then sums H/2 terms, the other one sums
-      // the mirrored terms n and H-1-n together.
-      const int Q = H / 2;
-      if (valid)
-        for (int n = gl; n < Q; n += G) {
-          const int ia = lv1 == 1 ? n : nx - 1 - n, ib = lv1 == 1 ? H - 1 - n : H + n;
-          const double a0 = r[ia], b0 = r[ib];
-          r[ia] = a0 + b0;
-          r[ib] = a0 - b0;
-        }
-      __syncwarp();
-      if (!valid) return;
-      for (int q = gl; q < H; q += G) {
-        const int b1 = q & 1;  // ((2q or 2q+1) >> 1) & 1
-        double a = 0.0, b = 0.0;
-        if (lv1 == 1) {  // mode 2q folded, mode 2q+1 on d
-          for (int n = 0; n < Q; ++n) {
-            const double2 f = *reinterpret_cast<const double2*>(FT + (long long)n * nx + 2 * q);
-            const double fm = FT[(long long)(H - 1 - n) * nx + 2 * q + 1];
-            a = fma(f.x, b1 ? r[H - 1 - n] : r[n], a);
-            b = fma(f.y, r[nx - 1 - n], b);
-            b = fma(fm, r[H + n], b);
-          }
-        } else {  // mode 2q on s, mode 2q+1 folded
-          for (int n = 0; n < Q; ++n) {
-            const double2 f = *reinterpret_cast<const double2*>(FT + (long long)n * nx + 2 * q);
-            const double fm = FT[(long long)(H - 1 - n) * nx + 2 * q];
-            a = fma(f.x, r[n], a);
-            a = fma(fm, r[H - 1 - n], a);
-            b = fma(f.y, b1 ? r[H + n] : r[nx - 1 - n], b);
-          }
-        }
-        out[q] = make_double2(a, b);
-      }
-      return;
-    }
-    if (!valid) return;
-    for (int q = gl; q < H; q += G) {
-      double a = 0.0, b = 0.0;
-      for (int n = 0; n < H; ++n) {
-        const double2 f = *reinterpret_cast<const double2*>(FT + (long long)n * nx + 2 * q);
-        a = fma(f.x, r[n], a);
-        b = fma(f.y, r[nx - 1 - n], b);
-      }
-      out[q] = make_double2(a, b);
-    }
-    return;
+  unsigned m = 0;
+  for (int i = gl; i < nx; i += G) {
+    const double x = valid ? rhs_cell(d, S, c, i + 1, j, k) : 0.0;
+    m = max(m, (unsigned)__double2hiint(x) << 1);
+    r[i] = x;
   }
+  for (int o = G / 2; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+  const int E = dx_biased(m);
+  unsigned sum = 0;
+  for (int i = gl; i < nx; i += G) sum += dx_share(E, (unsigned)__double2hiint(r[i]) << 1);
+  for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  const DxExp e = dx_exp(E, dx_sum_bits(sum), 57);  // a bit for the fold
+  __syncwarp();
+  for (int n = gl; n < H; n += G) {
+    const long long a = dx_from(r[n], e), b = dx_from(r[nx - 1 - n], e);
+    v[n] = dx_split(a + b);
+    v[nx - 1 - n] = dx_split(a - b);
+  }
+  __syncwarp();
   if (!valid) return;
-  for (int q = gl; q < nx / 2; q += G) {
-    double a = 0.0, b = 0.0;
-    for (int n = 0; n < nx; ++n) {
-      const double2 f = *reinterpret_cast<const double2*>(FT + (long long)n * nx + 2 * q);
-      a = fma(f.x, r[n], a);
-      b = fma(f.y, r[n], b);
+  const int2* __restrict__ FT = S.fwd[0];  // F^T: FT[n * N + kk] = F[kk][n]
+  double2* out = spec + (long long)S.nxs * ((j - 1) + (long long)ny * (k - 1));
+  const FxOut fo = fx_out(e.eb);
+  for (int q = gl; q < H; q += G) {
+    DxSum a, b;
+    for (int n0 = 0; n0 < H; n0 += DX_SEG) {
+      const int n1 = min(H, n0 + DX_SEG);
+#pragma unroll 4
+      for (int n = n0; n < n1; ++n) {
+        const int4 f = __ldg(reinterpret_cast<const int4*>(FT + (long long)n * nx + 2 * q));
+        const int2 s = v[n], t = v[nx - 1 - n];
+        a.add(s.x, s.y, make_int2(f.x, f.y));
+        b.add(t.x, t.y, make_int2(f.z, f.w));
+      }
+      a.fold();
+      b.fold();
     }
-    out[q] = make_double2(a, b);
+    double2 y = fx_to(i2{a.hi, b.hi}, fo, c);
+    if (fo.odd) fx_rescale(y, fo);
+    out[q] = y;
   }
 }
 
 // x inverse for a non-periodic x axis: packed modes -> G_x -> dp slots 1..nx.
 __device__ __forceinline__ void dense_x_inv_body(const SpecPlan& S, const double2* __restrict__ spec, double* dp,
-                                                 const Layout& L, double* xs, int bx) {
-  const int G = dense_x_inv_group(S.sym[0], S.nx);
+                                                 const Layout& L, double* xs, int bx, const FOne& c) {
+  const int G = dense_x_group(S.nx);
   const int grp = threadIdx.x / G, gl = threadIdx.x % G;
   const int line = bx * (128 / G) + grp;
-  const int nx = S.nx, ny = S.ny, nz = S.nz;
+  const int nx = S.nx, ny = S.ny, nz = S.nz, H = nx / 2;
   const bool valid = line < ny * nz;
   const int j = valid ? 1 + line % ny : 1, k = valid ? 1 + line / ny : 1;
-  double* X = xs + grp * nx;
+  double2* raw = reinterpret_cast<double2*>(xs + grp * nx);
+  int4* v = reinterpret_cast<int4*>(raw);  // modes 2q, 2q+1
   const double2* in = spec + (long long)S.nxs * ((j - 1) + (long long)ny * (k - 1));
-  if (valid)
-    for (int q = gl; q < nx / 2; q += G) {
-      const double2 v = in[q];
-      X[2 * q] = v.x;
-      X[2 * q + 1] = v.y;
-    }
+  unsigned m = 0;
+  for (int q = gl; q < H; q += G) {
+    const double2 x = valid ? in[q] : make_double2(0.0, 0.0);
+    m = max(m, max((unsigned)__double2hiint(x.x) << 1, (unsigned)__double2hiint(x.y) << 1));
+    raw[q] = x;
+  }
+  for (int o = G / 2; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+  const int E = dx_biased(m);
+  unsigned sum = 0;
+  for (int q = gl; q < H; q += G)
+    sum += dx_share(E, (unsigned)__double2hiint(raw[q].x) << 1) + dx_share(E, (unsigned)__double2hiint(raw[q].y) << 1);
+  for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  const DxExp e = dx_exp(E, dx_sum_bits(sum), 58);
+  for (int q = gl; q < H; q += G) {  // each lane its own entries
+    const int2 a = dx_split(dx_from(raw[q].x, e)), b = dx_split(dx_from(raw[q].y, e));
+    v[q] = make_int4(a.x, a.y, b.x, b.y);
+  }
   __syncwarp();
   if (!valid) return;
-  const double* __restrict__ GT = S.inv[0];  // G^T: GT[kk * N + n] = G[n][kk] (x = G X)
+  const int2* __restrict__ GT = S.inv[0];  // G^T: GT[kk * N + n] = G[n][kk] (x = G X)
   double* o = dp + L.at(1, j, k);
-  const int lvi = (S.sym[0] >> 4) & 3;  // bit p: the columns of parity p fold once more
-  if ((S.sym[0] & 2) && (lvi == 1 || lvi == 2)) {
-    // Row pairs (n, H-1-n), n < H/2: G[H-1-n][k] = (-1)^((k >> 1) & 1) G[n][k]
-    // on the columns of parity pf, so their partial sums F0 (k = pf mod 4)
-    // and F1 (k = pf + 2 mod 4) give both rows as F0 + F1 and F0 - F1; the
-    // other parity is summed for both rows.  Then out[r] = E_r + O_r and
-    // out[N-1-r] = E_r - O_r for r = n and H-1-n.
-    const int H = nx / 2, Q = H / 2, pf = lvi == 1 ? 0 : 1, pu = 1 - pf;
-    for (int n = gl; n < Q; n += G) {
-      const int m = H - 1 - n;
-      double f0 = 0.0, f1 = 0.0, un = 0.0, um = 0.0;
-      for (int c = 0; c < nx; c += 4) {
-        const double x0 = X[c + pf], x1 = X[c + pf + 2], y0 = X[c + pu], y1 = X[c + pu + 2];
-        f0 = fma(__ldg(GT + (long long)(c + pf) * nx + n), x0, f0);
-        f1 = fma(__ldg(GT + (long long)(c + pf + 2) * nx + n), x1, f1);
-        un = fma(__ldg(GT + (long long)(c + pu) * nx + n), y0, un);
-        un = fma(__ldg(GT + (long long)(c + pu + 2) * nx + n), y1, un);
-        um = fma(__ldg(GT + (long long)(c + pu) * nx + m), y0, um);
-        um = fma(__ldg(GT + (long long)(c + pu + 2) * nx + m), y1, um);
+  const FxOut fo = fx_out(e.eb >= kFxNonfinite / 2 ? e.eb : e.eb - S.gexp[0]);
+  for (int n = gl; n < H; n += G) {
+    DxSum ev, od;
+    for (int q0 = 0; q0 < H; q0 += DX_SEG) {
+      const int q1 = min(H, q0 + DX_SEG);
+#pragma unroll 4
+      for (int q = q0; q < q1; ++q) {
+        const int4 x = v[q];
+        ev.add(x.x, x.y, __ldg(GT + (long long)(2 * q) * nx + n));
+        od.add(x.z, x.w, __ldg(GT + (long long)(2 * q + 1) * nx + n));
       }
-      const double fn = f0 + f1, fm = f0 - f1;
-      const double en = pf ? un : fn, on = pf ? fn : un;  // even and odd sums of row n
-      const double em = pf ? um : fm, om = pf ? fm : um;  // and of row m
-      o[n] = en + on;
-      o[nx - 1 - n] = en - on;
-      o[m] = em + om;
-      o[nx - 1 - m] = em - om;
+      ev.fold();
+      od.fold();
     }
-    return;
-  }
-  if (S.sym[0] & 2) {
-    // G[N-1-n][k] = (-1)^k G[n][k]: out[n] = E + O, out[N-1-n] = E - O
-    for (int n = gl; n < nx / 2; n += G) {
-      double e = 0.0, od = 0.0;
-      for (int kk = 0; kk + 1 < nx; kk += 2) {
-        e = fma(__ldg(GT + (long long)kk * nx + n), X[kk], e);
-        od = fma(__ldg(GT + (long long)(kk + 1) * nx + n), X[kk + 1], od);
-      }
-      o[n] = e + od;
-      o[nx - 1 - n] = e - od;
-    }
-    return;
-  }
-  for (int n = gl; n < nx; n += G) {
-    double a = 0.0;
-    for (int kk = 0; kk < nx; ++kk) a = fma(__ldg(GT + (long long)kk * nx + n), X[kk], a);
-    o[n] = a;
+    double2 y = fx_to(i2{ev.hi + od.hi, ev.hi - od.hi}, fo, c);
+    if (fo.odd) fx_rescale(y, fo);
+    o[n] = y.x;
+    o[nx - 1 - n] = y.y;
   }
 }
 
 // Dense transform of complex lines along y (AXIS 1) or z (AXIS 2).  Lines are
 // numbered t = col + nxs * o (o: z for y-lines, y for z-lines) and a CTA takes
-// 16 consecutive ones, so narrow spectra fill it too; neighbouring lanes read
-// neighbouring columns (coalesced).
+// DX_LPC consecutive ones, so narrow spectra fill it too; neighbouring lanes
+// read neighbouring columns (coalesced).  DX_T threads a line.
+constexpr int DX_LPC = 8, DX_T = 16;
+__host__ __device__ constexpr size_t dense_yz_smem(int n) {
+  return (size_t)n * DX_LPC * sizeof(int4) + DX_LPC * DX_T * sizeof(unsigned);
+}
 template <int AXIS, bool FWD>
-__device__ __forceinline__ void dense_yz_body(const SpecPlan& S, double2* __restrict__ spec, double2* ls, int bx) {
-  constexpr int LPC = 16, T = 8;  // 16 lines x 8 threads per line
+__device__ __forceinline__ void dense_yz_body(const SpecPlan& S, double2* __restrict__ spec, double2* ls, int bx,
+                                              const FOne& c) {
+  constexpr int LPC = DX_LPC, T = DX_T;
   const int l = threadIdx.x % LPC, t = threadIdx.x / LPC;
   const int N = (AXIS == 1) ? S.ny : S.nz;
   const int n_other = (AXIS == 1) ? S.nz : S.ny;
@@ -231,181 +240,124 @@ __device__ __forceinline__ void dense_yz_body(const SpecPlan& S, double2* __rest
   const int o = valid ? tl / S.nxs : 0;
   const long long st = (AXIS == 1) ? (long long)S.nxs : (long long)S.nxs * S.ny;
   const long long base = (AXIS == 1) ? col + (long long)S.nxs * S.ny * o : col + (long long)S.nxs * o;
-  double2* line = ls + l;  // element n at line[n * LPC]
+  double2* raw = ls + l;  // element n at raw[n * LPC], then its integers at v[n * LPC]
+  int4* v = reinterpret_cast<int4*>(ls) + l;
+  unsigned* mx = reinterpret_cast<unsigned*>(ls + (long long)N * LPC);
   double2* g = spec + base;
-  if (valid)
-    for (int n = t; n < N; n += T) line[n * LPC] = g[(long long)n * st];
+  const int H = N / 2, He = (N + 1) / 2;  // pairs; terms of an even mode, rows of an inverse
+  unsigned m = 0;
+  for (int n = t; n < He; n += T) {  // both samples of a pair by one thread
+    const double2 a = valid ? g[(long long)n * st] : make_double2(0.0, 0.0);
+    const double2 b = valid ? g[(long long)(N - 1 - n) * st] : make_double2(0.0, 0.0);
+    m = max(max(m, (unsigned)__double2hiint(a.x) << 1), (unsigned)__double2hiint(a.y) << 1);
+    m = max(max(m, (unsigned)__double2hiint(b.x) << 1), (unsigned)__double2hiint(b.y) << 1);
+    raw[n * LPC] = a;
+    raw[(N - 1 - n) * LPC] = b;
+  }
+  mx[t * LPC + l] = m;
   __syncthreads();
-  const double* __restrict__ M = FWD ? S.fwd[AXIS] : S.inv[AXIS];  // row = output index
-  const bool sym = (S.sym[AXIS] >> (FWD ? 0 : 1)) & 1;
-  if (sym && FWD) {
-    // F[k][N-1-n] = (-1)^k F[k][n]: fold the line into s[n] = x[n] + x[N-1-n]
-    // (kept at n) and d[n] = x[n] - x[N-1-n] (kept at N-1-n); an even mode
-    // then sums F[k][n] s[n], an odd one F[k][n] d[n], over n < N/2.
-    const int H = N / 2;
-    if (valid)
-      for (int n = t; n < H; n += T) {
-        const double2 a = line[n * LPC], b = line[(N - 1 - n) * LPC];
-        line[n * LPC] = make_double2(a.x + b.x, a.y + b.y);
-        line[(N - 1 - n) * LPC] = make_double2(a.x - b.x, a.y - b.y);
-      }
-    __syncthreads();
-    const int lv1 = (S.sym[AXIS] >> 2) & 3;  // bit p: the modes of parity p fold once more
-    if (lv1 == 1 || lv1 == 2) {
-      // Second fold of branch p over its H points (sign (-1)^((k >> 1) & 1)):
-      // the even branch s (at 0..H-1) into s2 at q and d2 at H-1-q, the odd
-      // branch d (d[q] at N-1-q) into s2 at N-1-q and d2 at H+q, q < H/2.
-      const int Q = H / 2, pf = lv1 == 1 ? 0 : 1;
-      if (valid)
-        for (int q = t; q < Q; q += T) {
-          const int ia = pf ? N - 1 - q : q, ib = pf ? H + q : H - 1 - q;
-          const double2 a = line[ia * LPC], b = line[ib * LPC];
-          line[ia * LPC] = make_double2(a.x + b.x, a.y + b.y);
-          line[ib * LPC] = make_double2(a.x - b.x, a.y - b.y);
-        }
-      __syncthreads();
-      if (!valid) return;
-      // each thread takes modes 2m + pu (H terms) and 2m + pf (H/2 terms) for
-      // m = t, t + T, ..., so every thread has the same loop lengths
-      const int pu = 1 - pf;
-      for (int m = t; m < H; m += T) {
-        {
-          const int kk = 2 * m + pu;
-          const double2* src = pu ? line + (long long)(N - 1) * LPC : line;
-          const int step = pu ? -LPC : LPC;
-          const double* __restrict__ row = M + (long long)kk * N;
-          double2 acc = make_double2(0.0, 0.0);
-          for (int n = 0; n < H; ++n) {
-            const double2 v = src[n * step];
-            const double mm = __ldg(row + n);
-            acc.x = fma(mm, v.x, acc.x);
-            acc.y = fma(mm, v.y, acc.y);
-          }
-          g[(long long)kk * st] = acc;
-        }
-        {
-          const int kk = 2 * m + pf, b1 = m & 1;  // (kk >> 1) & 1
-          const double2* src;
-          int step;
-          if (pf == 0) { src = b1 ? line + (long long)(H - 1) * LPC : line; step = b1 ? -LPC : LPC; }
-          else { src = b1 ? line + (long long)H * LPC : line + (long long)(N - 1) * LPC; step = b1 ? LPC : -LPC; }
-          const double* __restrict__ row = M + (long long)kk * N;
-          double2 acc = make_double2(0.0, 0.0);
-          for (int n = 0; n < Q; ++n) {
-            const double2 v = src[n * step];
-            const double mm = __ldg(row + n);
-            acc.x = fma(mm, v.x, acc.x);
-            acc.y = fma(mm, v.y, acc.y);
-          }
-          g[(long long)kk * st] = acc;
-        }
-      }
-      return;
-    }
-    if (!valid) return;
-    for (int kk = t; kk < N; kk += T) {  // kk has the parity of t
-      const double2* src = (kk & 1) ? line + (long long)(N - 1) * LPC : line;
-      const int step = (kk & 1) ? -LPC : LPC;
-      const double* __restrict__ row = M + (long long)kk * N;
-      double2 acc = make_double2(0.0, 0.0);
-      for (int n = 0; n < H; ++n) {
-        const double2 v = src[n * step];
-        const double m = __ldg(row + n);
-        acc.x = fma(m, v.x, acc.x);
-        acc.y = fma(m, v.y, acc.y);
-      }
-      g[(long long)kk * st] = acc;
-    }
-    return;
-  }
-  const int lvi = (S.sym[AXIS] >> 4) & 3;  // bit p: the columns of parity p fold once more
-  if (sym && (lvi == 1 || lvi == 2) && N % 8 == 0) {
-    // Row pairs (n, H-1-n), n < H/2, from the second fold of the columns of
-    // parity pf (see dense_x_inv_body).  The two threads t and t^1 of a pair
-    // (lanes 16 apart) take one half of the columns each and add their sums
-    // by shuffle; every lane stays in the loop for the shuffles.
-    const int H = N / 2, Q = H / 2, pf = lvi == 1 ? 0 : 1, pu = 1 - pf;
-    const int half = t & 1, pr = t >> 1;
-    const int c0 = half ? H : 0, c1 = half ? N : H;
-    for (int n = pr; n < Q; n += T / 2) {
-      const int m = H - 1 - n;
-      const double* __restrict__ rn = M + (long long)n * N;
-      const double* __restrict__ rm = M + (long long)m * N;
-      double2 f0 = make_double2(0.0, 0.0), f1 = f0, un = f0, um = f0;
-      for (int c = c0; c < c1; c += 4) {
-        const double2 x0 = line[(c + pf) * LPC], x1 = line[(c + pf + 2) * LPC];
-        const double2 y0 = line[(c + pu) * LPC], y1 = line[(c + pu + 2) * LPC];
-        const double a0 = __ldg(rn + c + pf), a1 = __ldg(rn + c + pf + 2);
-        const double b0 = __ldg(rn + c + pu), b1 = __ldg(rn + c + pu + 2);
-        const double e0 = __ldg(rm + c + pu), e1 = __ldg(rm + c + pu + 2);
-        f0.x = fma(a0, x0.x, f0.x); f0.y = fma(a0, x0.y, f0.y);
-        f1.x = fma(a1, x1.x, f1.x); f1.y = fma(a1, x1.y, f1.y);
-        un.x = fma(b0, y0.x, un.x); un.y = fma(b0, y0.y, un.y);
-        un.x = fma(b1, y1.x, un.x); un.y = fma(b1, y1.y, un.y);
-        um.x = fma(e0, y0.x, um.x); um.y = fma(e0, y0.y, um.y);
-        um.x = fma(e1, y1.x, um.x); um.y = fma(e1, y1.y, um.y);
-      }
-      f0.x += __shfl_xor_sync(0xffffffffu, f0.x, 16); f0.y += __shfl_xor_sync(0xffffffffu, f0.y, 16);
-      f1.x += __shfl_xor_sync(0xffffffffu, f1.x, 16); f1.y += __shfl_xor_sync(0xffffffffu, f1.y, 16);
-      un.x += __shfl_xor_sync(0xffffffffu, un.x, 16); un.y += __shfl_xor_sync(0xffffffffu, un.y, 16);
-      um.x += __shfl_xor_sync(0xffffffffu, um.x, 16); um.y += __shfl_xor_sync(0xffffffffu, um.y, 16);
-      if (valid && half == 0) {
-        const double2 fn = make_double2(f0.x + f1.x, f0.y + f1.y), fm = make_double2(f0.x - f1.x, f0.y - f1.y);
-        const double2 en = pf ? un : fn, on = pf ? fn : un;  // even and odd sums of row n
-        const double2 em = pf ? um : fm, om = pf ? fm : um;  // and of row m
-        g[(long long)n * st] = make_double2(en.x + on.x, en.y + on.y);
-        g[(long long)(N - 1 - n) * st] = make_double2(en.x - on.x, en.y - on.y);
-        g[(long long)m * st] = make_double2(em.x + om.x, em.y + om.y);
-        g[(long long)(N - 1 - m) * st] = make_double2(em.x - om.x, em.y - om.y);
-      }
-    }
-    return;
-  }
-  if (sym) {
-    // G[N-1-n][k] = (-1)^k G[n][k]: even and odd partial sums of row n give
-    // out[n] = E + O and out[N-1-n] = E - O
-    if (!valid) return;
-    const int H = N / 2;
-    for (int r = t; r < H; r += T) {
-      const double* __restrict__ row = M + (long long)r * N;
-      double2 e = make_double2(0.0, 0.0), od = make_double2(0.0, 0.0);
-      for (int c = 0; c + 1 < N; c += 2) {
-        const double2 v0 = line[c * LPC], v1 = line[(c + 1) * LPC];
-        const double m0 = __ldg(row + c), m1 = __ldg(row + c + 1);
-        e.x = fma(m0, v0.x, e.x);
-        e.y = fma(m0, v0.y, e.y);
-        od.x = fma(m1, v1.x, od.x);
-        od.y = fma(m1, v1.y, od.y);
-      }
-      g[(long long)r * st] = make_double2(e.x + od.x, e.y + od.y);
-      g[(long long)(N - 1 - r) * st] = make_double2(e.x - od.x, e.y - od.y);
-    }
-    return;
-  }
-  // general N: the full matrix product, outputs k = t + T*q
-  double2 acc[16];
-  const int nq = (N + T - 1) / T;
 #pragma unroll
-  for (int q = 0; q < 16; ++q) acc[q] = make_double2(0.0, 0.0);
-  for (int n = 0; n < N; ++n) {
-    const double2 v = line[n * LPC];
-#pragma unroll
-    for (int q = 0; q < 16; ++q) {
-      if (q < nq) {
-        const int kk = t + T * q;
-        if (kk < N) {
-          const double m = __ldg(M + (long long)kk * N + n);
-          acc[q].x = fma(m, v.x, acc[q].x);
-          acc[q].y = fma(m, v.y, acc[q].y);
-        }
-      }
-    }
+  for (int q = 0; q < T; ++q) m = max(m, mx[q * LPC + l]);
+  const int E = dx_biased(m);
+  unsigned sum = 0;
+  for (int n = t; n < He; n += T) {  // of the larger component of each sample
+    const double2 a = raw[n * LPC], b = raw[(N - 1 - n) * LPC];
+    sum += dx_share(E, max((unsigned)__double2hiint(a.x) << 1, (unsigned)__double2hiint(a.y) << 1));
+    if (n < H) sum += dx_share(E, max((unsigned)__double2hiint(b.x) << 1, (unsigned)__double2hiint(b.y) << 1));
   }
+  __syncthreads();
+  mx[t * LPC + l] = sum;
+  __syncthreads();
+  sum = 0;
+#pragma unroll
+  for (int q = 0; q < T; ++q) sum += mx[q * LPC + l];
+  const DxExp e = dx_exp(E, dx_sum_bits(sum), FWD ? 57 : 58);  // a bit for the fold
+  for (int n = t; n < He; n += T) {
+    const double2 a = raw[n * LPC], b = raw[(N - 1 - n) * LPC];
+    i2 p{dx_from(a.x, e), dx_from(a.y, e)}, q{dx_from(b.x, e), dx_from(b.y, e)};
+    if (FWD && n < H) {
+      const i2 s = p + q;
+      q = p - q;
+      p = s;
+    }
+    const int2 px = dx_split(p.x), py = dx_split(p.y), qx = dx_split(q.x), qy = dx_split(q.y);
+    if (n < H) v[(N - 1 - n) * LPC] = make_int4(qx.x, qx.y, qy.x, qy.y);
+    v[n * LPC] = make_int4(px.x, px.y, py.x, py.y);
+  }
+  __syncthreads();
   if (!valid) return;
-#pragma unroll
-  for (int q = 0; q < 16; ++q) {
-    const int kk = t + T * q;
-    if (q < nq && kk < N) g[(long long)kk * st] = acc[q];
+  const int2* __restrict__ M = FWD ? S.fwd[AXIS] : S.inv[AXIS];  // row = output index
+  if (FWD) {
+    const FxOut fo = fx_out(e.eb);
+    // two modes of one parity at a time: kk and kk + T
+    for (int kk = t; kk < N; kk += 2 * T) {
+      const bool odd = kk & 1, two = kk + T < N;
+      const int4* src = odd ? v + (long long)(N - 1) * LPC : v;
+      const int step = odd ? -LPC : LPC, terms = odd ? H : He;
+      const int2* __restrict__ r0 = M + (long long)kk * N;
+      const int2* __restrict__ r1 = M + (long long)(two ? kk + T : kk) * N;
+      DxSum a, b, p, q;
+      for (int n0 = 0; n0 < terms; n0 += DX_SEG) {
+        const int n1 = min(terms, n0 + DX_SEG);
+#pragma unroll 4
+        for (int n = n0; n < n1; ++n) {
+          const int4 x = src[n * step];
+          const int2 w0 = __ldg(r0 + n), w1 = __ldg(r1 + n);
+          a.add(x.x, x.y, w0);
+          b.add(x.z, x.w, w0);
+          p.add(x.x, x.y, w1);
+          q.add(x.z, x.w, w1);
+        }
+        a.fold();
+        b.fold();
+        p.fold();
+        q.fold();
+      }
+      double2 y = fx_to(i2{a.hi, b.hi}, fo, c);
+      if (fo.odd) fx_rescale(y, fo);
+      g[(long long)kk * st] = y;
+      if (two) {
+        y = fx_to(i2{p.hi, q.hi}, fo, c);
+        if (fo.odd) fx_rescale(y, fo);
+        g[(long long)(kk + T) * st] = y;
+      }
+    }
+  } else {
+    const FxOut fo = fx_out(e.eb >= kFxNonfinite / 2 ? e.eb : e.eb - S.gexp[AXIS]);
+    for (int n = t; n < He; n += T) {
+      const int2* __restrict__ row = M + (long long)n * N;
+      DxSum ex, ey, ox, oy;
+      for (int q0 = 0; q0 < N; q0 += DX_SEG) {
+        const int q1 = min(N, q0 + DX_SEG);  // q0 is even
+#pragma unroll 2
+        for (int q = q0; q + 1 < q1; q += 2) {
+          const int4 x = v[q * LPC], z = v[(q + 1) * LPC];
+          const int2 w0 = __ldg(row + q), w1 = __ldg(row + q + 1);
+          ex.add(x.x, x.y, w0);
+          ey.add(x.z, x.w, w0);
+          ox.add(z.x, z.y, w1);
+          oy.add(z.z, z.w, w1);
+        }
+        if ((q1 - q0) & 1) {  // the last mode of an odd N
+          const int4 x = v[(q1 - 1) * LPC];
+          const int2 w0 = __ldg(row + q1 - 1);
+          ex.add(x.x, x.y, w0);
+          ey.add(x.z, x.w, w0);
+        }
+        ex.fold();
+        ey.fold();
+        ox.fold();
+        oy.fold();
+      }
+      double2 y = fx_to(i2{ex.hi + ox.hi, ey.hi + oy.hi}, fo, c);
+      if (fo.odd) fx_rescale(y, fo);
+      g[(long long)n * st] = y;
+      if (n < H) {
+        y = fx_to(i2{ex.hi - ox.hi, ey.hi - oy.hi}, fo, c);
+        if (fo.odd) fx_rescale(y, fo);
+        g[(long long)(N - 1 - n) * st] = y;
+      }
+    }
   }
 }
 
@@ -583,14 +535,14 @@ __global__ void __launch_bounds__(128) dense_x_fwd_kernel(SpecPlan S, DivArgs d,
   dense_x_fwd_body(S, d, spec, xs_fwd, blockIdx.x);
 }
 __global__ void __launch_bounds__(128) dense_x_inv_kernel(SpecPlan S, const double2* __restrict__ spec, double* dp,
-                                                          Layout L) {
+                                                          Layout L, FOne c) {
   extern __shared__ __align__(16) double xs_inv[];
-  dense_x_inv_body(S, spec, dp, L, xs_inv, blockIdx.x);
+  dense_x_inv_body(S, spec, dp, L, xs_inv, blockIdx.x, c);
 }
 template <int AXIS, bool FWD>
-__global__ void __launch_bounds__(128) dense_yz_kernel(SpecPlan S, double2* __restrict__ spec) {
+__global__ void __launch_bounds__(128) dense_yz_kernel(SpecPlan S, double2* __restrict__ spec, FOne c) {
   extern __shared__ __align__(16) double2 ls_yz[];
-  dense_yz_body<AXIS, FWD>(S, spec, ls_yz, blockIdx.x);
+  dense_yz_body<AXIS, FWD>(S, spec, ls_yz, blockIdx.x, c);
 }
 
 template <int AXIS, bool PACKED>
@@ -856,9 +808,10 @@ __global__ void __launch_bounds__(128) spec_batch_kernel(const BatchSpecArgs* __
     // memory would be reloaded after every barrier of the passes)
     const BatchSpecArgs& a = tab[w.sub];
     if (PASS == 0) dense_x_fwd_body(a.S, a.d, a.spec, sm_b, w.bx);
-    if (PASS == 1) dense_x_inv_body(a.S, a.spec, a.dp, a.L, sm_b, w.bx);
-    if (PASS == 2) dense_yz_body<1, true>(a.S, a.spec, reinterpret_cast<double2*>(sm_b), w.bx);
-    if (PASS == 3) dense_yz_body<1, false>(a.S, a.spec, reinterpret_cast<double2*>(sm_b), w.bx);
+    const FOne c{a.d.one, a.d.mzero};
+    if (PASS == 1) dense_x_inv_body(a.S, a.spec, a.dp, a.L, sm_b, w.bx, c);
+    if (PASS == 2) dense_yz_body<1, true>(a.S, a.spec, reinterpret_cast<double2*>(sm_b), w.bx, c);
+    if (PASS == 3) dense_yz_body<1, false>(a.S, a.spec, reinterpret_cast<double2*>(sm_b), w.bx, c);
     if (PASS == 4) tri_twist_body<2, true>(a.S, a.spec, sm_b, w.bx);
     __syncthreads();
   }
@@ -954,10 +907,10 @@ void spec_pass_grid(int pass, const SpecPlan& S, int& gx, int& gy) {
   if ((pass == 0 || pass == 1) && S.dct_x) gx = (S.ny * S.nz + 2 * batch_dct_lpc(S.nx) - 1) / (2 * batch_dct_lpc(S.nx));
   else if ((pass == 2 || pass == 3) && S.dct_y) gx = (S.nxs * S.nz + batch_dct_lpc(S.ny) - 1) / batch_dct_lpc(S.ny);
   else if (pass == 0 || pass == 1) {
-    const int per = 128 / (pass == 0 ? dense_x_group(S.nx) : dense_x_inv_group(S.sym[0], S.nx));
+    const int per = 128 / dense_x_group(S.nx);
     gx = (S.ny * S.nz + per - 1) / per;
   }
-  else if (pass == 2 || pass == 3) gx = (S.nxs * S.nz + 15) / 16;  // dense_yz_body: 16 lines per item
+  else if (pass == 2 || pass == 3) gx = (S.nxs * S.nz + DX_LPC - 1) / DX_LPC;
   else gx = (S.nxs * S.ny + 63) / 64;  // tri_twist_body: 64 lines per item
 }
 
@@ -967,9 +920,8 @@ size_t spec_pass_smem(int pass, const SpecPlan& S) {
     return (size_t)S.nx * L * sizeof(i2) + L * (S.nx + 1) * sizeof(double2) + 128 * sizeof(FxExp);
   }
   if ((pass == 2 || pass == 3) && S.dct_y) return (size_t)S.ny * batch_dct_lpc(S.ny) * sizeof(i2) + 128 * sizeof(FxExp);
-  if (pass == 0) return (size_t)(128 / dense_x_group(S.nx)) * S.nx * sizeof(double);
-  if (pass == 1) return (size_t)(128 / dense_x_inv_group(S.sym[0], S.nx)) * S.nx * sizeof(double);
-  if (pass == 2 || pass == 3) return (size_t)S.ny * 16 * sizeof(double2);
+  if (pass == 0 || pass == 1) return (size_t)(128 / dense_x_group(S.nx)) * S.nx * sizeof(double);
+  if (pass == 2 || pass == 3) return dense_yz_smem(S.ny);
   return (size_t)S.nz * TRI_T * sizeof(double) * 2;
 }
 
@@ -1002,57 +954,40 @@ cudaError_t launch_spec_batch(int pass, bool dct, const BatchSpecArgs* tab, cons
 
 cudaError_t launch_dense_x(bool fwd, const SpecPlan& S, const DivArgs& d, double2* spec, double* dp, const Layout& L,
                            cudaStream_t st) {
-  const int lines = S.ny * S.nz, per = 128 / (fwd ? dense_x_group(S.nx) : dense_x_inv_group(S.sym[0], S.nx));
+  const int lines = S.ny * S.nz, per = 128 / dense_x_group(S.nx);
   const size_t sm = (size_t)per * S.nx * sizeof(double);
   if (fwd) dense_x_fwd_kernel<<<(lines + per - 1) / per, 128, sm, st>>>(S, d, spec);
-  else dense_x_inv_kernel<<<(lines + per - 1) / per, 128, sm, st>>>(S, spec, dp, L);
+  else dense_x_inv_kernel<<<(lines + per - 1) / per, 128, sm, st>>>(S, spec, dp, L, FOne{1.0, -0.0});
   return cudaGetLastError();
 }
 
-int dense_symmetry(int n, const std::vector<double>& F, const std::vector<double>& G) {
-  if (n < 2 || n % 2) return 0;
-  double fm = 0.0, gm = 0.0;
-  for (double x : F) fm = std::fmax(fm, std::fabs(x));
-  for (double x : G) gm = std::fmax(gm, std::fabs(x));
-  bool fs = true, gs = true;
-  for (int r = 0; r < n && (fs || gs); ++r)
-    for (int q = 0; q < n; ++q) {
-      const double sg_r = (r & 1) ? -1.0 : 1.0, sg_q = (q & 1) ? -1.0 : 1.0;
-      if (std::fabs(F[(size_t)r * n + (n - 1 - q)] - sg_r * F[(size_t)r * n + q]) > 4e-16 * fm) fs = false;
-      if (std::fabs(G[(size_t)(n - 1 - r) * n + q] - sg_q * G[(size_t)r * n + q]) > 4e-16 * gm) gs = false;
-    }
-  int bits = (fs ? 1 : 0) | (gs ? 2 : 0);
-  // Second level: within the modes of one parity, over the first H = n/2
-  // points, F[k][H-1-q] = s_k F[k][q] and G[H-1-q][k] = s_k G[q][k] with
-  // s_k = (-1)^((k >> 1) & 1).  DCT-II has it on its even modes (a half-size
-  // DCT-II), DST-II on its odd ones.
-  const int H = n / 2;
-  if (H % 2 == 0) {
-    bool f1[2] = {fs, fs}, g1[2] = {gs, gs};
-    for (int k = 0; k < n; ++k) {
-      const double sg = ((k >> 1) & 1) ? -1.0 : 1.0;
-      for (int q = 0; q < H; ++q) {
-        if (std::fabs(F[(size_t)k * n + (H - 1 - q)] - sg * F[(size_t)k * n + q]) > 4e-16 * fm) f1[k & 1] = false;
-        if (std::fabs(G[(size_t)(H - 1 - q) * n + k] - sg * G[(size_t)q * n + k]) > 4e-16 * gm) g1[k & 1] = false;
-      }
-    }
-    bits |= (f1[0] ? 4 : 0) | (f1[1] ? 8 : 0) | (g1[0] ? 16 : 0) | (g1[1] ? 32 : 0);
+int q54_table(std::vector<double>& M) {
+  double m = 0.0;
+  for (double x : M) m = std::fmax(m, std::fabs(x));
+  int e = 0;
+  if (m > 0.0) (void)std::frexp(m, &e);  // m in [2^(e-1), 2^e)
+  if (m == std::ldexp(1.0, e - 1)) --e;  // an exact power of two is 1 in its own units
+  for (double& x : M) {
+    const long long q = std::llrint(std::ldexp(x, 54 - e));
+    const int h = (int)((q + (1ll << 26)) >> 27);
+    const int2 w = make_int2(h, (int)(q - ((long long)h << 27)));
+    std::memcpy(&x, &w, sizeof(w));
   }
-  return bits;
+  return -e;
 }
 
 cudaError_t launch_dense_yz(int axis, bool fwd, const SpecPlan& S, double2* spec, cudaStream_t st) {
   const int N = axis == 1 ? S.ny : S.nz;
   if (N > 512) return cudaErrorInvalidValue;
-  // 16 lines of N complex values staged in shared memory: 32 KB at N = 128,
-  // 128 KB at 512 (past the 48 KB default: opt in)
-  const size_t sm = (size_t)N * 16 * sizeof(double2);
-  dim3 grid((S.nxs * (axis == 1 ? S.nz : S.ny) + 15) / 16);
+  // DX_LPC lines of N complex values staged in shared memory: 64 KB at N = 512 (past the 48 KB
+  // default: opt in)
+  const size_t sm = dense_yz_smem(N);
+  dim3 grid((S.nxs * (axis == 1 ? S.nz : S.ny) + DX_LPC - 1) / DX_LPC);
   auto kern = (axis == 1) ? (fwd ? dense_yz_kernel<1, true> : dense_yz_kernel<1, false>)
                           : (fwd ? dense_yz_kernel<2, true> : dense_yz_kernel<2, false>);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
-  kern<<<grid, 128, sm, st>>>(S, spec);
+  kern<<<grid, DX_LPC * DX_T, sm, st>>>(S, spec, FOne{1.0, -0.0});
   return cudaGetLastError();
 }
 

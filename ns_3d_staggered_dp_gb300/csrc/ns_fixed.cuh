@@ -122,6 +122,16 @@ __device__ __forceinline__ long long fx_from(double d, int E) {
   const long long v = (long long)((m << (B - 53)) >> s), sg = (long long)(hi >> 31);
   return (v ^ sg) - sg;
 }
+// The same, rounded (half away from zero).
+template <int B>
+__device__ __forceinline__ long long fx_round(double d, int E) {
+  const int hi = __double2hiint(d);
+  const unsigned long long m = ((unsigned long long)(unsigned)((hi & 0xfffff) | 0x100000) << 32) |
+                               (unsigned)__double2loint(d);
+  const unsigned s = min((unsigned)(E - ((hi >> 20) & 0x7ff)), 63u);
+  const long long v = (long long)(((m << (B - 53)) + ((1ull << s) >> 1)) >> s), sg = (long long)(hi >> 31);
+  return (v ^ sg) - sg;
+}
 // The block's integers and its eb.  Blocks of very large or very small
 // values (where the exponents of the way back could leave a double's range)
 // are scaled by a power of two first; values below 2^-64 of the block's

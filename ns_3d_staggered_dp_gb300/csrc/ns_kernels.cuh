@@ -260,9 +260,9 @@ struct FftPlan {
   int dp_unaligned;       // 1: dp slot pairs (2m+1, 2m+2) are not 16-byte aligned (scalar stores)
   int nxs;                // spectrum row length: nx/2+1 (periodic x) or nx/2 (packed wall x)
   int kind[3];            // 0: FFT axis, 1: dense transform axis, 2: tridiagonal solve axis (a wall)
-  const double* fwd[3];   // dense forward matrices (x: F^T [n][k]; y, z: F [k][n])
-  const double* inv[3];   // dense inverse matrices (x: G^T [k][n]; y, z: G [n][k])
-  int sym[3];             // bit 0: F[k][N-1-n] = (-1)^k F[k][n]; bit 1: G[N-1-n][k] = (-1)^k G[n][k]
+  const int2* fwd[3];     // dense forward matrices (x: F^T [n][k]; y, z: F [k][n]), q54_table entries
+  const int2* inv[3];     // dense inverse matrices (x: G^T [k][n]; y, z: G [n][k]), times 2^gexp
+  int gexp[3];
   // A dense y axis of power-of-two length 32..512 with pbc 2 or 3 transformed through an FFT
   // (Makhoul) instead of the dense products (session plans; ns_fft.cu dct_y_kernel):
   int dct_y;              // 0: dense products; 2 or 3: the pressure code of the FFT-based transform
@@ -397,9 +397,10 @@ cudaError_t launch_poisson_inv_x(const FftPlan& P, const DivArgs& d, double2* sp
                                  cudaStream_t st, const Marker& mk, int k0, int k1);
 cudaError_t launch_poisson_inv(const FftPlan& P, const DivArgs& d, double2* spec, double* dp, const Layout& L,
                                cudaStream_t st, const Marker& mk, int k0, int k1);
-// Symmetry bits of a dense transform pair of even size n (sym in FftPlan),
-// checked entry by entry on the host (ns_dct.cu).
-int dense_symmetry(int n, const std::vector<double>& F, const std::vector<double>& G);
+// A dense transform matrix in place as fixed-point entries: M 2^e (the largest
+// magnitude in (1/2, 1]) in units of 2^-54, split at bit 27 with a signed low
+// part (int2 in each double's storage); returns e.
+int q54_table(std::vector<double>& M);
 // The cyclic z solve of an all-periodic plan (ns_cyclic.cu): the size of its
 // tables, their construction (sets P.cyc_*; eig_x, eig_o, cyc_h2, cyc_rs set
 // before), and the solve of every z line of the spectrum in place.
@@ -413,12 +414,6 @@ __host__ __device__ __forceinline__ int dense_x_group(int nx) {
   int g = 1;
   while (g < h && g < 32) g <<= 1;
   return g;
-}
-// The x inverse takes row pairs (n, H-1-n) when its matrix folds twice
-// (sym bits 1 and 4 or 5), so its groups cover nx/4 lanes.
-__host__ __device__ __forceinline__ int dense_x_inv_group(const int sym, const int nx) {
-  const int lvi = (sym >> 4) & 3;
-  return ((sym & 2) && (lvi == 1 || lvi == 2)) ? dense_x_group(nx / 2) : dense_x_group(nx);
 }
 // Dense passes (ns_dct.cu): x forward/inverse, y/z forward/inverse.
 cudaError_t launch_dense_x(bool fwd, const SpecPlan& S, const DivArgs& d, double2* spec, double* dp, const Layout& L,

@@ -203,3 +203,21 @@ def test_sweeps_for_every_halo(n, bc, alpha, closure):
         assert rel_l2(g[k][sl], parts[k][sl]) < 1e-13, k
     for k in "uvw":
         assert rel_l2(out[k], getattr(ref, k)) < 1e-10, k
+
+
+# --- the dense wall transforms ------------------------------------------------------------------
+DENSE = [((16, m, 9), b) for m in (5, 8, 15, 16, 17, 31, 75, 100, 127, 129, 200, 257, 300) for b in (2, 3, 4)]
+DENSE += [((m, 8, 9), b) for m in (6, 16, 18, 34, 90, 130, 256, 320) for b in (2, 3, 4)]
+
+
+@pytest.mark.parametrize("n,pbc", DENSE)
+def test_dense_lengths(n, pbc):
+    """Odd and even lengths on both sides of the partial sums' length, every pressure code; the routine
+    tolerance, and an extreme magnitude."""
+    rng = np.random.default_rng(sum(n) + pbc)
+    rhs = rng.standard_normal(n)
+    rhs -= rhs.mean()
+    ref = _oracle(n, (pbc,) * 3, rhs)
+    assert rel_l2(_solve(n, (pbc,) * 3, rhs), ref) < 1e-12
+    two = 2.0 ** 960
+    assert rel_l2(_solve(n, (pbc,) * 3, rhs * two) / two, ref) < 1e-12
