@@ -150,7 +150,7 @@ __device__ __forceinline__ int fx_block(double (&d)[N], long long (&v)[N]) {
   }
   const int Ec = max(E, 64);
 #pragma unroll
-  for (int i = 0; i < N; ++i) v[i] = fx_from<B>(d[i], Ec);
+  for (int i = 0; i < N; ++i) v[i] = fx_round<B>(d[i], Ec);
   return E == 0x7ff ? kFxNonfinite : Ec - 1022 - B - adj;
 }
 // The same for complex values.
