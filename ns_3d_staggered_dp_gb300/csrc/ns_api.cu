@@ -714,7 +714,7 @@ int enqueue_poisson(ns_handle* h, const double* rhs = nullptr) {
   const DivArgs d = div_args(h, rhs);
   NS_CUDA(h, launch_fft_poisson(h->plan, d, h->spec, h->dp, h->L, h->stream, marker(h)));
   NS_CUDA(h, launch_pr_bc(h->L, h->dp, h->faces[0], c.pbc, h->dx, h->dy, h->dz, h->stream));
-  mark(h, "pr_bc", 3);
+  mark(h, "pr_bc");
   return NS_OK;
 }
 
@@ -742,7 +742,7 @@ int enqueue_viscous(ns_handle* h, bool adi_xy_done) {
     }
   } else {
     NS_CUDA(h, launch_vel_bc(h->L, h->us, h->vs, h->ws, h->faces[0], c.bc, h->stream));
-    mark(h, "vel_bc", 3);
+    mark(h, "vel_bc");
   }
   return NS_OK;
 }

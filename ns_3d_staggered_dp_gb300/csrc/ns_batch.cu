@@ -483,10 +483,10 @@ cudaError_t launch_stage_kernel(ns_batch* b, int set, int stage, bool first, cud
         break;
       case ST_VBC_X: case ST_VBC_Y: case ST_VBC_Z:  // AB2-CN: the ADI sweeps take these slots
         if (c.scheme == NS_AB2_CN) e = launch_adi_batch(stage - ST_VBC_X, b->d_adi, p, cnt, grid, st);
-        else e = launch_bc_batch(stage - ST_VBC_X, false, b->d_bc, p, cnt, grid, st);
+        else e = launch_bc_batch(false, b->d_bc, p, cnt, grid, st);
         break;
       case ST_PBC_X: case ST_PBC_Y: case ST_PBC_Z:
-        e = launch_bc_batch(stage - ST_PBC_X, true, b->d_bc, p, cnt, grid, st);
+        e = launch_bc_batch(true, b->d_bc, p, cnt, grid, st);
         break;
       case ST_XF: case ST_YF: case ST_TRI: case ST_YI: case ST_XI: {
         const int pass = pass_of[stage - ST_XF];
@@ -1040,10 +1040,13 @@ int ns_batch_create(const ns_batch_config* cfg, const ns_subdomain* subs, int n,
           for (int f = 0; f < 3; ++f)
             for (int q = 0; q < (nl + kAdiBatchLines - 1) / kAdiBatchLines; ++q) v.push_back(BatchItem{i, q, f, 0});
         } else {
-          add1(chunks(plane_count(L, stage - ST_VBC_X)), 0);
+          if (stage == ST_VBC_X)  // the three passes in one launch
+            for (int f = 0; f < 3; ++f)
+              for (int q = 0; q < chunks(fill_count(L)); ++q) v.push_back(BatchItem{i, q, f, 0});
         }
         break;
-      case ST_PBC_X: case ST_PBC_Y: case ST_PBC_Z: add1(chunks(plane_count(L, stage - ST_PBC_X)), 0); break;
+      case ST_PBC_X: add1(chunks(fill_count(L)), 0); break;  // likewise
+      case ST_PBC_Y: case ST_PBC_Z: break;
       case ST_XF: case ST_YF: case ST_TRI: case ST_YI: case ST_XI: {
         const int pass_of[5] = {0, 2, 4, 3, 1};
         int gx, gy;

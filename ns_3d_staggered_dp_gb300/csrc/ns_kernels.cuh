@@ -143,12 +143,12 @@ struct FaceSet {
   FacePlanes ax[3];
 };
 
-// vel_bc_staggered (NS_functions.f90:213-310), one axis pass.
+// vel_bc_staggered (NS_functions.f90:213-310).
 cudaError_t launch_vel_bc(const Layout& L, double* us, double* vs, double* ws, const FaceSet& F, const int bc[3],
                           cudaStream_t st);
 // Face slot 0 of each periodic axis's face field from face n (after a state load).
 cudaError_t launch_extra_slots(const Layout& L, double* u, double* v, double* w, const int bc[3], cudaStream_t st);
-// pr_bc_staggered (NS_functions.f90:1403-1464), the three axis passes.
+// pr_bc_staggered (NS_functions.f90:1403-1464).
 cudaError_t launch_pr_bc(const Layout& L, double* dp, const FaceSet& F, const int pbc[3], double dx, double dy,
                          double dz, cudaStream_t st);
 // The same fill in parts: the x and y passes over the planes z in [k0, k1),
@@ -172,9 +172,11 @@ struct BatchBcArgs {
   int bc[3], pbc[3];
   double h[3];
 };
-// One axis pass of vel_bc_staggered (pr false) or pr_bc_staggered (pr true)
-// over the items (sub, 256-element chunk bx of the plane).
-cudaError_t launch_bc_batch(int axis, bool pr, const BatchBcArgs* tab, const BatchItem* items, int n_items, int grid,
+// Filled slots of one field of a box (a thread each).
+long long fill_count(const Layout& L);
+// vel_bc_staggered (pr false; by: the field) or pr_bc_staggered (pr true) over
+// the items (sub, 256-slot chunk bx).
+cudaError_t launch_bc_batch(bool pr, const BatchBcArgs* tab, const BatchItem* items, int n_items, int grid,
                             cudaStream_t st);
 
 // ---------------------------------------------------------------------------

@@ -221,3 +221,34 @@ def test_dense_lengths(n, pbc):
     assert rel_l2(_solve(n, (pbc,) * 3, rhs), ref) < 1e-12
     two = 2.0 ** 960
     assert rel_l2(_solve(n, (pbc,) * 3, rhs * two) / two, ref) < 1e-12
+
+
+# --- the one-launch fills ---------------------------------------------------
+@pytest.mark.parametrize("bc", [(1, 1, 1), (1, 2, 1), (1, 1, 4), (1, 4, 2), (2, 2, 2), (4, 2, 4), (4, 4, 4)])
+def test_fills_of_every_code(bc):
+    """vel_bc_staggered and the pressure ghosts with non-zero faces, edges and corners included."""
+    from ns_3d_staggered_dp_gb300 import Session, make_config
+
+    n = (32, 16, 16)
+    rng = np.random.default_rng(sum(bc))
+    for pw in (2, 3, 4):
+        pbc = tuple(1 if b == 1 else pw for b in bc)
+        cfg = O.Config(*n, 3.0, 1.0, 2.0, bc=bc, pbc=pbc)
+        f = O.Faces.zeros(*n)
+        for k in f.d:
+            f.d[k] = rng.standard_normal(f.d[k].shape)
+        sh = O.State.zeros(*n)
+        us, vs, ws = (rng.standard_normal(a.shape) for a in (sh.u, sh.v, sh.w))
+        ref = [us.copy(), vs.copy(), ws.copy()]
+        O.vel_bc_staggered(*ref, f, *bc)
+        rhs = rng.standard_normal(n)
+        with Session(make_config(*n, lx=3.0, ly=1.0, lz=2.0, bc=bc, pbc=pbc)) as s:
+            s.set_faces(f.d)
+            got = s.vel_bc(us, vs, ws)
+            dp = s.poisson(rhs)
+        for a, b in zip(got, ref):
+            assert np.array_equal(a, b)
+        want = np.zeros(dp.shape)
+        want[1:-1, 1:-1, 1:-1] = dp[1:-1, 1:-1, 1:-1]
+        O.pr_bc_staggered(want, f, pbc, *cfg.h)
+        np.testing.assert_allclose(dp, want, rtol=0, atol=4e-16 * max(1.0, np.abs(want).max()))
