@@ -236,7 +236,7 @@ int ns_correct(ns_handle* h, const double* u_star, const double* v_star, const d
  *            the interior is the solution (zero mean) and the ghosts are
  *            the periodic copies;
  *   stream : cudaStream_t the work is enqueued on (NULL: legacy stream).
- * All scratch (half spectrum, twiddles, 1/lambda; 4 MiB) is one static
+ * All scratch (half spectrum, twiddles, mode constants; 4 MiB) is one static
  * device array held by every device that loads the library.  Grids are
  * limited to powers of two in [16, 64] per axis (NS_ERR_SHAPE otherwise).
  * The first call on a device looks up the array's device address

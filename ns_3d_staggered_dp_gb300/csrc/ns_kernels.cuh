@@ -291,15 +291,11 @@ struct FftPlan {
   double* sing_cm;        // session solve from a table: global scratch (2 N TRI_T doubles) of the
                           // singular line's multipliers (the batch keeps them in shared memory)
   int tri_tw;             // 1: tri_m holds the twisted multipliers, solved two lanes per line
-  // All-periodic boxes: the z stage as cyclic tridiagonal line solves (ns_cyclic.cu)
-  // instead of z FFT * 1/lambda * z IFFT.  Tables per (kx, ky) mode, laid out like the
-  // spectrum: T's multipliers, w = rs T^-1 e0, q = T^-1 u; per mode (1/c, SM denominator).
+  // All-periodic boxes: the z stage as cyclic line solves (ns_cyclic.cu) instead of
+  // z FFT * 1/lambda * z IFFT; two entries of constants per (kx, ky) mode (cyc_mode).
   int zcyc;
-  const double* cyc_m;
-  const double* cyc_w;
-  const double* cyc_q;
-  const double2* cyc_s;
-  const double* cyc_v;    // the singular (0, 0) line's solution mean, as a functional of its data
+  const double2* cyc_t;
+  const double* cyc_h;    // rho^8
   double cyc_rs;          // h_z^2 * scale * nz
   double cyc_h2;          // h_z^2
   double mod_lo[3], mod_hi[3];        // pr_bc_staggered_modify_rhs coefficients per axis
@@ -365,6 +361,14 @@ using SpecPlan = FftPlan;
 // The FFT-based y transform of a packed-x plan with dct_y set (ns_fft.cu).
 cudaError_t launch_dct_y(bool fwd, const FftPlan& P, double2* spec, cudaStream_t st);
 struct DivArgs;
+// Constants of the cyclic solve of a mode with sigma = -h_z^2 (lambda_x + lambda_y) on nz unknowns:
+// a = (rho, rho^16), b = (1 / (1 - rho^nz), -rho rs), h = rho^8.  The singular mode's (sigma 0) are 1, 1, inf, -rs.
+__device__ __forceinline__ void cyc_mode(double sigma, int nz, double rs, double2& a, double2& b, double& h) {
+  const double th = 2.0 * asinh(0.5 * sqrt(sigma)), rho = exp(-th);
+  h = exp(-8.0 * th);
+  a = make_double2(rho, exp(-16.0 * th));
+  b = make_double2(-1.0 / expm1(-nz * th), -rho * rs);
+}
 // The FFT-based x transforms of a plan with dct_x set (ns_fft.cu): divergence
 // (+ pressure-BC terms), or d.rhs when given, -> packed modes, and packed
 // modes -> dp slots 1..nx.
@@ -404,7 +408,7 @@ cudaError_t launch_poisson_inv(const FftPlan& P, const DivArgs& d, double2* spec
 // part (int2 in each double's storage); returns e.
 int q54_table(std::vector<double>& M);
 // The cyclic z solve of an all-periodic plan (ns_cyclic.cu): the size of its
-// tables, their construction (sets P.cyc_*; eig_x, eig_o, cyc_h2, cyc_rs set
+// table, its construction (sets P.cyc_t; eig_x, eig_o, cyc_h2, cyc_rs set
 // before), and the solve of every z line of the spectrum in place.
 size_t cyc_table_doubles(const FftPlan& P);
 cudaError_t launch_cyc_table(FftPlan& P, double* buf, cudaStream_t st);

@@ -1,5 +1,5 @@
 // ns_poisson_fft_noalloc: the periodic FFT pressure Poisson solve with all of
-// its scratch (half spectrum, twiddle tables, inverse eigenvalues) in one
+// its scratch (half spectrum, twiddle and mode tables) in one
 // file-scope device array, for callers that must not allocate device memory.
 //
 // Who cannot allocate: solvers embedded in a host application whose device
@@ -49,34 +49,28 @@ constexpr int kMaxDevices = 64;
 std::mutex g_setup_mutex;
 double* g_scratch_addr[kMaxDevices] = {nullptr};
 
-// Twiddles W_N^m = exp(-2 pi i m/N) of the four transforms and the inverse
-// eigenvalues 1/(2 N lambda) (lambda as big_periodic_3D.f90:242-255; mean mode 0).
-__global__ void noalloc_tables(int4* tw, int M, int nx, int ny, int nz, double* inv_lam, double dx, double dy,
-                               double dz) {
+// Twiddles W_N^m = exp(-2 pi i m/N) of the three transforms, and the constants
+// of the cyclic z solve of every (kx, ky) mode (lambda as
+// big_periodic_3D.f90:242-255).
+__global__ void noalloc_tables(int4* tw, int M, int nx, int ny, int nz, double2* cyc, double dx, double dy, double dz,
+                               double rs) {
   const int nxh = M + 1;
-  const int ntw = M + (M / 2 + 1) + ny + nz;
-  const long long nl = (long long)nxh * ny * nz;
-  const double scale = 1.0 / (2.0 * (double)nx * (double)ny * (double)nz);
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < ntw + nl;
-       t += (long long)gridDim.x * blockDim.x) {
-    if (t < ntw) {
-      int m = (int)t, N;
-      if (m < M) { N = M; }
-      else if ((m -= M) < M / 2 + 1) { N = nx; }
-      else if ((m -= M / 2 + 1) < ny) { N = ny; }
-      else { m -= ny; N = nz; }
-      double s, c;
-      sincospi(2.0 * (double)m / (double)N, &s, &c);
-      const long long re = __double2ll_rn(c * 0x1p60), im = __double2ll_rn(-s * 0x1p60), low = (1ll << 30) - 1;
-      tw[t] = make_int4((int)(re >> 30), (int)(re & low), (int)(im >> 30), (int)(im & low));  // as q60_entry
-    } else {
-      const long long q = t - ntw;
-      const int i = (int)(q % nxh), j = (int)((q / nxh) % ny), k = (int)(q / ((long long)nxh * ny));
-      const double pi = 3.1415926535897932;
-      const double sx = sin(pi * i / nx) / dx, sy = sin(pi * j / ny) / dy, sz = sin(pi * k / nz) / dz;
-      const double lam = -4.0 * ((sx * sx + sy * sy) + sz * sz);
-      inv_lam[q] = (i == 0 && j == 0 && k == 0) ? 0.0 : scale / lam;
-    }
+  const int ntw = M + (M / 2 + 1) + ny;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < ntw) {
+    int m = t, N;
+    if (m < M) { N = M; }
+    else if ((m -= M) < M / 2 + 1) { N = nx; }
+    else { m -= M / 2 + 1; N = ny; }
+    double s, c;
+    sincospi(2.0 * (double)m / (double)N, &s, &c);
+    const long long re = __double2ll_rn(c * 0x1p60), im = __double2ll_rn(-s * 0x1p60), low = (1ll << 30) - 1;
+    tw[t] = make_int4((int)(re >> 30), (int)(re & low), (int)(im >> 30), (int)(im & low));  // as q60_entry
+  } else if (t - ntw < nxh * ny) {
+    const int q = t - ntw, i = q % nxh, j = q / nxh;
+    const double sx = sinpi((double)i / nx) / dx, sy = sinpi((double)j / ny) / dy;
+    cyc_mode(4.0 * dz * dz * (sx * sx + sy * sy), nz, rs, cyc[2 * q], cyc[2 * q + 1],
+             reinterpret_cast<double*>(cyc + 2 * nxh * ny)[q]);
   }
 }
 
@@ -99,9 +93,9 @@ extern "C" int ns_poisson_fft_noalloc(const double* rhs_dev, double* dp_dev, int
   }
   const int M = nx / 2, nxh = M + 1;
   const size_t n_spec = (size_t)nxh * ny * nz * 2;          // doubles of the half spectrum
-  const size_t n_lam = (size_t)nxh * ny * nz;
-  const size_t n_tw = (size_t)(M + M / 2 + 1 + ny + nz) * 2;
-  if (n_spec + n_lam + n_tw > kNoAllocScratchDoubles) return NS_ERR_SHAPE;
+  const size_t n_cyc = ((size_t)nxh * ny * 5 + 1) & ~size_t(1);
+  const size_t n_tw = (size_t)(M + M / 2 + 1 + ny) * 2;
+  if (n_spec + n_cyc + n_tw > kNoAllocScratchDoubles) return NS_ERR_SHAPE;
 
   // An error left by the caller's earlier work is not ours to consume: report it, launch nothing.
   if (cudaPeekAtLastError() != cudaSuccess) {
@@ -127,11 +121,13 @@ extern "C" int ns_poisson_fft_noalloc(const double* rhs_dev, double* dp_dev, int
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   double2* spec = reinterpret_cast<double2*>(base);  // 256-byte aligned
-  double* inv_lam = base + n_spec;
-  int4* tw = reinterpret_cast<int4*>(base + n_spec + n_lam + ((n_spec + n_lam) & 1));
+  double2* cyc = reinterpret_cast<double2*>(base + n_spec);
+  int4* tw = reinterpret_cast<int4*>(base + n_spec + n_cyc);
   const double dx = lx / nx, dy = ly / ny, dz = lz / nz;
+  const double rs = dz * dz * (1.0 / (2.0 * (double)nx * (double)ny * (double)nz)) * nz;
 
-  noalloc_tables<<<152, 256, 0, st>>>(tw, M, nx, ny, nz, inv_lam, dx, dy, dz);
+  const int n_tab = (int)(n_tw / 2) + nxh * ny;
+  noalloc_tables<<<(n_tab + 63) / 64, 64, 0, st>>>(tw, M, nx, ny, nz, cyc, dx, dy, dz, rs);
   if (cudaGetLastError() != cudaSuccess) return NS_ERR_CUDA;
 
   FftPlan P{};
@@ -139,8 +135,10 @@ extern "C" int ns_poisson_fft_noalloc(const double* rhs_dev, double* dp_dev, int
   P.tw_x = tw;
   P.tw_xr = tw + M;
   P.tw_y = tw + M + (M / 2 + 1);
-  P.tw_z = tw + M + (M / 2 + 1) + ny;
-  P.inv_lam = inv_lam;
+  P.zcyc = 1;
+  P.cyc_rs = rs;
+  P.cyc_t = cyc;
+  P.cyc_h = reinterpret_cast<double*>(cyc + 2 * nxh * ny);
   P.dp_unaligned = 1;  // dp is the caller's (nx+2)^3 array: pairs (2m+1, 2m+2) are not 16-byte aligned
 
   // rhs (nx, ny, nz), Fortran order: cell slot (s, j, k) at (s-1) + nx (j-1) + nx ny (k-1)

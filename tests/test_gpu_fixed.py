@@ -223,7 +223,21 @@ def test_dense_lengths(n, pbc):
     assert rel_l2(_solve(n, (pbc,) * 3, rhs * two) / two, ref) < 1e-12
 
 
-# --- the one-launch fills ---------------------------------------------------
+# --- the cyclic z solve and the one-launch fills ------------------------------------------------
+@pytest.mark.parametrize("nz", [16, 32, 64, 128, 256, 512])
+@pytest.mark.parametrize("lz", [0.05, 1.0, 40.0])
+def test_cyclic_solve_lengths(nz, lz):
+    """Every segment count; flat boxes (rho next to 1 in the low modes) and tall ones."""
+    from ns_3d_staggered_dp_gb300 import Session, make_config
+
+    n = (32, 16, nz)
+    rhs = np.random.default_rng(nz).standard_normal(n)
+    rhs -= rhs.mean()
+    ref = O.spectral_poisson(rhs, (1, 1, 1), 1.0 / 32, 1.0 / 16, lz / nz)
+    with Session(make_config(*n, lx=1.0, ly=1.0, lz=lz)) as s:
+        assert rel_l2(s.poisson(rhs)[1:-1, 1:-1, 1:-1], ref) < 1e-11
+
+
 @pytest.mark.parametrize("bc", [(1, 1, 1), (1, 2, 1), (1, 1, 4), (1, 4, 2), (2, 2, 2), (4, 2, 4), (4, 4, 4)])
 def test_fills_of_every_code(bc):
     """vel_bc_staggered and the pressure ghosts with non-zero faces, edges and corners included."""
