@@ -438,11 +438,8 @@ cudaError_t launch_adi_batch(int axis, const BatchAdiArgs* tab, const BatchItem*
 // 16) away.  A thread solves CH unknowns of a line from CH + 2 halo right-hand
 // sides held in registers: one read and one write of the fields, no
 // intermediate in memory, and CH-fold parallelism along the line.  The
-// right-hand sides come scaled by the pivots (ChunkSys), one FMA each way:
-// 2.75 FP64 instructions an unknown at CH 32, halo 8, against 3 and 1.9 times
-// the traffic of the whole-line kernels.  At 256^3 (whole lines before, in
-// parentheses): x 0.36 ms (0.51), y 0.29 (0.38), z 0.29 (0.37), the FP64 pipe
-// at 61-78%; at 32^3 10 us a sweep (20).
+// right-hand sides come scaled by the pivots (ChunkSys), one FMA each way.
+// These kernels take the lines that do not fit a CTA (launch_adi_chunks).
 // Rows q of [T0, T1) take their factors from the tables, the others the converged ones.
 template <int R, int W, int T0, int T1>
 __device__ __forceinline__ void chunk_rows(double (&r)[R], const ChunkSys& S, int e0) {
@@ -639,18 +636,282 @@ cudaError_t launch_adi_chunk(int axis, const AdiArgs& a, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-// Unknowns per chunk: 32, or 34 where that saves a chunk (the n + 2 unknowns
-// of a wall line), and 16 on boxes whose 32-unknown chunks leave SMs idle.
+// ---------------------------------------------------------------------------
+// Chunked sweeps, whole lines in a CTA
+// ---------------------------------------------------------------------------
+// The same with a line's chunks in one CTA (32 lines, a thread CH unknowns of
+// one): what enters a chunk is worked out by its neighbour from its W
+// outermost unknowns and handed over through shared memory, so every
+// right-hand side is read once and takes part in 2 (CH + W) / CH FMAs: 2.5 at
+// CH 32, W 8, against 2.75 and a second read of the halos.  Bound by the FP64
+// unit, 75 to 80% busy.  Sweeps x, y, z in us (chunks with halos; whole lines
+// with one thread each): 256^3 278, 266, 267 (371, 317, 290; 512, 385, 369),
+// 128^3 52, 46, 49 (65, 58, 58), with walls 70, 61, 62 (82, 73, 73), 32^3 12,
+// 8, 8 (10, 11, 10).  The same in 58-bit integers with the exponent of the
+// line takes 319, 296, 292 at 256^3: the chain of a product waits longer there
+// than for an FMA.  The batch keeps the whole-line kernels: 185, 108, 107 us
+// for 64 blocks of 16 to 64 cells, in chunks of 18 172, 176, 155.
+// Chunks of a line in one CTA, at most: 10 of 26 unknowns (258: a wall line of
+// 256 cells), else 8.
+constexpr int line_chunks_max(int ch) { return ch == 26 ? 10 : 8; }
+// Rows of a line's first end that may differ from the converged ones.
+__host__ __device__ constexpr int line_low(int W) { return W + 2; }
+// The system has its special rows where the kernels look for them: a few at
+// the first end, the last one of a wall line; and chunks divide a cyclic line.
+inline bool line_chunk_ok(const ChunkSys& S, int ch, int W) {
+  return S.c0 <= std::min(line_low(W), ch) && S.c1 >= (S.periodic ? S.m : S.m - 1) &&
+         S.m <= line_chunks_max(ch) * ch && !(S.periodic && S.m % ch);
+}
+// The recurrences over the unknowns [Q0, Q1) of a chunk, forward and backward,
+// from the value that enters.  Rows below T1 take their factors from the
+// tables; END: row ql is the line's last, with its own factor (selects, which
+// cost nothing beside an FMA; its pivot is in the right-hand side, last_pivot).
+// STORE: in place, else only the value that leaves.
+template <int CH, int Q0, int Q1, int T1, bool END, bool STORE>
+__device__ __forceinline__ double chunk_fwd(double (&r)[CH], const ChunkSys& S, int e0, int ql, double y) {
+  const double* l = S.l + kAdiExt + e0;
+  const double nl = -S.lc, ll = END ? -__ldg(l + ql) * __ldg(S.dm + kAdiExt + e0 + ql) : 0.0;
+#pragma unroll
+  for (int q = Q0; q < Q1; ++q) {
+    const double f = q < T1 ? -__ldg(l + q) : (END ? (q < ql ? nl : (q == ql ? ll : 0.0)) : nl);
+    y = fma(f, y, r[q]);
+    if (STORE) r[q] = y;
+  }
+  return y;
+}
+template <int CH, int Q0, int Q1, int T1, bool STORE>
+__device__ __forceinline__ double chunk_bwd(double (&r)[CH], const ChunkSys& S, int e0, double x) {
+  const double* dm = S.dm + kAdiExt + e0;
+  const double* cu = S.cu + kAdiExt + e0;
+  const double nc = -S.cc;
+#pragma unroll
+  for (int q = Q1 - 1; q >= Q0; --q) {
+    x = q < T1 ? fma(-__ldg(cu + q), x, r[q] * __ldg(dm + q)) : fma(nc, x, r[q]);
+    if (STORE) r[q] = x;
+  }
+  return x;
+}
+
+// r: the right-hand sides of chunk s of T (zero past the line's end), replaced by the solution.
+// sh: 16 bytes a thread.
+template <int CH, int W>
+__device__ __forceinline__ void chunk_line_solve(double (&r)[CH], const ChunkSys& S, int s, int T, int l, double* sh) {
+  constexpr int LOW = line_low(W) < CH ? line_low(W) : CH;
+  double* ys = sh;
+  double* xs = sh + 32 * T;
+  const int e0 = s * CH, ql = S.m - 1 - e0;
+  const bool low = s == 0 && S.c0 > 0, end = e0 + CH > S.c1;
+  ys[32 * s + l] = chunk_fwd<CH, CH - W, CH, CH - W < LOW ? LOW : 0, false, false>(r, S, e0, 0, 0.0);
+  __syncthreads();
+  const double yi = s > 0 ? ys[32 * (s - 1) + l] : (S.wrap_lo ? ys[32 * (T - 1) + l] : 0.0);
+  double x;
+  if (!low && !end) {
+    chunk_fwd<CH, 0, CH, 0, false, true>(r, S, e0, 0, yi);
+    x = chunk_bwd<CH, 0, W, 0, false>(r, S, e0, 0.0);
+  } else if (!end) {
+    chunk_fwd<CH, 0, CH, LOW, false, true>(r, S, e0, 0, yi);
+    x = chunk_bwd<CH, 0, W, LOW, false>(r, S, e0, 0.0);
+  } else if (!low) {
+    if (ql >= 0) chunk_fwd<CH, 0, CH, 0, true, true>(r, S, e0, ql, yi);  // below: no row of the line
+    x = chunk_bwd<CH, 0, W, 0, false>(r, S, e0, 0.0);
+  } else {
+    chunk_fwd<CH, 0, CH, LOW, true, true>(r, S, e0, ql, yi);
+    x = 0.0;
+  }
+  xs[32 * s + l] = x;
+  __syncthreads();
+  const double xi = s + 1 < T ? xs[32 * (s + 1) + l] : (S.wrap_hi ? xs[l] : 0.0);
+  if (low) chunk_bwd<CH, 0, CH, LOW, true>(r, S, e0, xi);
+  else chunk_bwd<CH, 0, CH, 0, true>(r, S, e0, xi);
+}
+
+// Pivot ratio by which the last row's right-hand side of a wall line is given
+// (one of the table rows scales it itself).
+template <int CH, int W>
+__device__ __forceinline__ double last_pivot(const ChunkSys& S) {
+  return S.m > (line_low(W) < CH ? line_low(W) : CH) ? __ldg(S.dm + kAdiExt + S.m - 1) : 1.0;
+}
+// One sweep's lines of one field: n1 lines a row, nl lines from z slot zlo on,
+// source, destination, BC-row planes.
+struct LineJob {
+  int n1, zlo, nl;
+  const double* src;
+  double* dst;
+  const double* face_lo;
+  const double* face_hi;
+  double face_scale;
+};
+
+// y and z sweeps: blockDim (32 lines, T chunks), lanes over x; lines [t0, t0 + 32).
+template <int AXIS, int CH, int W>
+__device__ __forceinline__ void line_chunks(const Layout& L, const ChunkSys& S, const LineJob& J, int t0, double* sh) {
+  const int l = threadIdx.x, s = threadIdx.y, T = blockDim.y, n1 = J.n1;
+  const bool valid = t0 + l < J.nl;
+  const int tl = min(t0 + l, J.nl - 1);  // lanes past the end repeat the last line (never stored)
+  long long base, st;
+  line_of<AXIS>(L, tl % n1, J.zlo + tl / n1, base, st);
+  const double* src = J.src + base;
+  double* dst = J.dst + base;
+  const int e0 = s * CH, m = S.m;
+  const double* sl = src + (S.lo + e0) * st;
+  double r[CH];
+#pragma unroll
+  for (int q = 0; q < CH; ++q, sl += st) r[q] = e0 + q < m ? *sl : 0.0;
+  const int nax = axis_n(L, AXIS);
+  if (!S.periodic) {
+    if (e0 == 0) r[0] = J.face_lo ? J.face_scale * __ldg(J.face_lo + tl + J.zlo * n1) : 0.0;
+    if (e0 < m && e0 + CH >= m) {  // the BC rows take the sweep's face values
+      const double hi = J.face_hi ? last_pivot<CH, W>(S) * J.face_scale * __ldg(J.face_hi + tl + J.zlo * n1) : 0.0;
+#pragma unroll
+      for (int q = 0; q < CH; ++q)
+        if (e0 + q == m - 1) r[q] = hi;
+    }
+    if (valid && s == 0) {  // the carried slots
+      for (int i = 0; i < S.lo; ++i) dst[i * st] = src[i * st];
+      for (int i = S.lo + m; i <= nax + 1; ++i) dst[i * st] = src[i * st];
+    }
+  }
+  chunk_line_solve<CH, W>(r, S, s, T, l, sh);
+  if (!valid) return;
+  double* xl = dst + (S.lo + e0) * st;
+#pragma unroll
+  for (int q = 0; q < CH; ++q, xl += st)
+    if (e0 + q < m) *xl = r[q];
+  if (S.periodic) {  // chunks divide m
+    if (s == 0) dst[(nax + 1) * st] = r[0];       // slot n+1 <- slot 1
+    if (s == T - 1) dst[0] = r[CH - 1];           // slot 0 <- slot n
+  }
+}
+
+// x sweep: the CTA's 32 lines pass through shared memory in 16-byte units,
+// unit u of line l at place u ^ (l & 7), so that rows are whole on the global
+// side and 8 lanes read 8 different banks' worth on the other.
+__host__ __device__ constexpr int line_pitch(int ch, int T) { return (ch / 2 * T + 7) & ~7; }  // units a line
+template <int CH, int W>
+__device__ __forceinline__ void line_chunks_x(const Layout& L, const ChunkSys& S, const LineJob& J, int t0, double* sh) {
+  const int l = threadIdx.x, s = threadIdx.y, T = blockDim.y;
+  const int pitch = line_pitch(CH, T), m = S.m, e0 = s * CH;
+  double2* sb = reinterpret_cast<double2*>(sh);
+  double* ex = sh + 64LL * pitch;
+  const int nl = min(32, J.nl - t0);
+  const int t = t0 + min(l, nl - 1);  // lanes past the end repeat the last line (never stored)
+  const int j = t % J.n1, k = J.zlo + t / J.n1;
+  const int my_off = (int)L.at(S.lo, j, k);  // unknown 0 of this lane's line
+  // slot 1 is 16-byte aligned: whole units where it is unknown 0
+  const int nu = S.lo == 1 ? m / 2 : 0;
+  for (int q = s; q < 32; q += T) {
+    const double* g = J.src + __shfl_sync(0xffffffffu, my_off, q);
+    double2* row = sb + q * pitch;
+    for (int u = l; u < nu; u += 32) cp_async16(row + (u ^ (q & 7)), g + 2 * u);
+    for (int e = 2 * nu + l; e < CH * T; e += 32) {
+      double* at = reinterpret_cast<double*>(row + ((e >> 1) ^ (q & 7))) + (e & 1);
+      if (e < m) cp_async8(at, g + e);
+      else *at = 0.0;
+    }
+  }
+  cp_async_commit();
+  const bool walls = !S.periodic;
+  double lo = 0.0, hi = 0.0;
+  if (walls) {
+    if (J.face_lo) lo = J.face_scale * __ldg(J.face_lo + j + J.n1 * k);
+    if (J.face_hi) hi = last_pivot<CH, W>(S) * J.face_scale * __ldg(J.face_hi + j + J.n1 * k);
+  }
+  cp_async_wait<0>();
+  __syncthreads();
+  double2* row = sb + l * pitch;
+  double r[CH];
+#pragma unroll
+  for (int q = 0; q < CH; q += 2) {
+    const double2 d = row[((e0 + q) >> 1) ^ (l & 7)];
+    r[q] = d.x;
+    r[q + 1] = d.y;
+  }
+  if (walls) {  // the BC rows take the sweep's face values
+    if (e0 == 0) r[0] = lo;
+    if (e0 < m && e0 + CH >= m) {
+#pragma unroll
+      for (int q = 0; q < CH; ++q)
+        if (e0 + q == m - 1) r[q] = hi;
+    }
+  }
+  chunk_line_solve<CH, W>(r, S, s, T, l, ex);
+#pragma unroll
+  for (int q = 0; q < CH; q += 2) row[((e0 + q) >> 1) ^ (l & 7)] = make_double2(r[q], r[q + 1]);
+  __syncthreads();
+  for (int q = s; q < nl; q += T) {
+    double* g = J.dst + __shfl_sync(0xffffffffu, my_off, q);
+    const double2* rq = sb + q * pitch;
+    for (int u = l; u < nu; u += 32) *reinterpret_cast<double2*>(g + 2 * u) = rq[u ^ (q & 7)];
+    for (int e = 2 * nu + l; e < m; e += 32)
+      g[e] = reinterpret_cast<const double*>(rq + ((e >> 1) ^ (q & 7)))[e & 1];
+  }
+  if (l < nl) {
+    const double* xs = J.src + L.at(0, j, k);
+    double* xd = J.dst + L.at(0, j, k);
+    if (walls) {  // the carried slots
+      if (s == 0) {
+        for (int i = 0; i < S.lo; ++i) xd[i] = xs[i];
+        for (int i = S.lo + m; i <= L.nx + 1; ++i) xd[i] = xs[i];
+      }
+    } else {  // chunks divide m
+      if (s == 0) xd[L.nx + 1] = r[0];    // slot n+1 <- slot 1
+      if (s == T - 1) xd[0] = r[CH - 1];  // slot 0 <- slot n
+    }
+  }
+}
+size_t line_smem(int axis, int ch, int T) {
+  return (size_t)T * 32 * 16 + (axis == 0 ? (size_t)32 * line_pitch(ch, T) * sizeof(double2) : 0);
+}
+
+template <int AXIS, int CH, int W>
+__global__ void __launch_bounds__(32 * line_chunks_max(CH), CH == 16 ? 4 : (CH == 26 ? 2 : 3))
+    adi_line_chunk_kernel(const __grid_constant__ AdiArgs a) {
+  extern __shared__ __align__(16) double sh_line[];
+  const int fld = blockIdx.y;
+  const bool part = AXIS != 2 && a.z1 > 0;  // only the lines of z slots [z0, z1)
+  const int n1 = AXIS == 0 ? a.L.ny + 2 : a.L.nx + 2;
+  const int n2 = AXIS == 2 ? a.L.ny + 2 : (part ? a.z1 - a.z0 : a.L.nz + 2);
+  const LineJob J{n1,        part ? a.z0 : 0, n1 * n2,          a.src[fld], a.dst[fld], a.face_lo[fld],
+                  a.face_hi[fld], a.face_scale};
+  if (AXIS == 0) line_chunks_x<CH, W>(a.L, a.ch[fld], J, blockIdx.x * 32, sh_line);
+  else line_chunks<AXIS, CH, W>(a.L, a.ch[fld], J, blockIdx.x * 32, sh_line);
+}
+
+template <int AXIS, int CH, int W>
+cudaError_t launch_adi_line_chunk(const AdiArgs& a, int m, cudaStream_t st) {
+  const int n1 = AXIS == 0 ? a.L.ny + 2 : a.L.nx + 2;
+  const int n2 = AXIS == 2 ? a.L.ny + 2 : (a.z1 > 0 ? a.z1 - a.z0 : a.L.nz + 2);
+  if (n2 <= 0) return cudaSuccess;
+  const int T = (m + CH - 1) / CH;
+  const size_t sm = line_smem(AXIS, CH, T);
+  auto kern = adi_line_chunk_kernel<AXIS, CH, W>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (e != cudaSuccess) return e;
+  kern<<<dim3((unsigned)((n1 * n2 + 31) / 32), 3), dim3(32, T), sm, st>>>(a);
+  return cudaGetLastError();
+}
+
+// Unknowns per chunk: 32 or 26, whichever computes fewer (130, the unknowns of
+// a wall line of 128 cells: 5 x 26), and 16 on boxes whose 32-unknown chunks
+// leave SMs idle (a 32^3 sweep: 8 to 12 us against 20 a whole line).
+// Lines that do not fit a CTA take the chunks that work out their own halos.
 cudaError_t launch_adi_chunks(int axis, const AdiArgs& a, cudaStream_t st) {
   const int m = std::max(a.ch[0].m, std::max(a.ch[1].m, a.ch[2].m));
   const long long cells = 3LL * (a.L.nx + 2) * (a.L.ny + 2) * (a.L.nz + 2);
-  const int ch = cells / 32 < 40000 ? 16 : ((m + 33) / 34 < (m + 31) / 32 ? 34 : 32);
-#define NS_ADI_HALO(W)                                                             \
-  if (a.halo == W)                                                                 \
-    return ch == 16 ? launch_adi_chunk<16, W>(axis, a, st)                         \
-                    : (ch == 34 ? launch_adi_chunk<34, W>(axis, a, st) : launch_adi_chunk<32, W>(axis, a, st));
-  NS_ADI_HALO(6) NS_ADI_HALO(8) NS_ADI_HALO(10) NS_ADI_HALO(12) NS_ADI_HALO(16)
-#undef NS_ADI_HALO
+  const int W = a.halo <= 8 ? 8 : (a.halo <= 12 ? 12 : 16);
+  auto work = [&](int c) { return (m + c - 1) / c * (c + W); };
+  const int ch = cells / 32 < 40000 && m <= 16 * line_chunks_max(16) ? 16 : (work(26) < work(32) ? 26 : 32);
+  bool fits = true;
+  for (const ChunkSys& S : a.ch) fits = fits && line_chunk_ok(S, ch, W);
+  if (!fits) return a.halo <= 8 ? launch_adi_chunk<32, 8>(axis, a, st) : launch_adi_chunk<32, 16>(axis, a, st);
+#define NS_ADI_LINE(A, C, H) \
+  if (axis == A && ch == C && W == H) return launch_adi_line_chunk<A, C, H>(a, m, st);
+#define NS_ADI_LINES(C, H) NS_ADI_LINE(0, C, H) NS_ADI_LINE(1, C, H) NS_ADI_LINE(2, C, H)
+  NS_ADI_LINES(16, 8) NS_ADI_LINES(16, 12) NS_ADI_LINES(16, 16)
+  NS_ADI_LINES(32, 8) NS_ADI_LINES(32, 12) NS_ADI_LINES(32, 16)
+  NS_ADI_LINES(26, 8) NS_ADI_LINES(26, 12) NS_ADI_LINES(26, 16)
+#undef NS_ADI_LINES
+#undef NS_ADI_LINE
   return cudaErrorInvalidValue;
 }
 

@@ -205,6 +205,37 @@ def test_sweeps_for_every_halo(n, bc, alpha, closure):
         assert rel_l2(out[k], getattr(ref, k)) < 1e-10, k
 
 
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("m", [14, 16, 30, 32, 34, 46, 64, 66, 126, 128, 130, 134, 254, 256, 270, 272, 300])
+@pytest.mark.parametrize("bc", [1, 2, 4])
+def test_sweeps_of_every_line_length(axis, m, bc):
+    """Line lengths around every chunk count and past the longest line of one CTA."""
+    from ns_3d_staggered_dp_gb300 import Session, make_config
+    from tests.helpers import random_state
+
+    if bc == 1 and m & (m - 1):
+        pytest.skip("periodic lines are powers of two")
+    if axis == 2 and m > 256:
+        pytest.skip("the Poisson solve's line axis, 256 cells at most with a wall x")
+    if bc == 1:
+        m = max(m, 16) if m < 256 else 512
+    n, code = [16, 8, 9] if bc != 1 else [16, 16, 16], [2, 2, 2] if bc != 1 else [1, 1, 1]
+    n[axis], code[axis] = m, bc
+    wall = {1: 1, 2: 3, 4: 4}
+    dt, L = 0.003, [0.2 * q for q in n]
+    for alpha in (0.004, 0.07):
+        nu = 2.0 * alpha * 0.2 ** 2 / dt
+        cfg = O.Config(*n, *L, nu=nu, dt=dt, scheme=O.AB2_CN, bc=tuple(code), pbc=tuple(wall[b] for b in code))
+        st = random_state(cfg, m, amp=0.1, history=True)
+        _, parts = O.step(st.copy(), cfg, return_parts=True)
+        with Session(make_config(*n, lx=L[0], ly=L[1], lz=L[2], nu=nu, dt=dt, scheme=2, bc=cfg.bc, pbc=cfg.pbc)) as s:
+            s.set_state(st.u, st.v, st.w, st.p, (st.px, st.py, st.pz))
+            s.step(1)
+            g = s.get_stage()
+        for k, sl in (("us", np.s_[:, 1:-1, 1:-1]), ("vs", np.s_[1:-1, :, 1:-1]), ("ws", np.s_[1:-1, 1:-1, :])):
+            assert rel_l2(g[k][sl], parts[k][sl]) < 1e-13, k
+
+
 # --- the dense wall transforms ------------------------------------------------------------------
 DENSE = [((16, m, 9), b) for m in (5, 8, 15, 16, 17, 31, 75, 100, 127, 129, 200, 257, 300) for b in (2, 3, 4)]
 DENSE += [((m, 8, 9), b) for m in (6, 16, 18, 34, 90, 130, 256, 320) for b in (2, 3, 4)]
