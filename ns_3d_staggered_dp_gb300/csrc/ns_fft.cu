@@ -251,11 +251,30 @@ __global__ void __launch_bounds__(256, 2) fft_x_fwd_kernel(FftPlan P, DivArgs d,
       double r1 = fmul(cc, fsub(cc, ub, ua.y), d.cdx);
       r1 = fma(fsub(cc, vb.y, va.y), d.cdy, r1);
       r1 = fma(fsub(cc, wb.y, wa.y), d.cdz, r1);
-      if (HAS_BC) {  // pr_bc_staggered_modify_rhs on the wall cells of y and z
-        r0 += P.bc_term(s, j, k);
-        r1 += P.bc_term(s + 1, j, k);
-      }
       x[n2] = make_double2(r0, r1);
+    }
+    // pr_bc_staggered_modify_rhs (FftPlan::bc_term) on the wall lines of y and z, x being periodic:
+    // apart from the divergence and with all loads of a line in flight, 2 of 128 lines would
+    // otherwise hold up half of the CTAs (channel 256 x 128 x 256: 249 us with a call per cell)
+    if (HAS_BC && (j == 1 || j == ny || k == 1 || k == nz)) {
+      const int n1 = L.nx + 2;
+      const double* f1 = j == 1 ? P.face_lo[1] : (j == ny ? P.face_hi[1] : nullptr);
+      const double* f2 = k == 1 ? P.face_lo[2] : (k == nz ? P.face_hi[2] : nullptr);
+      const double m1 = j == 1 ? P.mod_lo[1] : P.mod_hi[1], m2 = k == 1 ? P.mod_lo[2] : P.mod_hi[2];
+      if (f1 && m1 != 0.0) {
+#pragma unroll
+        for (int n2 = 0; n2 < R2; ++n2) {
+          const double* f = f1 + 2 * (t + R1 * n2) + 1 + n1 * k;
+          x[n2] = make_double2(fma(m1, f[0], x[n2].x), fma(m1, f[1], x[n2].y));
+        }
+      }
+      if (f2 && m2 != 0.0) {
+#pragma unroll
+        for (int n2 = 0; n2 < R2; ++n2) {
+          const double* f = f2 + 2 * (t + R1 * n2) + 1 + n1 * j;
+          x[n2] = make_double2(fma(m2, f[0], x[n2].x), fma(m2, f[1], x[n2].y));
+        }
+      }
     }
     i2 v[R2];
     const int eb = fx_block2<X::B2>(x, v);
@@ -302,16 +321,22 @@ __global__ void __launch_bounds__(256, 2) fft_x_fwd_kernel(FftPlan P, DivArgs d,
   if (valid) {
     const FxOut fo = fx_out(ec);
     double2* out = spec + (long long)P.nxh * ((j - 1) + (long long)P.ny * (k - 1));
-    for (int kk = t; kk <= M / 2; kk += T) {
-      const i2 zk = zb[kk];
-      const i2 zm = zb[(M - kk) % M];
-      const i2 E{zk.x + zm.x, zk.y - zm.y};
-      const i2 O{zk.x - zm.x, zk.y + zm.y};
-      const i2 WO = fx_cmul(O, fx_ldg(P.tw_xr + kk));  // F = i W O
-      out[kk] = fx_to(i2{E.x + WO.y, E.y - WO.x}, fo, cc);
-      if (kk == 0) out[M] = fx_to(i2{E.x - WO.y, 0}, fo, cc);
-      else if (kk != M / 2) out[M - kk] = fx_to(i2{E.x - WO.y, -(E.y + WO.x)}, fo, cc);
-    }
+    // The FP64 unit is the busier one here (the divergence), so the results go back on the integer
+    // pipes, but for the extreme exponents.
+    auto split = [&](auto to) {
+      for (int kk = t; kk <= M / 2; kk += T) {
+        const i2 zk = zb[kk];
+        const i2 zm = zb[(M - kk) % M];
+        const i2 E{zk.x + zm.x, zk.y - zm.y};
+        const i2 O{zk.x - zm.x, zk.y + zm.y};
+        const i2 WO = fx_cmul(O, fx_ldg(P.tw_xr + kk));  // F = i W O
+        out[kk] = to(i2{E.x + WO.y, E.y - WO.x});
+        if (kk == 0) out[M] = to(i2{E.x - WO.y, 0});
+        else if (kk != M / 2) out[M - kk] = to(i2{E.x - WO.y, -(E.y + WO.x)});
+      }
+    };
+    if (FROM_RHS || ec < -1000 || ec > 850) split([&](i2 v) { return fx_to(v, fo, cc); });
+    else split([&](i2 v) { return make_double2(fx_to_int(v.x, ec), fx_to_int(v.y, ec)); });
     if (fo.odd)
       for (int kk = t; kk <= M / 2; kk += T) {
         fx_rescale(out[kk], fo);
