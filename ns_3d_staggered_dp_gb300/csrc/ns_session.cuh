@@ -102,6 +102,18 @@ void dense_pair(int n, int pb, std::vector<double>& F, std::vector<double>& G);
 double axis_eig(int n, int pb, int m, double h);
 // Predictor coefficients of a box with velocity codes bc (ns_api.cu).
 void set_predict_coeffs(PredictArgs& a, const int bc[3], double dx, double dy, double dz, double dt, double nu);
+// State read-back straight into the caller's page-locked arrays (ns_api.cu): up
+// to seven fields, a field's ex x ey x ez entries from slot (ox, oy, oz) on,
+// zero outside [lo, hi].
+struct GetFields {
+  Layout L;
+  const double* src[7];
+  double* dst[7];  // NULL: not asked for
+  int ext[7][3], off[7][3], lo[7][3], hi[7][3];
+};
+// Whether the kernel below may write to the n doubles at p.
+bool get_direct(const double* p, long long n);
+cudaError_t launch_get_fields(const GetFields& a, cudaStream_t st);
 // Host description of one tridiagonal line system of an ADI sweep: LU
 // factors without pivoting (forward multipliers l, 1/pivot dinv,
 // super-diagonal / pivot cu) and, periodic only, the Sherman-Morrison data.

@@ -297,3 +297,36 @@ def test_fills_of_every_code(bc):
         want[1:-1, 1:-1, 1:-1] = dp[1:-1, 1:-1, 1:-1]
         O.pr_bc_staggered(want, f, pbc, *cfg.h)
         np.testing.assert_allclose(dp, want, rtol=0, atol=4e-16 * max(1.0, np.abs(want).max()))
+
+
+# --- states into page-locked arrays -----------------------------------------------------------------
+@pytest.mark.parametrize("shift", [0, 1, 5])
+@pytest.mark.parametrize("n,bc", [((16, 16, 16), (1, 1, 1)), ((18, 9, 13), (2, 2, 2)), ((64, 21, 32), (1, 2, 1))])
+def test_state_into_page_locked_arrays(n, bc, shift):
+    """The kernel that writes page-locked arrays against the staged copies, some fields left out."""
+    import ctypes
+
+    import torch
+
+    from ns_3d_staggered_dp_gb300 import Session, make_config
+    from tests.helpers import random_state
+
+    cfg = O.Config(*n, 1.0, 1.0, 1.0, scheme=O.AB2, dt=1e-3, bc=bc, pbc=tuple(3 if b == 2 else 1 for b in bc))
+    st = random_state(cfg, 7, history=True)
+    with Session(make_config(*n, dt=1e-3, scheme=1, bc=bc, pbc=cfg.pbc)) as s:
+        s.set_state(st.u, st.v, st.w, st.p, (st.px, st.py, st.pz))
+        s.step(2)
+        ref = s.get_state()
+        keys = ("u", "v", "w", "p", "hx", "hy", "hz")
+        for skip in ((), ("v", "hz"), ("u", "p", "hx", "hy")):
+            buf, arg = {}, []
+            for k in keys:
+                buf[k] = torch.full((ref[k].size + shift + 3,), 7.0, dtype=torch.float64).pin_memory()
+                p = ctypes.cast(buf[k].data_ptr() + 8 * shift, ctypes.POINTER(ctypes.c_double))
+                arg.append(None if k in skip else p)
+            s._check(s.lib.ns_get_state(s.h, *arg))
+            for k in keys:
+                got = buf[k].numpy()
+                body = got[shift:shift + ref[k].size]
+                assert (got[:shift] == 7.0).all() and (got[shift + ref[k].size:] == 7.0).all()
+                assert (body == 7.0).all() if k in skip else np.array_equal(body, ref[k].ravel(order="F"))
