@@ -657,9 +657,9 @@ constexpr int line_chunks_max(int ch) { return ch == 26 ? 10 : 8; }
 // Rows of a line's first end that may differ from the converged ones.
 __host__ __device__ constexpr int line_low(int W) { return W + 2; }
 // The system has its special rows where the kernels look for them: a few at
-// the first end, the last one of a wall line; and chunks divide a cyclic line.
+// the first end, the last one of a line that does not go on; and chunks divide a cyclic line.
 inline bool line_chunk_ok(const ChunkSys& S, int ch, int W) {
-  return S.c0 <= std::min(line_low(W), ch) && S.c1 >= (S.periodic ? S.m : S.m - 1) &&
+  return S.c0 <= std::min(line_low(W), ch) && S.c1 >= (S.wrap_hi ? S.m : S.m - 1) &&
          S.m <= line_chunks_max(ch) * ch && !(S.periodic && S.m % ch);
 }
 // The recurrences over the unknowns [Q0, Q1) of a chunk, forward and backward,

@@ -365,6 +365,10 @@ struct AdjState {
   int cur = 0;
   double* pscr = nullptr;     // p output of the adjoint projection (discarded)
   LineSys sys_t[3][3]{};      // transposed CN line systems (AB2-CN)
+  ChunkSys csys_t[3][3]{};    // the same for the chunked sweeps (halo 0 on every axis: not used)
+  int halo_t[3] = {};
+  double d_t[3] = {1.0, 1.0, 1.0};  // 1 / converged pivot: with chunks, ls stands for ls / (d_x d_y d_z)
+  double* chunk_buf = nullptr;
   double* sys_buf = nullptr;
 };
 
@@ -418,8 +422,9 @@ int adj_ensure(ns_handle* h) {
     if ((s = adj_alloc(h, &A->ls[1][q]))) return s;
   }
   if ((s = adj_alloc(h, &A->pscr))) return s;
-  if (h->cfg.scheme == NS_AB2_CN && (s = api_build_line_tables(h, true, A->sys_t, &A->sys_buf))) return s;
-  return NS_OK;
+  if (h->cfg.scheme != NS_AB2_CN) return NS_OK;
+  if ((s = api_build_line_tables(h, true, A->sys_t, &A->sys_buf))) return s;
+  return api_build_line_chunks(h, true, A->csys_t, A->halo_t, A->d_t, &A->chunk_buf);
 }
 
 // Reference extent of field f (0 u, 1 v, 2 w) along axis a.
@@ -482,7 +487,9 @@ int adj_backward_step(ns_handle* h, AdjState* A, double* const fwd[3], bool firs
         a.sys[f] = A->sys_t[ax][f];
         a.face_lo[f] = nullptr;
         a.face_hi[f] = nullptr;
+        a.ch[f] = A->csys_t[ax][f];
       }
+      a.halo = A->halo_t[ax];
       ADJ_CUDA(h, launch_adi(ax, a, h->stream));
       api_mark(h, ax == 0 ? "adj_adi_x" : (ax == 1 ? "adj_adi_y" : "adj_adi_z"), 1);
     }
@@ -511,6 +518,8 @@ int adj_backward_step(ns_handle* h, AdjState* A, double* const fwd[3], bool firs
     a.l0 = -2.0 * nu * (ix2 + iy2 + iz2);
     a.lx = nu * ix2; a.ly = nu * iy2; a.lz = nu * iz2;
   }
+  const double scale = A->d_t[0] * A->d_t[1] * A->d_t[2];  // what the chunked sweeps left out
+  for (double* q : {&a.wS, &a.wN, &a.l0, &a.lx, &a.ly, &a.lz}) *q *= scale;
   const bool next = has_next && c.scheme != NS_EULER;
   ADJ_CUDA(h, launch_adj_predict(a, !cn, next, h->stream));
   api_mark(h, "adj_predict", 1);
@@ -536,6 +545,7 @@ void api_free_adjoint(ns_handle* h) {
   }
   if (A->pscr) cudaFree(A->pscr);
   if (A->sys_buf) cudaFree(A->sys_buf);
+  if (A->chunk_buf) cudaFree(A->chunk_buf);
   delete A;
   h->adj = nullptr;
 }
@@ -657,7 +667,7 @@ int ns_adj_backward(ns_handle* h, const double* dJ_du, const double* dJ_dv, cons
       std::memset(gh[f], 0, n * sizeof(double));
       continue;
     }
-    for (size_t e = 0; e < n; ++e) gh[f][e] *= -0.5 * c.dt;
+    for (size_t e = 0; e < n; ++e) gh[f][e] *= -0.5 * c.dt * A->d_t[0] * A->d_t[1] * A->d_t[2];
     zero_copies(c, f, gh[f]);
   }
   // back to the state after the forward run

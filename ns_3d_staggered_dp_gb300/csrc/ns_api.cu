@@ -49,7 +49,8 @@ namespace ns {
 // unknowns); otherwise tangential (B matrix, n+2 unknowns).
 // transposed (periodic only): the system M^T of the adjoint sweep, whose
 // corner entries are those of M exchanged.
-HostChunkSys build_chunk_system(int n, int bc, double h, double dt, double nu, bool normal, int closure) {
+HostChunkSys build_chunk_system(int n, int bc, double h, double dt, double nu, bool normal, int closure,
+                                bool transposed) {
   typedef long double ld;
   const double idx2 = 1.0 / (h * h);
   const double dg = 1.0 + 0.5 * dt * nu * 2.0 * idx2, of = -0.5 * dt * nu * 1.0 * idx2;  // as build_cn_system
@@ -60,10 +61,11 @@ HostChunkSys build_chunk_system(int n, int bc, double h, double dt, double nu, b
   if (bc == 1) {
     if (normal && closure == 0) {  // A(1,n+1) ties face 1 to itself (build_cn_system)
       b[0] = (ld)dg + of;
-      a[0] = 0;
+      (transposed ? c[m - 1] : a[0]) = 0;
     }
-    S.wrap_lo = !(normal && closure == 0);
-    S.wrap_hi = S.periodic = 1;
+    S.wrap_lo = transposed || !(normal && closure == 0);
+    S.wrap_hi = !transposed || !(normal && closure == 0);
+    S.periodic = 1;
   } else {
     const ld e = !normal && bc == 2 ? 0.5L : 1.0L, f = !normal && bc == 2 ? 0.5L : 0.0L;
     b[0] = b[m - 1] = e;
@@ -1194,11 +1196,10 @@ int build_line_tables(ns_handle* h, bool transposed, LineSys sys[3][3], double**
 // right-hand sides are scaled by the product of the pivots still to come, so
 // a session that hands out u* between the sweeps (keep_sweeps) keeps the
 // whole-line kernels.
-int build_adi_chunks(ns_handle* h) {
+int build_line_chunks(ns_handle* h, bool transposed, ChunkSys csys[3][3], int halo[3], double d[3], double** buf) {
   const ns_config& c = h->cfg;
   const int ns_[3] = {c.nx, c.ny, c.nz};
   const double hs[3] = {h->dx, h->dy, h->dz};
-  if (c.keep_sweeps) return NS_OK;
   HostChunkSys S[3][3];
   size_t total = 0;
   for (int ax = 0; ax < 3; ++ax)
@@ -1206,26 +1207,27 @@ int build_adi_chunks(ns_handle* h) {
       // the two tangential fields share a system
       const int first = ax == 0 ? 1 : 0;
       if (f != ax && f != first) S[ax][f] = S[ax][first];
-      else S[ax][f] = build_chunk_system(ns_[ax], c.bc[ax], hs[ax], c.dt, c.nu, f == ax, c.cn_periodic_closure);
+      else S[ax][f] = build_chunk_system(ns_[ax], c.bc[ax], hs[ax], c.dt, c.nu, f == ax, c.cn_periodic_closure,
+                                         transposed);
       if (!S[ax][f].halo) return NS_OK;
       total += 3 * S[ax][f].l.size();
     }
-  NS_CUDA(h, cudaMalloc(&h->adi_chunk_buf, total * sizeof(double)));
+  NS_CUDA(h, cudaMalloc(buf, total * sizeof(double)));
   std::vector<double> host;
   host.reserve(total);
   for (int ax = 0; ax < 3; ++ax)
     for (int f = 0; f < 3; ++f) {
       const HostChunkSys& q = S[ax][f];
-      ChunkSys& D = h->csys[ax][f];
-      D.l = h->adi_chunk_buf + host.size(); host.insert(host.end(), q.l.begin(), q.l.end());
-      D.dm = h->adi_chunk_buf + host.size(); host.insert(host.end(), q.dm.begin(), q.dm.end());
-      D.cu = h->adi_chunk_buf + host.size(); host.insert(host.end(), q.cu.begin(), q.cu.end());
+      ChunkSys& D = csys[ax][f];
+      D.l = *buf + host.size(); host.insert(host.end(), q.l.begin(), q.l.end());
+      D.dm = *buf + host.size(); host.insert(host.end(), q.dm.begin(), q.dm.end());
+      D.cu = *buf + host.size(); host.insert(host.end(), q.cu.begin(), q.cu.end());
       D.lc = q.lc; D.cc = q.cc; D.c0 = q.c0; D.c1 = q.c1; D.lo = q.lo; D.m = q.m;
       D.wrap_lo = q.wrap_lo; D.wrap_hi = q.wrap_hi; D.periodic = q.periodic;
-      h->adi_d[ax] = q.d;  // the converged pivot is the same for the three fields
-      h->adi_halo[ax] = std::max(h->adi_halo[ax], q.halo);
+      d[ax] = q.d;  // the converged pivot is the same for the three fields
+      halo[ax] = std::max(halo[ax], q.halo);
     }
-  NS_CUDA(h, cudaMemcpyAsync(h->adi_chunk_buf, host.data(), total * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+  NS_CUDA(h, cudaMemcpyAsync(*buf, host.data(), total * sizeof(double), cudaMemcpyHostToDevice, h->stream));
   NS_CUDA(h, cudaStreamSynchronize(h->stream));
   return NS_OK;
 }
@@ -1233,7 +1235,8 @@ int build_adi_chunks(ns_handle* h) {
 int build_adi(ns_handle* h) {
   if (h->cfg.scheme != NS_AB2_CN) return NS_OK;
   const int s = build_line_tables(h, false, h->sys, &h->adi_buf);
-  return s ? s : build_adi_chunks(h);
+  if (s || h->cfg.keep_sweeps) return s;
+  return build_line_chunks(h, false, h->csys, h->adi_halo, h->adi_d, &h->adi_chunk_buf);
 }
 
 void free_all(ns_handle* h) {
@@ -1287,6 +1290,9 @@ void api_mark(ns_handle* h, const char* name, int nkernels) { mark(h, name, nker
 Marker api_marker(ns_handle* h) { return marker(h); }
 int api_build_line_tables(ns_handle* h, bool transposed, LineSys sys[3][3], double** buf) {
   return build_line_tables(h, transposed, sys, buf);
+}
+int api_build_line_chunks(ns_handle* h, bool transposed, ChunkSys csys[3][3], int halo[3], double d[3], double** buf) {
+  return build_line_chunks(h, transposed, csys, halo, d, buf);
 }
 }  // namespace ns
 

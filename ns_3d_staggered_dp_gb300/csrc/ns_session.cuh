@@ -90,6 +90,7 @@ cudaError_t api_d2h_field(ns_handle* h, double* dst, const double* src, int fiel
 void api_mark(ns_handle* h, const char* name, int nkernels);
 Marker api_marker(ns_handle* h);
 int api_build_line_tables(ns_handle* h, bool transposed, LineSys sys[3][3], double** buf);
+int api_build_line_chunks(ns_handle* h, bool transposed, ChunkSys csys[3][3], int halo[3], double d[3], double** buf);
 void api_free_adjoint(ns_handle* h);
 }  // namespace ns
 
@@ -129,7 +130,8 @@ struct HostChunkSys {
   double lc = 0, cc = 0, d = 1;  // d: 1 / converged pivot (the right-hand sides' scale)
   int c0 = 0, c1 = 0, lo = 0, m = 0, wrap_lo = 0, wrap_hi = 0, periodic = 0, halo = 0;
 };
-HostChunkSys build_chunk_system(int n, int bc, double h, double dt, double nu, bool normal, int closure);
+HostChunkSys build_chunk_system(int n, int bc, double h, double dt, double nu, bool normal, int closure,
+                                bool transposed = false);
 // The CN system of one sweep axis (mat_CN / mat_CN_tridiagonal,
 // NS_functions.f90:1245-1342) for n cells with velocity code bc; normal: the
 // swept field is staggered along the axis (ns_api.cu).
