@@ -65,30 +65,28 @@ ALG_DOUBLES = {
     "tri_y_solve": 2.0,   # read + write half spectrum (line solves along the wall axis)
 }
 
-# FP64 instructions per cell of each kernel (thread-level, adds and multiplies
-# issued as DFMA), from ncu's sm__sass_thread_inst_executed_op_dfma_pred_on.sum
-# of this build's kernels at 256^3 divided by the cells of one launch.
+# FP64 instructions per cell of each kernel (thread-level), from ncu's
+# smsp__sass_thread_inst_executed_op_{dfma,dadd,dmul}_pred_on.sum of this
+# build's kernels at 128^3 divided by the cells of one launch.  (The stencils
+# and transforms run on the integer pipes: what is left are the conversions
+# back, the divergence, the line solves and the correction.)
 FP64_PER_CELL = {
-    "predict": 62.7, "adi_x": 9.5, "adi_y": 9.5, "adi_z": 9.5, "fft_x_fwd": 18.8, "fft_y_fwd": 11.2,
-    "fft_z_solve": 23.4, "fft_y_inv": 11.2, "fft_x_inv": 12.7, "correct": 7.2,
+    "predict": 12.0, "adi_x": 7.9, "adi_y": 7.9, "adi_z": 7.9, "fft_x_fwd": 6.1, "fft_y_fwd": 2.1,
+    "cyc_z_solve": 5.6, "fft_y_inv": 2.1, "fft_x_inv": 2.1, "correct": 7.3,
 }
 
 
 def fp64_per_cell(kernel, n):
-    """FP64 instructions per cell of a step kernel at n^3; the cyclic z line
-    solves do 10 per complex unknown, (n/2+1)/n complex unknowns per cell."""
-    if kernel == "cyc_z_solve":
-        return 10.0 * (n // 2 + 1) / n
+    """FP64 instructions per cell of a step kernel (0 for kernels not measured)."""
     return FP64_PER_CELL.get(kernel, 0.0)
+
+
 FP64_LANES_PER_CLK_SM = 2  # DFMA issue rate of this part (ncu ..._op_dfma_pred_on.sum.peak_sustained)
 
-# DRAM bytes per launch at 256^3 (dram__bytes_read.sum + dram__bytes_write.sum)
-# from one ncu capture of each kernel of this build's step.
-NCU_TRAFFIC_256 = {
-    "predict": 1659.0e6, "adi_x": 1574.2e6, "adi_y": 1486.3e6, "adi_z": 1480.0e6,
-    "fft_x_fwd": 533.7e6, "fft_y_fwd": 213.0e6, "fft_z_solve": 293.6e6, "fft_y_inv": 213.0e6,
-    "fft_x_inv": 219.9e6, "correct": 1112.1e6,
-}
+# DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) of one
+# ncu capture of the predictor and its pass over the plane maxima at 128^3,
+# times the 8 times as many cells.
+NCU_TRAFFIC_256 = {"predict": 8 * 226.5e6}
 
 
 @functools.lru_cache(maxsize=2)
@@ -933,7 +931,8 @@ def run_ours(args):
         "roofline": {"bound": "hbm", "kernel": dname, "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
                      "frac": achieved / hbm_peak, "traffic": traffic, "peak_source": peak_src,
                      "alg_bytes_per_launch": alg_bytes, "ms_per_launch": per_launch_ms,
-                     "note": "the step is bound by the FP64 pipe, not HBM, on this part: see the fp64 object"},
+                     "note": "the step is bound by instruction issue (FP64 and integer), not HBM, on this part: see the "
+                             "fp64 object"},
         "fp64": fp64_roof,
         "kernel_ms_per_step": {k: v[0] / 2 for k, v in sorted(prof.items(), key=lambda kv: -kv[1][0])},
         "kernel_share": {k: v[0] / total_prof for k, v in prof.items()},
