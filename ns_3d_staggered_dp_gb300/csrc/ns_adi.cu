@@ -898,7 +898,7 @@ cudaError_t launch_adi_line_chunk(const AdiArgs& a, int m, cudaStream_t st) {
 cudaError_t launch_adi_chunks(int axis, const AdiArgs& a, cudaStream_t st) {
   const int m = std::max(a.ch[0].m, std::max(a.ch[1].m, a.ch[2].m));
   const long long cells = 3LL * (a.L.nx + 2) * (a.L.ny + 2) * (a.L.nz + 2);
-  const int W = a.halo <= 8 ? 8 : (a.halo <= 12 ? 12 : 16);
+  const int W = std::max(a.halo, 8);
   auto work = [&](int c) { return (m + c - 1) / c * (c + W); };
   const int ch = cells / 32 < 40000 && m <= 16 * line_chunks_max(16) ? 16 : (work(26) < work(32) ? 26 : 32);
   bool fits = true;
@@ -907,9 +907,9 @@ cudaError_t launch_adi_chunks(int axis, const AdiArgs& a, cudaStream_t st) {
 #define NS_ADI_LINE(A, C, H) \
   if (axis == A && ch == C && W == H) return launch_adi_line_chunk<A, C, H>(a, m, st);
 #define NS_ADI_LINES(C, H) NS_ADI_LINE(0, C, H) NS_ADI_LINE(1, C, H) NS_ADI_LINE(2, C, H)
-  NS_ADI_LINES(16, 8) NS_ADI_LINES(16, 12) NS_ADI_LINES(16, 16)
-  NS_ADI_LINES(32, 8) NS_ADI_LINES(32, 12) NS_ADI_LINES(32, 16)
-  NS_ADI_LINES(26, 8) NS_ADI_LINES(26, 12) NS_ADI_LINES(26, 16)
+  NS_ADI_LINES(16, 8) NS_ADI_LINES(16, 10) NS_ADI_LINES(16, 12) NS_ADI_LINES(16, 16)
+  NS_ADI_LINES(32, 8) NS_ADI_LINES(32, 10) NS_ADI_LINES(32, 12) NS_ADI_LINES(32, 16)
+  NS_ADI_LINES(26, 8) NS_ADI_LINES(26, 10) NS_ADI_LINES(26, 12) NS_ADI_LINES(26, 16)
 #undef NS_ADI_LINES
 #undef NS_ADI_LINE
   return cudaErrorInvalidValue;
