@@ -3,10 +3,14 @@
 // mat_CN_tridiagonal).
 //
 // All lines of a sweep share one matrix, so its LU factors (no pivoting) are
-// precomputed on the host (ns_api.cu) and read as broadcast loads.  Per
-// unknown the solve is one FMA forward and one multiply + one FMA backward.
-// One thread solves one line; the sweep reads the line from one buffer and
-// writes it to another (fixed ping-pong roles, see ns_api.cu).
+// precomputed on the host (ns_api.cu) and read as broadcast loads.  A sweep
+// reads the lines from one buffer and writes them to another (fixed ping-pong
+// roles, see ns_api.cu).
+//
+// A step's sweeps solve a line in chunks ("Chunked sweeps" below).  The whole
+// lines that follow, one thread each, one FMA forward and one multiply + one
+// FMA backward an unknown, serve the sweeps whose unscaled result is handed
+// out (ns_adi, keep_sweeps), large viscous numbers, and the batch.
 //
 // y and z sweeps: a persistent kernel, lanes over consecutive x so every
 // access of the forward and backward walks is coalesced, right-hand sides

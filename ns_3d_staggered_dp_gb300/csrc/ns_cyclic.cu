@@ -21,8 +21,8 @@
 // spectrum, 10 FP64 instructions a complex unknown (the Thomas walk over
 // tabulated factors that it replaces: the same, one thread a line, 24 bytes of
 // tables an unknown).  A step's solve takes 10 us at 32^3 (the walk 23), 12 at
-// 64^3 (42), 33 at 128^3 (79) and 182 at 256^3 (187), where the FP64 unit is
-// 60% busy and the loads of the segments hide the rest badly.
+// 64^3 (42), 33 at 128^3 (79) and 182 at 256^3 (187), with the FP64 unit
+// 82% busy at 128^3.
 //
 // The mode (0, 0) is singular (rho = 1): the FFT solve drops its mean
 // (lambda(0) = +Inf), i.e. gives the zero-mean solution of the system with

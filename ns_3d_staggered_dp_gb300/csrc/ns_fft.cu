@@ -8,8 +8,9 @@
 //               x-line (an nx/2-point complex FFT of the packed even/odd
 //               samples and the split into nx/2+1 bins)
 //   y-forward : complex FFT along y
-//   z-solve   : complex FFT along z, multiply by 1/(lambda * scale), inverse
-//               FFT along z, all on the line held on chip
+//   z-solve   : cyclic line solves (ns_cyclic.cu), or complex FFT along z,
+//               multiply by 1/(lambda * scale), inverse FFT along z on the
+//               line held on chip (poisson_z = 1)
 //   y-inverse, x-inverse (c2r, writes dp slots 1..nx)
 // A line of N = R1*R2 points is transformed in two register passes
 // ("four-step"): R1 threads each do an R2-point DFT, a twiddle multiply and a
@@ -24,8 +25,9 @@
 // y forward 0.112 ms (0.372), y inverse 0.108 (0.371), x inverse 0.117
 // (0.440): integer issue at half of the slots beside the FP64 pipe at 50% (the
 // conversions back), DRAM at 2 TB/s; the FP64 transforms held that pipe at
-// 85-90%.  x forward 0.297 (0.626): the divergence and the conversions back,
-// 18 FP64 instructions a cell pair, hold the pipe at 75%.
+// 85-90%.  x forward 0.257 (0.626): the divergence holds the FP64 pipe at 57%, at
+// two CTAs an SM its loads' latency shows; its results go back on the integer
+// pipes (with two FP64 instructions each 0.300).
 #include "ns_fft_core.cuh"
 #include "ns_internal.cuh"
 #include "ns_kernels.cuh"

@@ -26,8 +26,7 @@
 // What bounds it: the FP64 stencils issue 62.7 FP64 instructions a cell, one
 // per 64 clocks and SM partition: 2.09 ms at 256^3, 83% of that pipe.  The
 // integer stencils take about 900 integer issue clocks a warp of cells beside
-// 10 FP64 instructions: 0.76 ms, plus 0.06 ms for the plane maxima; issue
-// slots 51% busy.  TY = 8 at three CTAs per SM (72 registers) leaves room to
+// 12 FP64 instructions: 0.77 ms with the plane maxima; issue slots 51% busy.  TY = 8 at three CTAs per SM (72 registers) leaves room to
 // hold the next plane's and the history's loads in flight; TY = 16 at two CTAs
 // (56 registers) waited for them at 1.9 ms.
 #include <algorithm>
