@@ -671,9 +671,36 @@ __global__ void __launch_bounds__(TX*(TY + 1)) predict_tma_kernel(PredictArgs a,
                                                  blockIdx.y, k0, k1, &mu, &mv, &mw);
 }
 
-// Largest magnitude (high word) of each z plane of u, v, w: CTA (plane, field), a warp per row,
-// four rows at once: with one row's loads in flight the predictor stage takes 831 us at 256^3
-// and 134 at 128^3, so 774 and 124.
+// Whether the stencils of an output read slot (i, j, k) of field f.  The other
+// slots (most edges of the box; the extra slot of a wall axis) hold whatever
+// the caller's arrays hold there, and must not set a block exponent.  With a
+// the field's own axis and b another one: its ghosts along b are read beside
+// the field's own faces [lo, n], the low ones also beside every face in
+// [1, n + 1] when b's lowest face has an output.
+__device__ __forceinline__ bool slot_read(const PredictArgs& a, int f, int i, int j, int k) {
+  const int pos[3] = {i, j, k}, n[3] = {a.L.nx, a.L.ny, a.L.nz}, lo[3] = {a.ulo, a.vlo, a.wlo};
+  const int p = f == 0 ? i : f == 1 ? j : k, np = f == 0 ? n[0] : f == 1 ? n[1] : n[2];
+  const int lp = f == 0 ? lo[0] : f == 1 ? lo[1] : lo[2];
+  int ghosts = 0, first = lp - 1, last = np + 1;
+#pragma unroll
+  for (int b = 0; b < 3; ++b) {
+    if (b == f) continue;
+    const bool low = pos[b] == 0, high = pos[b] > n[b];
+    ghosts += low || high;
+    if (high || (low && lo[b] > 1)) {
+      first = lp;
+      last = np;
+    } else if (low) {
+      first = 1;
+    }
+  }
+  return ghosts < 2 && p >= first && p <= last;
+}
+
+// Largest magnitude (high word) of the slots of each z plane of u, v, w that
+// are read: CTA (plane, field), a warp per row, four rows at once: with one
+// row's loads in flight the predictor stage takes 831 us at 256^3 and 134 at
+// 128^3, so 774 and 124.
 constexpr int kMaxThreads = 512;
 __device__ __forceinline__ void plane_max_body(const PredictArgs& a, int k, int f) {
   const Layout& L = a.L;
@@ -690,7 +717,9 @@ __device__ __forceinline__ void plane_max_body(const PredictArgs& a, int k, int 
       unsigned h[RJ];
 #pragma unroll
       for (int q = 0; q < RJ; ++q)
-        h[q] = j + q * NW < ny2 ? (unsigned)__double2hiint(__ldg(row + L.sy * (q * NW) + i)) & 0x7fffffffu : 0u;
+        h[q] = j + q * NW < ny2 && slot_read(a, f, i, j + q * NW, k)
+                   ? (unsigned)__double2hiint(__ldg(row + L.sy * (q * NW) + i)) & 0x7fffffffu
+                   : 0u;
 #pragma unroll
       for (int q = 0; q < RJ; ++q) m = max(m, h[q]);
     }
