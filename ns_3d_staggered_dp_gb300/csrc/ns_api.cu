@@ -694,7 +694,7 @@ PredictArgs predict_args(ns_handle* h) {
     const double d = h->adi_d[0] * h->adi_d[1] * h->adi_d[2];
     for (double* q : {&a.c0, &a.ca, &a.cb, &a.cc, &a.cu, &a.cC, &a.cP, &a.dt, &a.gpx, &a.gpy, &a.gpz}) *q *= d;
   }
-  set_predict_fixed(a, c.scheme, h->pmax);
+  set_predict_fixed(a, c.scheme);
   return a;
 }
 
@@ -812,7 +812,7 @@ int enqueue_step(ns_handle* h, bool first, cudaEvent_t after_predict = nullptr) 
   const ns_config& c = h->cfg;
   PredictArgs a = predict_args(h);
   NS_CUDA(h, launch_predict(a, c.scheme, first, c.dp_flag != 0, 0, h->stream, &h->tma));
-  mark(h, "predict", 2);
+  mark(h, "predict");
   if (after_predict) NS_CUDA(h, cudaEventRecord(after_predict, h->stream));
   return enqueue_tail(h, false);
 }
@@ -1267,7 +1267,6 @@ void free_all(ns_handle* h) {
   for (cudaEvent_t e : h->ev_slab) cudaEventDestroy(e);
   for (cudaEvent_t e : h->trace_pool) cudaEventDestroy(e);
   if (h->tw) cudaFree(h->tw);
-  if (h->pmax) cudaFree(h->pmax);
   if (h->adi_chunk_buf) cudaFree(h->adi_chunk_buf);
   if (h->diag_bits) cudaFree(h->diag_bits);
   if (h->dev_err) cudaFree(h->dev_err);
@@ -1394,7 +1393,6 @@ int ns_create(const ns_config* cfg, ns_handle** out) {
       for (int f = 0; f < 4; ++f)
         for (int d = 0; d < 2; ++d) h->faces[set].ax[a].f[f][d] = h->face_buf + face_offset(h->L, set, a, f, d);
   if (cudaMalloc(&h->diag_bits, sizeof(unsigned long long)) != cudaSuccess) return bail(NS_ERR_NOMEM);
-  if (cudaMalloc(&h->pmax, 3 * (size_t)(h->L.nz + 2) * sizeof(unsigned)) != cudaSuccess) return bail(NS_ERR_NOMEM);
   if (cudaMalloc(&h->dev_err, sizeof(int)) != cudaSuccess) return bail(NS_ERR_NOMEM);
   if (cudaMemsetAsync(h->dev_err, 0, sizeof(int), h->stream) != cudaSuccess) return bail(NS_ERR_CUDA);
   // The predictor prefetches its planes into registers.  NS_PREDICT_TMA=1 in
@@ -1651,7 +1649,7 @@ int ns_step_host(ns_handle* h, const double* u, const double* v, const double* w
       int kc = KC;
       while (kc > 2 && kc > (e - pred_done) / 4) kc /= 2;
       NS_CUDA(h, launch_predict_planes(pa, c.scheme, first, c.dp_flag != 0, pred_done, e, kc, h->stream, &h->tma));
-      mark(h, "predict", 2);
+      mark(h, "predict");
       trace_mark(h, h->stream, "predict", s, lo, hi);
       pred_done = e;
       // the history of the finished planes is final: out on the copy stream

@@ -397,10 +397,6 @@ struct ns_batch {
   // x), and those of their boundary cells' pressure-BC terms
   std::vector<Range> div_rng, bc_rng;                   // [set]
   std::vector<std::vector<Range>> sub_div_rng, sub_bc_rng;  // [set][sub]
-  // the planes whose largest velocities the predictor takes first (item: subdomain, plane)
-  std::vector<Range> pm_rng;                            // [set]
-  std::vector<std::vector<Range>> sub_pm_rng;           // [set][sub]
-  unsigned* pmax = nullptr;                             // 3 (nz + 2) words per subdomain
   bool iso = false;                                     // the predictor's axis coefficients are equal
   int pred_kc = 0;                                      // its planes per CTA
   std::vector<std::vector<int>> active;                 // [set] -> subdomains
@@ -471,11 +467,7 @@ cudaError_t launch_stage_kernel(ns_batch* b, int set, int stage, bool first, cud
         e = cudaGetLastError();
         break;
       case ST_PREDICT:
-        {
-          const ns_batch::Range& m = loop ? b->sub_pm_rng[set][act[k]] : b->pm_rng[set];
-          e = launch_predict_batch(b->d_pred[v], p, cnt, b->d_items + m.off, m.cnt, b->iso, c.scheme, first,
-                                   c.dp_flag != 0, want > 0 ? grid : 0, st);
-        }
+        e = launch_predict_batch(b->d_pred[v], p, cnt, b->iso, c.scheme, first, c.dp_flag != 0, want > 0 ? grid : 0, st);
         break;
       case ST_HIST:
         hist_kernel<<<grid, kChunk, 0, st>>>(b->d_geo, p, cnt);
@@ -645,7 +637,6 @@ int ns_batch_destroy(ns_batch* b) {
   if (b->tables) cudaFree(b->tables);
   if (b->adi_tab) cudaFree(b->adi_tab);
   if (b->tri_tab) cudaFree(b->tri_tab);
-  if (b->pmax) cudaFree(b->pmax);
   if (b->snaps) cudaFree(b->snaps);
   if (b->snap_mean) cudaFree(b->snap_mean);
   if (b->p_prev) cudaFree(b->p_prev);
@@ -847,19 +838,14 @@ int ns_batch_create(const ns_batch_config* cfg, const ns_subdomain* subs, int n,
     if (cudaMalloc(&b->tri_tab, std::max<size_t>(t, 1) * sizeof(double2)) != cudaSuccess) return bail(NS_ERR_NOMEM);
   }
 
-  // the predictor's plane maxima and its planes per CTA
-  std::vector<size_t> pm_off(n);
+  // the predictor's planes per CTA
   {
-    size_t t = 0;
     std::vector<std::pair<long long, int>> boxes;
     for (int i = 0; i < n; ++i) {
-      pm_off[i] = t;
-      t += 3 * ((size_t)subs[i].nz + 2);
       int gx, gy, gz;
       predict_tiles(b->L[i], 1, gx, gy, gz);
       boxes.emplace_back((long long)gx * gy, gz);
     }
-    if (cudaMalloc(&b->pmax, t * sizeof(unsigned)) != cudaSuccess) return bail(NS_ERR_NOMEM);
     b->pred_kc = predict_chunk(boxes);
   }
 
@@ -975,7 +961,7 @@ int ns_batch_create(const ns_batch_config* cfg, const ns_subdomain* subs, int n,
       a.us = us; a.vs = vs; a.ws = ws;
       a.hx = g.fld[4]; a.hy = g.fld[5]; a.hz = g.fld[6];
       set_predict_coeffs(a, bc3, c.dx, c.dy, c.dz, dt, c.nu);
-      set_predict_fixed(a, c.scheme, b->pmax + pm_off[i]);
+      set_predict_fixed(a, c.scheme);
       a.kc = b->pred_kc;
       b->iso = a.iso != 0;
       BatchSpecArgs& sa = spec[v][i];
@@ -1125,18 +1111,6 @@ int ns_batch_create(const ns_batch_config* cfg, const ns_subdomain* subs, int n,
       for (int q = 0; q < nq; ++q) all.push_back(BatchItem{i, q, 0, 0});
     }
     b->bc_rng[set].cnt = (int)((long long)all.size() - b->bc_rng[set].off);
-  }
-  b->pm_rng.assign(nsets, ns_batch::Range{});
-  b->sub_pm_rng.assign(nsets, std::vector<ns_batch::Range>(n));
-  for (int set = 0; set < nsets; ++set) {
-    b->pm_rng[set].off = (long long)all.size();
-    for (int i : b->active[set]) {
-      const int np = b->L[i].nz + 2;
-      b->sub_pm_rng[set][i].off = (long long)all.size();
-      b->sub_pm_rng[set][i].cnt = np;
-      for (int q = 0; q < np; ++q) all.push_back(BatchItem{i, q, 0, 0});
-    }
-    b->pm_rng[set].cnt = (int)((long long)all.size() - b->pm_rng[set].off);
   }
   b->gather_rng.off = (long long)all.size();
   for (int i = 0; i < n; ++i) {

@@ -56,10 +56,9 @@ struct PredictArgs {
   // the planes 1 + koff + kc*bz .. up to kend (exclusive; 0: nz + 1).
   int kc, koff, kend;
   int* err;  // device word set to 1 when a bounded wait of the tile loader gave up (may be null)
-  // Block fixed-point stencils (ns_predict.cu): the largest magnitudes of u, v, w per z plane (high
-  // words, [field][plane], nz + 2 planes each; null: FP64 stencils), and the coefficients in units of
+  // Block fixed-point stencils (ns_predict.cu; fixed 0: FP64 stencils): the coefficients in units of
   // 2^-60: -(1/4h) of each axis times 2^-kq, and the viscous coefficient of each axis times 2^-kv.
-  unsigned* pmax;
+  int fixed;
   long long q60[3], v60[3];
   int kq, kv;
   int iso;  // 1: the three axes have the same coefficients
@@ -109,8 +108,8 @@ __device__ __forceinline__ double predictor_combine(const PredictArgs& a, const 
   }
 }
 
-// The fixed-point coefficients of a scheme (host; pmax is kept null when a coefficient is not finite).
-void set_predict_fixed(PredictArgs& a, int scheme, unsigned* pmax);
+// The fixed-point coefficients of a scheme (host; fixed is 0 when a coefficient is not finite or out of range).
+void set_predict_fixed(PredictArgs& a, int scheme);
 size_t predict_smem_bytes();
 cudaError_t launch_predict(const PredictArgs& a, int scheme, bool first, bool dpf, int mode, cudaStream_t st,
                            const PredTma* tma = nullptr);
@@ -125,10 +124,9 @@ int predict_chunk(const std::vector<std::pair<long long, int>>& boxes);
 // Predictor tiles of one box in chunks of kc planes (work items of the batched launch; kc is the
 // subdomain's PredictArgs::kc).
 void predict_tiles(const Layout& L, int kc, int& gx, int& gy, int& gz);
-// Batched predictor over the items (grid <= 0: one wave of resident CTAs), after the plane maxima of
-// the items `planes` (subdomain, plane bx; all with pmax).
-cudaError_t launch_predict_batch(const PredictArgs* tab, const BatchItem* items, int n_items, const BatchItem* planes,
-                                 int n_planes, bool iso, int scheme, bool first, bool dpf, int grid, cudaStream_t st);
+// Batched predictor over the items (grid <= 0: one wave of resident CTAs).
+cudaError_t launch_predict_batch(const PredictArgs* tab, const BatchItem* items, int n_items, bool iso, int scheme,
+                                 bool first, bool dpf, int grid, cudaStream_t st);
 
 // ---------------------------------------------------------------------------
 // Boundary fills (ns_bc.cu)

@@ -25,11 +25,16 @@
 //
 // What bounds it: the FP64 stencils issue 62.7 FP64 instructions a cell, one
 // per 64 clocks and SM partition: 2.09 ms at 256^3, 83% of that pipe.  The
-// integer stencils take about 900 integer issue clocks a warp of cells beside
-// 12 FP64 instructions: 0.77 ms with the plane maxima; issue slots 51% busy.  TY = 8 at three CTAs per SM (72 registers) leaves room to
-// hold the next plane's and the history's loads in flight; TY = 16 at two CTAs
-// (56 registers) waited for them at 1.9 ms.
+// integer stencils take about 950 integer issue clocks a warp of cells beside
+// 12 FP64 instructions: 0.81 ms with the block exponents, half of the issue
+// slots busy.  TY = 8 at three CTAs per SM (72 registers) leaves room to hold
+// the next plane's and the history's loads in flight; TY = 16 at two CTAs (56
+// registers) waited for them at 1.9 ms.  Exponents of whole x-y planes, from a
+// pass of their own, without the test for cells far below them took 0.77 ms
+// (128^3 0.123 against 0.135 now, 128^3 with walls 0.130 against 0.158, FP64
+// 0.309) and lost the quiet cells' digits.
 #include <algorithm>
+#include <cstddef>
 #include <cmath>
 
 #include <cuda.h>
@@ -70,7 +75,7 @@ struct PredSmem {
 
 // The fixed-point stencils' planes: the same ring and products as integers.
 constexpr int GRP = 16;      // cell planes of one block exponent
-constexpr int NWIN = 3;      // groups that a CTA's planes can touch
+constexpr int NWARP = TY + 1;
 struct FxPredSmem {
   long long f[3][RING][SYH][SXW];
   long long sx2[PYH][PXW];
@@ -80,16 +85,18 @@ struct FxPredSmem {
   long long qxz[2][PYH][PXW];
   long long qyz[2][PYH][PXW];
 };
-struct FxTail {  // behind the planes: the groups' exponents, and the tile loader's barriers
-  int e[NWIN][3];
-  int pad;
-  unsigned long long bar[2];
+struct FxTail {  // behind the planes
+  unsigned part[3][NWARP];       // largest magnitude of each field, per warp
+  unsigned quiet[TY][GRP][3];    // cells left to the FP64 stencils: lanes of row, plane and component
+  unsigned short list[TY][64];   // those a row's warp works on
+  unsigned long long bar[2];     // the tile loader's barriers
 };
 struct FxRaw {  // tile loader: two planes of doubles, each field's box on a 128-byte boundary
   double f[2][3][SYH][SXW];
 };
 static_assert(sizeof(double) * SYH * SXW % 128 == 0, "boxes of the tile loader stay 128-byte aligned");
 static_assert(sizeof(FxPredSmem) == sizeof(PredSmem), "one shared-memory area serves both stencils");
+static_assert(offsetof(FxTail, bar) % 8 == 0, "the barriers are 8-byte aligned");
 
 // ---- tile loader (TMA): one thread fills a staging slot with three 40 x 10 x 1
 // boxes (u, v, w) and arms the slot's mbarrier with their byte count ----
@@ -379,25 +386,172 @@ __device__ __forceinline__ void predict_body(const PredictArgs& a, PredSmem& S, 
 // ---------------------------------------------------------------------------
 // The predictor on block fixed-point integers (MODE 0)
 // ---------------------------------------------------------------------------
-// The cell planes 16 g + 1 .. 16 g + 16 form a group; the exponents of the
-// largest magnitudes of the planes their stencils read (16 g .. 16 g + 17),
-// one per field, are its block exponents.  They depend on the fields alone,
-// so the results do not depend on how the box is cut into launches, chunks
-// or tiles.  (Exponents of each plane's own three planes changed every few
-// planes of a turbulent field, and every change is a new warm-up: 3.0 ms at
-// 256^3.)  A velocity takes 59 bits, a two-point sum 60, a product 60 (its
-// unit is 2^-60 of four times the largest velocity squared, rounded).  Per
-// component the convection C and the viscous increment L are formed as
-// integers (the axis coefficients in units of 2^-60), brought back to
-// doubles, and combined with u itself and the AB2 history in FP64: u* is u
-// plus increments, as accurate for small u as for large.  A group that reads
-// an Inf, a NaN or a velocity beyond 2^250 takes the FP64 stencils; velocities
-// below 2^-250 count as fixed-point values of that exponent.
+// The cell planes 16 g + 1 .. 16 g + 16 of a tile form a block; the exponents
+// of the largest magnitudes that its stencils read (planes 16 g .. 16 g + 17,
+// one row and column around the tile), one per field, are its block exponents
+// (tile_exponents).  They depend on the fields alone, so the results do not
+// depend on how the box is cut into launches or chunks.  (Exponents of each
+// plane's own three planes changed every few planes of a turbulent field, and
+// every change is a new warm-up: 3.0 ms at 256^3.)  A velocity is rounded to
+// 59 bits (exact down to 2^-6 of the largest), a two-point sum takes 60, a
+// product 60 (its unit is 2^-60 of four times the largest velocity squared,
+// rounded).  Per component the convection C and the viscous increment L are
+// formed as integers (the axis coefficients in units of 2^-60), brought back
+// to doubles, and combined with u itself and the AB2 history in FP64.
+//
+// What an integer lacks is a double's relative accuracy far below the block's
+// largest value.  So a cell whose component is below 2^-6 of it in all of the
+// 7 points of its stencil, or whose component times the largest velocity
+// beside it is below 2^-9 of the block's, gets the FP64 stencils instead
+// (cell_fp64): they are marked here and worked off behind the block's planes,
+// 32 marked cells of a row at a time.  What is left has a rounding error, in
+// units of the local velocity (product, for C), of 0.3 to 1 times that of the
+// FP64 stencils in the mean over turbulent and Taylor-Green fields and jets
+// beside quiet fluid, and of 4e-15 at most (theirs: 1e-15).  Of a turbulent
+// field no cell in ten thousand is marked, of a Taylor-Green vortex one in
+// fifty (the surroundings of its axes), of a quiet region beside a jet those
+// in the jet's own tiles; a field that is zero in a whole block marks none.
+//
+// A block that reads an Inf, a NaN or a velocity beyond 2^250, or whose
+// largest one is below 2^-250, takes the FP64 stencils altogether.
 constexpr int kFxB = 59;                    // bits of a velocity
 constexpr int kFxLo = 773, kFxHi = 1273;    // biased exponents of the fixed-point stencils
+constexpr unsigned kQuietOwn = 1u << (kFxB - 32 - 6 - 1);            // of high words below 2^(kFxB - 32)
+constexpr unsigned kQuietProduct = 1u << (2 * (kFxB - 32) - 32 - 9 - 2);  // of the product's high word
 struct FxPlane {
-  int e[3];  // biased block exponents of u, v, w
+  int e[3];      // biased block exponents of u, v, w
+  unsigned least[3], least_product[3];  // high words (of products) below these: FP64 stencils
 };
+
+// Whether the stencils of an output read slot (i, j, k) of field f.  The other
+// slots (most edges of the box; the extra slot of a wall axis) hold whatever
+// the caller's arrays hold there, and must not set a block exponent.  With a
+// the field's own axis and b another one: its ghosts along b are read beside
+// the field's own faces [lo, n], the low ones also beside every face in
+// [1, n + 1] when b's lowest face has an output.
+__device__ __forceinline__ bool slot_read(const PredictArgs& a, int f, int i, int j, int k) {
+  const int pos[3] = {i, j, k}, n[3] = {a.L.nx, a.L.ny, a.L.nz}, lo[3] = {a.ulo, a.vlo, a.wlo};
+  const int p = f == 0 ? i : f == 1 ? j : k, np = f == 0 ? n[0] : f == 1 ? n[1] : n[2];
+  const int lp = f == 0 ? lo[0] : f == 1 ? lo[1] : lo[2];
+  int ghosts = 0, first = lp - 1, last = np + 1;
+#pragma unroll
+  for (int b = 0; b < 3; ++b) {
+    if (b == f) continue;
+    const bool low = pos[b] == 0, high = pos[b] > n[b];
+    ghosts += low || high;
+    if (high || (low && lo[b] > 1)) {
+      first = lp;
+      last = np;
+    } else if (low) {
+      first = 1;
+    }
+  }
+  return ghosts < 2 && p >= first && p <= last;
+}
+
+// This thread's two column pairs of a plane (of 3 fields x 10 rows x 18 pairs).
+constexpr int NV = (TX + 4) / 2, NPAIR = 3 * NV * SYH, NTHR = TX * NWARP;
+static_assert(NPAIR <= 2 * NTHR, "two pairs per thread cover a plane");
+struct FxPairs {
+  const double* src[2];
+  int f[2], yy[2], xv[2];
+  bool two;  // the second one is a pair of its own
+};
+__device__ __forceinline__ FxPairs tile_pairs(const PredictArgs& a, int i0, int j0) {
+  FxPairs p;
+  const int tid = threadIdx.x + TX * threadIdx.y;
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const int e = min(tid + q * NTHR, NPAIR - 1);
+    p.f[q] = e / (NV * SYH);
+    p.yy[q] = e / NV % SYH;
+    p.xv[q] = e % NV;
+    p.src[q] = (p.f[q] == 0 ? a.u : p.f[q] == 1 ? a.v : a.w) +
+               a.L.at(i0 - 2 + 2 * p.xv[q], clampi(j0 - 1 + p.yy[q], 0, a.L.ny + 1), 0);
+  }
+  p.two = tid + NTHR < NPAIR;
+  return p;
+}
+
+// The largest magnitudes (high word; 0 for zeros alone) of the tile's group g
+// of planes, per field.  A pass of its own over planes that the stencils are
+// about to read (they come from L2 then): six planes of a thread in flight.
+__device__ __forceinline__ void tile_exponents(const PredictArgs& a, FxTail& T, int i0, int j0, int g,
+                                               unsigned (&top)[3]) {
+  const Layout& L = a.L;
+  const FxPairs pr = tile_pairs(a, i0, j0);
+  const int kg = GRP * g, np = min(GRP + 2, L.nz + 2 - kg);
+  unsigned m[2] = {0u, 0u};
+  // whether a pair's two slots are read: a bit for plane 0, plane 1, the other inner ones, nz + 1
+  // (plane 1 apart for w, whose own axis this is)
+  unsigned rd[2][2];
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+      const int i = i0 - 2 + 2 * pr.xv[q] + x, j = j0 - 1 + pr.yy[q];
+      rd[q][x] = 0u;
+      if (i < i0 - 1 || i > min(i0 + TX, L.nx + 1) || j > L.ny + 1) continue;
+      rd[q][x] = (slot_read(a, pr.f[q], i, j, 0) ? 1u : 0u) | (slot_read(a, pr.f[q], i, j, 1) ? 2u : 0u) |
+                 (slot_read(a, pr.f[q], i, j, 2) ? 4u : 0u) | (slot_read(a, pr.f[q], i, j, L.nz + 1) ? 8u : 0u);
+    }
+#pragma unroll 1
+  for (int p0 = 0; p0 < np; p0 += 6) {
+    double2 d[6][2];
+#pragma unroll
+    for (int p = 0; p < 6; ++p) {
+      const long long o = L.sz * (long long)(kg + min(p0 + p, np - 1));
+#pragma unroll
+      for (int q = 0; q < 2; ++q) d[p][q] = *reinterpret_cast<const double2*>(pr.src[q] + o);
+    }
+#pragma unroll
+    for (int p = 0; p < 6; ++p) {
+      const int k = kg + min(p0 + p, np - 1);
+      const unsigned plane = k == 0 ? 1u : k > L.nz ? 8u : k == 1 ? 2u : 4u;
+      auto mag = [](double v) {
+        return ((unsigned)__double2hiint(v) & 0x7fffffffu) | (__double2loint(v) != 0 ? 1u : 0u);
+      };
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        if (rd[q][0] & plane) m[q] = max(m[q], mag(d[p][q].x));
+        if (rd[q][1] & plane) m[q] = max(m[q], mag(d[p][q].y));
+      }
+    }
+  }
+#pragma unroll
+  for (int f = 0; f < 3; ++f) {
+    const unsigned r = __reduce_max_sync(0xffffffffu, max(pr.f[0] == f ? m[0] : 0u, pr.f[1] == f ? m[1] : 0u));
+    if (threadIdx.x == 0) T.part[f][threadIdx.y] = r;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int f = 0; f < 3; ++f) {
+    top[f] = 0u;
+#pragma unroll
+    for (int w = 0; w < NWARP; ++w) top[f] = max(top[f], T.part[f][w]);
+  }
+}
+
+// C (minus the convection) and the viscous increment of one component at one
+// cell in FP64: f the component at its face, g and h the two others at the
+// same slot; strides and coefficients in the order own axis, g's, h's.
+struct CellFp {
+  double C, Lv;
+};
+__device__ __noinline__ CellFp cell_fp64(const double* __restrict__ f, const double* __restrict__ g,
+                                         const double* __restrict__ h, long long s0, long long s1, long long s2,
+                                         double c0, double c1, double c2, double v0, double v1, double v2) {
+  const double x = f[0], a0 = f[-s0], b0 = f[s0], a1 = f[-s1], b1 = f[s1], a2 = f[-s2], b2 = f[s2];
+  CellFp r;
+  r.C = ((x + b0) * (x + b0) - (a0 + x) * (a0 + x)) * c0;
+  r.C = fma((x + b1) * (g[s1 - s0] + g[s1]) - (a1 + x) * (g[-s0] + g[0]), c1, r.C);
+  r.C = fma((x + b2) * (h[s2 - s0] + h[s2]) - (a2 + x) * (h[-s0] + h[0]), c2, r.C);
+  r.Lv = fma(v0, fma(-2.0, x, a0 + b0), fma(v1, fma(-2.0, x, a1 + b1), v2 * fma(-2.0, x, a2 + b2)));
+  return r;
+}
+
+// Bits in use of a velocity's high word.
+__device__ __forceinline__ unsigned hi_bits(long long v) { return (unsigned)abs((int)(v >> 32)); }
 
 __device__ __forceinline__ void products_fx(FxPredSmem& S, int xa, int yb, int s0, int s1, int pb, bool zonly) {
   const long long (*U0)[SXW] = S.f[0][s0], (*U1)[SXW] = S.f[0][s1];
@@ -426,28 +580,22 @@ __device__ __forceinline__ void predict_fx_planes(const PredictArgs& a, FxPredSm
   const int xa = lane + 1, yb = wy;
   const int tid = lane + TX * wy;
   const bool producer = tid == 0;
-  // this thread's two column pairs of a plane (of 3 x 10 x 18)
-  constexpr int NV = (TX + 4) / 2, NPAIR = 3 * NV * SYH, NTHR = TX * (TY + 1);
-  static_assert(NPAIR <= 2 * NTHR, "two pairs per thread cover a plane");
-  const double* src[2];
+  const FxPairs pr = tile_pairs(a, i0, j0);
   int dst[2], ee[2];
 #pragma unroll
   for (int q = 0; q < 2; ++q) {
-    const int e = min(tid + q * NTHR, NPAIR - 1);
-    const int f = e / (NV * SYH), yy = e / NV % SYH, xv = e % NV;
-    src[q] = (f == 0 ? a.u : f == 1 ? a.v : a.w) + L.at(i0 - 2 + 2 * xv, clampi(j0 - 1 + yy, 0, L.ny + 1), 0);
-    dst[q] = (f * RING * SYH + yy) * SXW + 2 * xv;
-    ee[q] = f == 0 ? P.e[0] : f == 1 ? P.e[1] : P.e[2];
+    dst[q] = (pr.f[q] * RING * SYH + pr.yy[q]) * SXW + 2 * pr.xv[q];
+    ee[q] = pr.f[q] == 0 ? P.e[0] : pr.f[q] == 1 ? P.e[1] : P.e[2];
   }
-  const bool two = tid + NTHR < NPAIR;
+  const bool two = pr.two;
   double2 r[2];
   auto fetch = [&](int k) {  // plane k on its way: into registers, or (tile loader) into its staging slot
     if (TMA) {
       if (producer) tma_plane(*raw, T, mu, mv, mw, L.nz, i0, j0, k, k & 1);
     } else {
       const long long o = L.sz * (long long)clampi(k, 0, L.nz + 1);
-      r[0] = *reinterpret_cast<const double2*>(src[0] + o);
-      if (two) r[1] = *reinterpret_cast<const double2*>(src[1] + o);
+      r[0] = *reinterpret_cast<const double2*>(pr.src[0] + o);
+      if (two) r[1] = *reinterpret_cast<const double2*>(pr.src[1] + o);
     }
   };
   auto convert = [&](int k) {  // and into the ring
@@ -464,7 +612,7 @@ __device__ __forceinline__ void predict_fx_planes(const PredictArgs& a, FxPredSm
         const int e = tid + q * NTHR;
         d = *reinterpret_cast<const double2*>(&raw->f[k & 1][e / (NV * SYH)][e / NV % SYH][2 * (e % NV)]);
       }
-      *reinterpret_cast<longlong2*>(ring + dst[q]) = make_longlong2(fx_from<kFxB>(d.x, ee[q]), fx_from<kFxB>(d.y, ee[q]));
+      *reinterpret_cast<longlong2*>(ring + dst[q]) = make_longlong2(fx_round<kFxB>(d.x, ee[q]), fx_round<kFxB>(d.y, ee[q]));
     }
   };
   // units: a velocity of field f is v 2^(e[f] - 1022 - kFxB), a product of fields f, g the product's
@@ -504,17 +652,17 @@ __device__ __forceinline__ void predict_fx_planes(const PredictArgs& a, FxPredSm
     else s = fx_mul(we - 2 * uc, vw[0]) + fx_mul(sn - 2 * uc, vw[1]) + fx_mul(bt - 2 * uc, vw[2]);
     return fx_to_int(s, e + kL);
   };
-  auto combine = [&](double uc, double Lv, double C, double prev, double* __restrict__ hist, long long g) -> double {
+  // (u* but for the pressure gradient, the new history)
+  auto combine = [&](double uc, double Lv, double C, double prev) -> double2 {
     if (SCHEME == 2) {  // AB2-CN explicit half (big_periodic_3D.f90:398-423)
       double t = fma(FIRST ? a.dt : a.cC, C, fma(a.cu, uc, Lv));  // Euler start: nu/2 diff - conv (:400-408)
       if (!FIRST) t = fma(a.cP, prev, t);
-      hist[g] = C;  // rhs_?_previous = -conv
-      return t;
+      return make_double2(t, C);  // rhs_?_previous = -conv
     }
     const double rhs = fadd(c, Lv, C);  // nu*diff - conv
-    hist[g] = SCHEME == 0 ? 0.0 : rhs;
-    if (SCHEME == 1 && !FIRST) return fma(a.e1, rhs, fma(a.e2, prev, uc));  // AB2 (:369-396)
-    return fma(a.dt, rhs, uc);  // Euler, or the Euler start of AB2
+    const double h = SCHEME == 0 ? 0.0 : rhs;
+    if (SCHEME == 1 && !FIRST) return make_double2(fma(a.e1, rhs, fma(a.e2, prev, uc)), h);  // AB2 (:369-396)
+    return make_double2(fma(a.dt, rhs, uc), h);  // Euler, or the Euler start of AB2
   };
 
   // Warm-up: planes k0-1, k0, k0+1 in the ring, k0+2 on its way; products at z-face k0.
@@ -534,6 +682,7 @@ __device__ __forceinline__ void predict_fx_planes(const PredictArgs& a, FxPredSm
   const int i = i0 + lane, j = j0 - 1 + wy;
   const bool in_xy = (wy >= 1) && (i <= L.nx) && (j <= L.ny);
   const bool act_u = in_xy && (i >= a.ulo), act_v = in_xy && (j >= a.vlo);
+  unsigned marked = 0;  // planes (from k0 on) with cells left to the FP64 stencils
   for (int k = k0; k < k1; ++k) {
     const int s0 = k & 3, s1 = (k + 1) & 3, sm = (k + 3) & 3;  // planes k, k+1, k-1
     const int pb = k & 1, pbm = (k - 1) & 1;
@@ -556,37 +705,96 @@ __device__ __forceinline__ void predict_fx_planes(const PredictArgs& a, FxPredSm
     products_fx(S, xa, yb, s0, s1, pb, false);
     if (wy == 0 && lane <= TY) products_fx(S, 0, lane, s0, s1, pb, false);
     __syncthreads();
-    if (!in_xy) continue;
-    if (act_u) {  // x-component at x-face i
-      const long long (*F)[SXW] = S.f[0][s0];
-      const double C = conv(S.sx2[yb][xa] - S.sx2[yb][xa - 1], S.qxy[yb][xa - 1] - S.qxy[yb - 1][xa - 1],
-                            S.qxz[pb][yb][xa - 1] - S.qxz[pbm][yb][xa - 1], P.e[0]);
-      const double Lv = visc(F[yb][xa + 1], F[yb][xa] + F[yb][xa + 2], F[yb - 1][xa + 1] + F[yb + 1][xa + 1],
-                             S.f[0][sm][yb][xa + 1] + S.f[0][s1][yb][xa + 1], P.e[0]);
-      double out = combine(uc, Lv, C, hu, a.hx, g);
-      if (DPF) out = fma(a.gpx, fsub(c, __ldg(a.p + g), __ldg(a.p + g - 1)), out);
-      a.us[g] = out;
+    unsigned mark = 0;  // components left to the FP64 stencils
+    if (in_xy) {
+      unsigned bits[3];  // of the 7 points of a component's stencil
+      double2 res[3];
+      auto component = [&](int f, double own, double prev, auto convection) {
+        const long long (*F)[SXW] = S.f[f][s0];
+        const long long x = F[yb][xa + 1], xw = F[yb][xa], xe = F[yb][xa + 2], xs = F[yb - 1][xa + 1],
+                        xn = F[yb + 1][xa + 1], xb = S.f[f][sm][yb][xa + 1], xt = S.f[f][s1][yb][xa + 1];
+        bits[f] = hi_bits(x) | hi_bits(xw) | hi_bits(xe) | hi_bits(xs) | hi_bits(xn) | hi_bits(xb) | hi_bits(xt);
+        const double Lv = visc(x, xw + xe, xs + xn, xb + xt, P.e[f]);
+        res[f] = combine(own, Lv, convection(), prev);
+      };
+      component(0, uc, hu, [&]() {  // at x-face i
+        return conv(S.sx2[yb][xa] - S.sx2[yb][xa - 1], S.qxy[yb][xa - 1] - S.qxy[yb - 1][xa - 1],
+                    S.qxz[pb][yb][xa - 1] - S.qxz[pbm][yb][xa - 1], P.e[0]);
+      });
+      component(1, vc, hv, [&]() {  // at y-face j
+        return conv(S.qxy[yb - 1][xa] - S.qxy[yb - 1][xa - 1], S.sy2[yb][xa] - S.sy2[yb - 1][xa],
+                    S.qyz[pb][yb - 1][xa] - S.qyz[pbm][yb - 1][xa], P.e[1]);
+      });
+      component(2, wc, hw, [&]() {  // at z-face k
+        return conv(S.qxz[pbm][yb][xa] - S.qxz[pbm][yb][xa - 1], S.qyz[pbm][yb][xa] - S.qyz[pbm][yb - 1][xa],
+                    S.sz2[pb][yb][xa] - S.sz2[pbm][yb][xa], P.e[2]);
+      });
+      unsigned near = 0;  // the largest velocity, at the largest block exponent
+#pragma unroll
+      for (int f = 0; f < 3; ++f) near |= bits[f] >> min(em - P.e[f], 31);
+      auto put = [&](int f, double* __restrict__ hist, double* __restrict__ star, long long sp, double gp) {
+        if (bits[f] < P.least[f] || __umulhi(bits[f], near) < P.least_product[f]) {
+          mark |= 1u << f;
+          return;
+        }
+        hist[g] = res[f].y;
+        star[g] = DPF ? fma(gp, fsub(c, __ldg(a.p + g), __ldg(a.p + g - sp)), res[f].x) : res[f].x;
+      };
+      if (act_u) put(0, a.hx, a.us, 1, a.gpx);
+      if (act_v) put(1, a.hy, a.vs, L.sy, a.gpy);
+      if (k >= a.wlo) put(2, a.hz, a.ws, L.sz, a.gpz);
     }
-    if (act_v) {  // y-component at y-face j
-      const long long (*F)[SXW] = S.f[1][s0];
-      const double C = conv(S.qxy[yb - 1][xa] - S.qxy[yb - 1][xa - 1], S.sy2[yb][xa] - S.sy2[yb - 1][xa],
-                            S.qyz[pb][yb - 1][xa] - S.qyz[pbm][yb - 1][xa], P.e[1]);
-      const double Lv = visc(F[yb][xa + 1], F[yb][xa] + F[yb][xa + 2], F[yb - 1][xa + 1] + F[yb + 1][xa + 1],
-                             S.f[1][sm][yb][xa + 1] + S.f[1][s1][yb][xa + 1], P.e[1]);
-      double out = combine(vc, Lv, C, hv, a.hy, g);
-      if (DPF) out = fma(a.gpy, fsub(c, __ldg(a.p + g), __ldg(a.p + g - L.sy)), out);
-      a.vs[g] = out;
+    if (__any_sync(0xffffffffu, mark)) {  // (never in warp 0)
+#pragma unroll
+      for (int f = 0; f < 3; ++f) {
+        const unsigned w = __ballot_sync(0xffffffffu, (mark >> f) & 1u);
+        if (lane == 0) T.quiet[wy - 1][k - k0][f] = w;
+      }
+      marked |= 1u << (k - k0);
     }
-    if (k >= a.wlo) {  // z-component at z-face k
-      const long long (*F)[SXW] = S.f[2][s0];
-      const double C = conv(S.qxz[pbm][yb][xa] - S.qxz[pbm][yb][xa - 1], S.qyz[pbm][yb][xa] - S.qyz[pbm][yb - 1][xa],
-                            S.sz2[pb][yb][xa] - S.sz2[pbm][yb][xa], P.e[2]);
-      const double Lv = visc(F[yb][xa + 1], F[yb][xa] + F[yb][xa + 2], F[yb - 1][xa + 1] + F[yb + 1][xa + 1],
-                             S.f[2][sm][yb][xa + 1] + S.f[2][s1][yb][xa + 1], P.e[2]);
-      double out = combine(wc, Lv, C, hw, a.hz, g);
-      if (DPF) out = fma(a.gpz, fsub(c, __ldg(a.p + g), __ldg(a.p + g - L.sz)), out);
-      a.ws[g] = out;
+  }
+  // The marked cells of this warp's row, 32 at a time.
+  __syncwarp();
+  int n = 0, f = 3, plane = 0;
+  while (marked || f < 3 || n > 0) {
+    while (n < 32 && (marked || f < 3)) {
+      if (f == 3) {
+        plane = __ffs((int)marked) - 1;
+        marked &= marked - 1;
+        f = 0;
+      }
+      const unsigned w = T.quiet[wy - 1][plane][f];
+      if ((w >> lane) & 1u)
+        T.list[wy - 1][n + __popc(w & ((1u << lane) - 1u))] = (unsigned short)(lane | f << 5 | plane << 7);
+      n += __popc(w);
+      ++f;
     }
+    __syncwarp();
+    if (lane < n) {
+      const int code = T.list[wy - 1][lane], q = (code >> 5) & 3;
+      const long long g = L.at(i0 + (code & 31), j, k0 + (code >> 7));
+      const double *fu = a.u + g, *fv = a.v + g, *fw = a.w + g;
+      const double vx = SCHEME == 2 ? a.ca : a.kx, vy = SCHEME == 2 ? a.cb : a.ky, vz = SCHEME == 2 ? a.cc : a.kz;
+      double* hist = q == 0 ? a.hx : q == 1 ? a.hy : a.hz;
+      const double own = q == 0 ? *fu : q == 1 ? *fv : *fw;
+      const double prev = SCHEME != 0 && !FIRST ? hist[g] : 0.0;
+      const CellFp r = cell_fp64(q == 0 ? fu : q == 1 ? fv : fw, q == 0 ? fv : fu, q == 2 ? fv : fw,
+                                 q == 0 ? 1 : q == 1 ? L.sy : L.sz, q == 0 ? L.sy : 1, q == 2 ? L.sy : L.sz,
+                                 q == 0 ? a.cx : q == 1 ? a.cy : a.cz, q == 0 ? a.cy : a.cx, q == 2 ? a.cy : a.cz,
+                                 q == 0 ? vx : q == 1 ? vy : vz, q == 0 ? vy : vx, q == 2 ? vy : vz);
+      double2 out = combine(own, r.Lv, r.C, prev);
+      if (DPF)
+        out.x = fma(q == 0 ? a.gpx : q == 1 ? a.gpy : a.gpz,
+                    fsub(c, __ldg(a.p + g), __ldg(a.p + g - (q == 0 ? 1 : q == 1 ? L.sy : L.sz))), out.x);
+      hist[g] = out.y;
+      (q == 0 ? a.us : q == 1 ? a.vs : a.ws)[g] = out.x;
+    }
+    __syncwarp();
+    const unsigned short rest = T.list[wy == 0 ? 0 : wy - 1][32 + lane];
+    __syncwarp();
+    if (n > 32) T.list[wy - 1][lane] = rest;
+    n = max(n - 32, 0);
+    __syncwarp();
   }
 }
 
@@ -600,13 +808,6 @@ __device__ __forceinline__ void predict_fx_body(const PredictArgs& a, unsigned c
   FxTail& T = *reinterpret_cast<FxTail*>(reinterpret_cast<unsigned char*>(&S) + sizeof(FxPredSmem));
   const int tid = threadIdx.x + TX * threadIdx.y;
   const int g0 = (k0 - 1) / GRP, ng = (k1 - 2) / GRP - g0 + 1;
-  if (a.pmax && (int)threadIdx.y < 3 * ng) {  // a warp per group and field
-    const int f = threadIdx.y % 3, gi = threadIdx.y / 3, lane = threadIdx.x;
-    const int k = GRP * (g0 + gi) + lane;
-    const unsigned m = lane < GRP + 2 && k <= a.L.nz + 1 ? __ldg(a.pmax + f * (a.L.nz + 2) + k) : 0u;
-    const unsigned r = __reduce_max_sync(0xffffffffu, m);
-    if (lane == 0) T.e[gi][f] = (int)(r >> 20);
-  }
   unsigned phase = 0;  // tile loader: bit s is the parity of slot s's next phase
   bool ok = true;      // false once a wait gave up (recorded in a.err); every issued plane
                        // is still waited for (bounded), so none is in flight at exit
@@ -620,13 +821,23 @@ __device__ __forceinline__ void predict_fx_body(const PredictArgs& a, unsigned c
   __syncthreads();
   for (int gi = 0; gi < ng; ++gi) {
     const int ks = max(k0, GRP * (g0 + gi) + 1), ke = min(k1, GRP * (g0 + gi + 1) + 1);
-    FxPlane P;
-    bool bad = !a.pmax;  // coefficients outside the fixed-point range: FP64 stencils everywhere
+    FxPlane P{};
+    bool bad = !a.fixed;  // coefficients outside the fixed-point range: FP64 stencils everywhere
+    if (a.fixed) {
+      unsigned top[3];
+      tile_exponents(a, T, 1 + TX * bx, 1 + TY * by, g0 + gi, top);
+      int em = kFxLo;
 #pragma unroll
-    for (int f = 0; f < 3; ++f) {
-      P.e[f] = T.e[gi][f];
-      bad = bad || P.e[f] > kFxHi;
-      P.e[f] = max(P.e[f], kFxLo);
+      for (int f = 0; f < 3; ++f) {
+        P.e[f] = (int)(top[f] >> 20);
+        P.least[f] = top[f] ? kQuietOwn : 0u;
+        P.least_product[f] = top[f] ? kQuietProduct : 0u;
+        bad = bad || P.e[f] > kFxHi || (P.e[f] < kFxLo && top[f] != 0u);
+        em = max(em, P.e[f]);
+      }
+#pragma unroll
+      for (int f = 0; f < 3; ++f)
+        if (top[f] == 0u) P.e[f] = em;
     }
     if (bad) predict_body<SCHEME, FIRST, DPF, 0>(a, reinterpret_cast<PredSmem&>(S), bx, by, ks, ke);
     else predict_fx_planes<SCHEME, FIRST, DPF, ISO, TMA>(a, S, T, raw, P, bx, by, ks, ke, phase, ok, mu, mv, mw);
@@ -671,77 +882,6 @@ __global__ void __launch_bounds__(TX*(TY + 1)) predict_tma_kernel(PredictArgs a,
                                                  blockIdx.y, k0, k1, &mu, &mv, &mw);
 }
 
-// Whether the stencils of an output read slot (i, j, k) of field f.  The other
-// slots (most edges of the box; the extra slot of a wall axis) hold whatever
-// the caller's arrays hold there, and must not set a block exponent.  With a
-// the field's own axis and b another one: its ghosts along b are read beside
-// the field's own faces [lo, n], the low ones also beside every face in
-// [1, n + 1] when b's lowest face has an output.
-__device__ __forceinline__ bool slot_read(const PredictArgs& a, int f, int i, int j, int k) {
-  const int pos[3] = {i, j, k}, n[3] = {a.L.nx, a.L.ny, a.L.nz}, lo[3] = {a.ulo, a.vlo, a.wlo};
-  const int p = f == 0 ? i : f == 1 ? j : k, np = f == 0 ? n[0] : f == 1 ? n[1] : n[2];
-  const int lp = f == 0 ? lo[0] : f == 1 ? lo[1] : lo[2];
-  int ghosts = 0, first = lp - 1, last = np + 1;
-#pragma unroll
-  for (int b = 0; b < 3; ++b) {
-    if (b == f) continue;
-    const bool low = pos[b] == 0, high = pos[b] > n[b];
-    ghosts += low || high;
-    if (high || (low && lo[b] > 1)) {
-      first = lp;
-      last = np;
-    } else if (low) {
-      first = 1;
-    }
-  }
-  return ghosts < 2 && p >= first && p <= last;
-}
-
-// Largest magnitude (high word) of the slots of each z plane of u, v, w that
-// are read: CTA (plane, field), a warp per row, four rows at once: with one
-// row's loads in flight the predictor stage takes 831 us at 256^3 and 134 at
-// 128^3, so 774 and 124.
-constexpr int kMaxThreads = 512;
-__device__ __forceinline__ void plane_max_body(const PredictArgs& a, int k, int f) {
-  const Layout& L = a.L;
-  if (!a.pmax) return;
-  const double* p = (f == 0 ? a.u : f == 1 ? a.v : a.w) + L.at(0, 0, k);
-  const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
-  unsigned m = 0;
-  constexpr int NW = kMaxThreads / 32, RJ = 4;  // RJ rows of a warp at once keep its loads in flight
-  const int nx2 = L.nx + 2, ny2 = L.ny + 2;
-  for (int j = warp; j < ny2; j += RJ * NW) {
-    const double* row = p + L.sy * (long long)j;
-#pragma unroll 2
-    for (int i = lane; i < nx2; i += 32) {
-      unsigned h[RJ];
-#pragma unroll
-      for (int q = 0; q < RJ; ++q)
-        h[q] = j + q * NW < ny2 && slot_read(a, f, i, j + q * NW, k)
-                   ? (unsigned)__double2hiint(__ldg(row + L.sy * (q * NW) + i)) & 0x7fffffffu
-                   : 0u;
-#pragma unroll
-      for (int q = 0; q < RJ; ++q) m = max(m, h[q]);
-    }
-  }
-  m = __reduce_max_sync(0xffffffffu, m);
-  __shared__ unsigned w[kMaxThreads / 32];
-  if (lane == 0) w[warp] = m;
-  __syncthreads();
-  if (warp == 0) {
-    m = __reduce_max_sync(0xffffffffu, lane < kMaxThreads / 32 ? w[lane] : 0u);
-    if (lane == 0) a.pmax[f * (L.nz + 2) + k] = m;
-  }
-}
-__global__ void __launch_bounds__(kMaxThreads) plane_max_kernel(PredictArgs a, int p0) {
-  plane_max_body(a, p0 + blockIdx.x, blockIdx.y);
-}
-__global__ void __launch_bounds__(kMaxThreads) plane_max_batch_kernel(const PredictArgs* __restrict__ tab,
-                                                                      const BatchItem* __restrict__ items) {
-  const BatchItem w = items[blockIdx.x];
-  plane_max_body(tab[w.sub], w.bx, blockIdx.y);
-}
-
 // Batched: persistent CTAs walk the work items (subdomain, tile) of a batch.
 template <int SCHEME, bool FIRST, bool DPF, bool ISO>
 __global__ void __launch_bounds__(TX*(TY + 1), 3) predict_batch_kernel(const PredictArgs* __restrict__ tab,
@@ -768,7 +908,7 @@ static bool tma_serves(const PredTma* t, const PredictArgs& a) {
   return t && t->ready && a.u == t->pu && a.v == t->pv && a.w == t->pw;
 }
 
-void set_predict_fixed(PredictArgs& a, int scheme, unsigned* pmax) {
+void set_predict_fixed(PredictArgs& a, int scheme) {
   const double c[3] = {a.cx, a.cy, a.cz};
   const double v[3] = {scheme == 2 ? a.ca : a.kx, scheme == 2 ? a.cb : a.ky, scheme == 2 ? a.cc : a.kz};
   auto scale = [](const double (&x)[3], long long (&q)[3], int& k, int below) {  // largest in [2^-below-1, 2^-below)
@@ -782,16 +922,16 @@ void set_predict_fixed(PredictArgs& a, int scheme, unsigned* pmax) {
     return std::abs(k) <= 200;
   };
   const bool okc = scale(c, a.q60, a.kq, 0), okv = scale(v, a.v60, a.kv, 1);
-  a.pmax = okc && okv ? pmax : nullptr;
+  a.fixed = okc && okv;
   a.iso = c[0] == c[1] && c[0] == c[2] && v[0] == v[1] && v[0] == v[2];
 }
 
 // Planes per CTA: a chunk's cost is its planes plus about two (its first
-// planes and the products of its first face), and two CTAs share an SM, so
+// planes and the products of its first face), and three CTAs share an SM, so
 // the depth with the fewest waves x (depth + 2) is taken, of those that
 // divide a group.  At 256^3 that is 16 (4096 CTAs), at 64^3 4 (256 CTAs), at
 // 32^3 1 (128 CTAs).  With 16 planes a CTA at every size the 64^3 predictor
-// took 0.180 ms (now 0.035), the 32^3 one 0.165 (0.017).
+// took 0.180 ms (now 0.034), the 32^3 one 0.165 (0.017).
 int predict_chunk(const std::vector<std::pair<long long, int>>& boxes) {
   int dev = 0, nsm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -820,14 +960,8 @@ static cudaError_t launch_smem(K kern, dim3 grid, size_t sm, cudaStream_t st, co
   return cudaGetLastError();
 }
 
-// The largest magnitudes of the planes [p0, p1) that the launch reads, then the predictor.
 template <int SCHEME, bool FIRST, bool DPF>
-static cudaError_t launch_grid(const PredictArgs& b, dim3 grid, int p0, int p1, cudaStream_t st, const PredTma* tma) {
-  if (b.pmax) {
-    plane_max_kernel<<<dim3(p1 - p0, 3), kMaxThreads, 0, st>>>(b, p0);
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
+static cudaError_t launch_grid(const PredictArgs& b, dim3 grid, cudaStream_t st, const PredTma* tma) {
   if (tma_serves(tma, b)) {
     const size_t sm = kFxSmem + sizeof(FxRaw) + 128;
     if (b.iso) return launch_smem(predict_tma_kernel<SCHEME, FIRST, DPF, true>, grid, sm, st, b, tma->u, tma->v, tma->w);
@@ -847,7 +981,7 @@ static cudaError_t launch_t(const PredictArgs& a, cudaStream_t st, const PredTma
   const dim3 t = tile_grid(a.L, a.L.nz, 1);
   b.kc = predict_chunk({{(long long)t.x * t.y, a.L.nz}});
   b.koff = b.kend = 0;
-  return launch_grid<SCHEME, FIRST, DPF>(b, tile_grid(a.L, a.L.nz, b.kc), 0, a.L.nz + 2, st, tma);
+  return launch_grid<SCHEME, FIRST, DPF>(b, tile_grid(a.L, a.L.nz, b.kc), st, tma);
 }
 
 // Convection (mode 1) or diffusion (mode 2) alone, in FP64.
@@ -871,12 +1005,12 @@ static cudaError_t launch_planes_t(PredictArgs b, cudaStream_t st, int p0, int p
   b.kc = kc;
   b.koff = p0 - 1;
   b.kend = p1;
-  return launch_grid<SCHEME, FIRST, DPF>(b, tile_grid(b.L, p1 - p0, kc), p0 - 1, p1 + 1, st, tma);
+  return launch_grid<SCHEME, FIRST, DPF>(b, tile_grid(b.L, p1 - p0, kc), st, tma);
 }
 
 cudaError_t launch_predict_planes(PredictArgs a, int scheme, bool first, bool dpf, int p0, int p1, int kc,
                                   cudaStream_t st, const PredTma* tma) {
-  if (p0 < 1 || p1 > a.L.nz + 1 || p0 > p1 || kc < 1 || kc > GRP * (NWIN - 1)) return cudaErrorInvalidValue;
+  if (p0 < 1 || p1 > a.L.nz + 1 || p0 > p1 || kc < 1 || kc > 2 * GRP) return cudaErrorInvalidValue;
   if (p0 == p1) return cudaSuccess;
 #define NS_PRED_PCASE(S, F, D) \
   if (scheme == S && first == F && dpf == D) return launch_planes_t<S, F, D>(a, st, p0, p1, kc, tma);
@@ -952,13 +1086,8 @@ static cudaError_t launch_bt(const PredictArgs* tab, const BatchItem* items, int
   return cudaGetLastError();
 }
 
-cudaError_t launch_predict_batch(const PredictArgs* tab, const BatchItem* items, int n_items, const BatchItem* planes,
-                                 int n_planes, bool iso, int scheme, bool first, bool dpf, int grid, cudaStream_t st) {
-  if (n_planes > 0) {
-    plane_max_batch_kernel<<<dim3(n_planes, 3), kMaxThreads, 0, st>>>(tab, planes);
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
+cudaError_t launch_predict_batch(const PredictArgs* tab, const BatchItem* items, int n_items, bool iso, int scheme,
+                                 bool first, bool dpf, int grid, cudaStream_t st) {
 #define NS_PRED_CASE(S, F, D)                                                         \
   if (scheme == S && first == F && dpf == D)                                          \
     return iso ? launch_bt<S, F, D, true>(tab, items, n_items, grid, st)              \

@@ -58,7 +58,6 @@ struct ns_handle {
   ns::FaceSet faces[4]{};
   bool face_set_nonzero[4] = {false, false, false, false};
   unsigned long long* diag_bits = nullptr;
-  unsigned* pmax = nullptr;  // largest magnitudes of u, v, w per z plane (predictor)
   int* dev_err = nullptr;  // set on the device when a bounded wait of the predictor's tile loader gave up
   ns::PredTma tma{};        // tile-loader maps of u, v, w (tma.ready = 0: the predictor loads tiles itself)
   // state
