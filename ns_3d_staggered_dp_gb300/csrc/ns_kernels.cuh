@@ -62,6 +62,7 @@ struct PredictArgs {
   long long q60[3], v60[3];
   int kq, kv;
   int iso;  // 1: the three axes have the same coefficients
+  int far;  // 1: they differ by more than a factor of 4
 };
 // Tile-loader maps (TMA) of three fields of one layout for the session
 // predictor (ns_predict.cu): 3D tensors (px, ny+2, nz+2) of doubles, boxes of

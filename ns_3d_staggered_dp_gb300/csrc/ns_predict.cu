@@ -619,9 +619,12 @@ __device__ __forceinline__ void predict_fx_planes(const PredictArgs& a, FxPredSm
   // 2^60 more.  The terms of C along the axes differ by the advecting field, so fields of about the
   // same magnitude are summed as integers (at the largest one's unit); otherwise every term is
   // brought back by itself, so that a small term keeps its digits where the large one vanishes
-  // (a shear layer u(y): du/dx = 0).
+  // (a shear layer u(y): du/dx = 0).  Likewise where the axes' coefficients differ by more than 4
+  // (far): summed as integers, the term along an axis 16 times coarser is off by 1e-15 of itself, 1000
+  // times coarser by 5e-11.
   const int em = max(P.e[0], max(P.e[1], P.e[2]));
-  const bool apart = em - min(P.e[0], min(P.e[1], P.e[2])) > 1;
+  const bool far = !ISO && a.far;
+  const bool apart = far || em - min(P.e[0], min(P.e[1], P.e[2])) > 1;
   FxW qw[3], vw[3];
   if (ISO) {
     vw[0] = fxw62(a.v60[0]);
@@ -647,6 +650,12 @@ __device__ __forceinline__ void predict_fx_planes(const PredictArgs& a, FxPredSm
     return fx_to_int(fx_mul(dx, qw[0]) + fx_mul(dy, qw[1]) + fx_mul(dz, qw[2]), e + em + kP + a.kq);
   };
   auto visc = [&](long long uc, long long we, long long sn, long long bt, int e) -> double {
+    if (far) {  // the coarse axis' coefficient would have few digits beside the fine one's
+      const int k = e - 1022 - kFxB;
+      double t = fmul(c, fx_to_int(we - 2 * uc, k), SCHEME == 2 ? a.ca : a.kx);
+      t = fma(fx_to_int(sn - 2 * uc, k), SCHEME == 2 ? a.cb : a.ky, t);
+      return fma(fx_to_int(bt - 2 * uc, k), SCHEME == 2 ? a.cc : a.kz, t);
+    }
     long long s;
     if (ISO) s = fx_mul62((we + sn + bt - 6 * uc + 1) >> 1, vw[0]);
     else s = fx_mul(we - 2 * uc, vw[0]) + fx_mul(sn - 2 * uc, vw[1]) + fx_mul(bt - 2 * uc, vw[2]);
@@ -923,6 +932,11 @@ void set_predict_fixed(PredictArgs& a, int scheme) {
   };
   const bool okc = scale(c, a.q60, a.kq, 0), okv = scale(v, a.v60, a.kv, 1);
   a.fixed = okc && okv;
+  auto spread = [](const double (&x)[3]) {
+    const double lo = std::min(std::fabs(x[0]), std::min(std::fabs(x[1]), std::fabs(x[2])));
+    return 4.0 * lo < std::max(std::fabs(x[0]), std::max(std::fabs(x[1]), std::fabs(x[2])));
+  };
+  a.far = spread(c) || spread(v);
   a.iso = c[0] == c[1] && c[0] == c[2] && v[0] == v[1] && v[0] == v[2];
 }
 
