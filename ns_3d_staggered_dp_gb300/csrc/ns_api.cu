@@ -242,7 +242,7 @@ void dense_pair(int n, int pb, std::vector<double>& F, std::vector<double>& G) {
 double axis_eig(int n, int pb, int m, double h) {
   const double pi = 3.1415926535897932;
   double s;
-  if (pb == 1) s = std::sin(pi * m / n);
+  if (pb == 1) s = std::sin(pi * std::min(m, n - m) / n);  // sin(pi m / n) of m next to n has few digits
   else if (pb == 2) s = std::sin((m + 1) * pi / 2 / n);
   else if (pb == 3) s = std::sin(m * pi / 2 / n);
   else s = std::sin((m + 1) * pi / 2 / (n + 1));
