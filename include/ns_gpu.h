@@ -398,8 +398,10 @@ int ns_batch_autotune(ns_batch* b, int reps);
 /* Device time of every stage kernel of one regular step (mean over reps
  * launches, on a copy of the state), in the stage order interp, predict,
  * vel_bc x/y/z, x forward, y forward, z solve, y inverse, x inverse,
- * pr_bc x/y/z, correct, hist: ms_per_stage[16] (the last two unused).  With
- * AB2-CN the vel_bc x/y/z entries are the x, y, z ADI sweeps. */
+ * pr_bc x/y/z, correct, hist: ms_per_stage[16] (the last two unused).  The
+ * pressure fill is one launch: its time is the pr_bc x entry, pr_bc y and z
+ * are 0.  The velocity fill likewise (vel_bc x); with AB2-CN the vel_bc x/y/z
+ * entries are the x, y, z ADI sweeps. */
 int ns_batch_profile(ns_batch* b, int reps, double* ms_per_stage);
 int ns_batch_get_config(const ns_batch* b, ns_batch_config* out);
 

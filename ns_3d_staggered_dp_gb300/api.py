@@ -501,7 +501,8 @@ class Batch:
               "x_inv", "pr_bc_x", "pr_bc_y", "pr_bc_z", "correct")
 
     def profile(self, reps=3):
-        """{stage: ms} of one regular step's stage kernels (ns_batch_profile)."""
+        """{stage: ms} of one regular step's stage kernels (ns_batch_profile).  A fill's three passes
+        are one launch: vel_bc_x (but with AB2-CN, whose sweeps take these entries) and pr_bc_x."""
         out = np.zeros(16)
         self._check(self.lib.ns_batch_profile(self.h, int(reps), _ptr(out)))
         return dict(zip(self.STAGES, out[:len(self.STAGES)]))

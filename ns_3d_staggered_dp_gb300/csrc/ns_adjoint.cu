@@ -462,7 +462,7 @@ int adj_backward_step(ns_handle* h, AdjState* A, double* const fwd[3], bool firs
   d.one = 1.0; d.mzero = -0.0; d.rhs = nullptr;
   ADJ_CUDA(h, launch_fft_poisson(h->plan, d, h->spec, h->dp, h->L, h->stream, api_marker(h)));
   ADJ_CUDA(h, launch_pr_bc(h->L, h->dp, h->faces[0], c.pbc, h->dx, h->dy, h->dz, h->stream));
-  api_mark(h, "adj_pr_bc", 3);
+  api_mark(h, "adj_pr_bc", 1);
   CorrectArgs ca{};
   ca.L = h->L;
   ca.us = A->lam[0]; ca.vs = A->lam[1]; ca.ws = A->lam[2]; ca.dp = h->dp;
