@@ -438,226 +438,32 @@ cudaError_t launch_adi_batch(int axis, const BatchAdiArgs* tab, const BatchItem*
 // Chunked sweeps
 // ---------------------------------------------------------------------------
 // With a small viscous number every factor of the LU is small (nu dt / 2 h^2 =
-// 0.002: 0.002), so a row hears nothing, to the last bit, of rows `halo` (6 to
-// 16) away.  A thread solves CH unknowns of a line from CH + 2 halo right-hand
-// sides held in registers: one read and one write of the fields, no
-// intermediate in memory, and CH-fold parallelism along the line.  The
-// right-hand sides come scaled by the pivots (ChunkSys), one FMA each way.
-// These kernels take the lines that do not fit a CTA (launch_adi_chunks).
-// Rows q of [T0, T1) take their factors from the tables, the others the converged ones.
-template <int R, int W, int T0, int T1>
-__device__ __forceinline__ void chunk_rows(double (&r)[R], const ChunkSys& S, int e0) {
-  const double* l = S.l + kAdiExt + e0;
-  const double* dm = S.dm + kAdiExt + e0;
-  const double* cu = S.cu + kAdiExt + e0;
-  const double nl = -S.lc, nc = -S.cc;
-#pragma unroll
-  for (int q = 1; q < R; ++q) r[q] = fma(q >= T0 && q < T1 ? -__ldg(l + q) : nl, r[q - 1], r[q]);
-  if (R - 1 >= T0 && R - 1 < T1) r[R - 1] *= __ldg(dm + R - 1);
-#pragma unroll
-  for (int q = R - 2; q >= W; --q)
-    r[q] = q >= T0 && q < T1 ? fma(-__ldg(cu + q), r[q + 1], r[q] * __ldg(dm + q)) : fma(nc, r[q + 1], r[q]);
-}
-// The factors differ from the converged ones on a few rows at a line's first
-// end and on its last row (and where a periodic line goes on with row 0).
-template <int CH, int W>
-__device__ __forceinline__ void chunk_solve(double (&r)[CH + 2 * W], const ChunkSys& S, int e0) {
-  constexpr int R = CH + 2 * W, LOW = 2 * W + 2, HIGH = W + CH - 2;
-  if (e0 >= S.c0 && e0 + R <= S.c1) chunk_rows<R, W, 0, 0>(r, S, e0);
-  else if (e0 + LOW >= S.c0 && e0 + R <= S.c1) chunk_rows<R, W, 0, LOW>(r, S, e0);
-  else if (e0 >= S.c0 && e0 + HIGH <= S.c1) chunk_rows<R, W, HIGH, R>(r, S, e0);
-  else chunk_rows<R, W, 0, R>(r, S, e0);
-}
-// First unknown that chunk c works out: the last chunk ends at the line's end
-// (and writes only the unknowns past the chunk before it).
-template <int CH>
-__device__ __forceinline__ int chunk_first(const ChunkSys& S, int s) { return min(s, max(S.m - CH, 0)); }
-// Unknown index e continued past an end: where its right-hand side is (within
-// [0, m)), or -1 past an end that does not wrap.
-__device__ __forceinline__ int chunk_row(const ChunkSys& S, int e) {
-  if (e < 0 ? !S.wrap_lo : e >= S.m && !S.wrap_hi) return -1;
-  while (e < 0) e += S.m;
-  while (e >= S.m) e -= S.m;
-  return e;
-}
-
-// y and z sweeps: a thread per (field, chunk, line), lanes over x.
-template <int AXIS, int CH, int W>
-__global__ void __launch_bounds__(128, CH + 2 * W <= 50 ? 4 : 3) adi_chunk_kernel(const __grid_constant__ AdiArgs a) {
-  constexpr int R = CH + 2 * W;
-  const Layout& L = a.L;
-  const int fld = blockIdx.z, s = blockIdx.y * CH;
-  const ChunkSys& S = a.ch[fld];
-  if (s >= S.m) return;
-  const int n1 = L.nx + 2;
-  const int zlo = (AXIS == 1 && a.z1 > 0) ? a.z0 : 0;
-  const int n2 = AXIS == 2 ? L.ny + 2 : ((AXIS == 1 && a.z1 > 0) ? a.z1 - a.z0 : L.nz + 2);
-  const int tl = blockIdx.x * 128 + threadIdx.x;
-  if (tl >= n1 * n2) return;
-  long long base, st;
-  line_of<AXIS>(L, tl % n1, zlo + tl / n1, base, st);
-  const double* __restrict__ src = a.src[fld] + base;
-  double* __restrict__ dst = a.dst[fld] + base;
-  const double* sl = src + S.lo * st;
-  const bool walls = !S.periodic;
-  const int f = chunk_first<CH>(S, s), e0 = f - W, skip = s - f;
-  double r[R];
-  int er = chunk_row(S, e0 < 0 && !S.wrap_lo ? 0 : e0);
-#pragma unroll
-  for (int q = 0; q < R; ++q) {
-    const int e = e0 + q;
-    const bool in = (e >= 0 || S.wrap_lo) && (e < S.m || S.wrap_hi);
-    r[q] = in ? sl[er * st] : 0.0;
-    if (in) er = er + 1 == S.m ? 0 : er + 1;
-  }
-  if (walls && (f == 0 || f + CH + W >= S.m)) {  // the BC rows take the sweep's face values
-    const int pl = tl + zlo * n1;                // index in the full face plane
-    const double lo = a.face_lo[fld] ? a.face_scale * __ldg(a.face_lo[fld] + pl) : 0.0;
-    const double hi = a.face_hi[fld] ? a.face_scale * __ldg(a.face_hi[fld] + pl) : 0.0;
-#pragma unroll
-    for (int q = 0; q < R; ++q) {
-      if (e0 + q == 0) r[q] = lo;
-      if (e0 + q == S.m - 1) r[q] = hi;
-    }
-  }
-  chunk_solve<CH, W>(r, S, e0);
-  double* xl = dst + S.lo * st;
-  const int n = S.m - s;  // unknowns from this chunk's first on
-#pragma unroll
-  for (int q = 0; q < CH; ++q)
-    if (q >= skip && f + q < S.m) xl[(f + q) * st] = r[W + q];
-  const int nax = axis_n(L, AXIS);
-  if (walls) {  // the carried slots
-    if (s == 0)
-      for (int i = 0; i < S.lo; ++i) dst[i * st] = src[i * st];
-    if (n <= CH)
-      for (int i = S.lo + S.m; i <= nax + 1; ++i) dst[i * st] = src[i * st];
-  } else {
-    if (s == 0) dst[(nax + 1) * st] = xl[0];  // slot n+1 <- slot 1
-    if (n <= CH) dst[0] = xl[(S.m - 1) * st];  // slot 0 <- slot n (written above; a register picked by n
-  }                                            // would put the array on the stack)
-}
-
-// x sweep: a warp takes one chunk of 32 consecutive lines; its rows pass
-// through shared memory (stride 33), so that every global access is a row
-// segment.
-template <int CH, int W>
-__global__ void __launch_bounds__(32 * XW, CH + 2 * W <= 50 ? 4 : 3) adi_chunk_x_kernel(const __grid_constant__ AdiArgs a) {
-  constexpr int R = CH + 2 * W;
-  extern __shared__ double sh_x[];
-  const Layout& L = a.L;
-  const int fld = blockIdx.z, s = blockIdx.y * CH;
-  const ChunkSys& S = a.ch[fld];
-  if (s >= S.m) return;
-  const int n1 = L.ny + 2;
-  const int nlines = n1 * (a.z1 > 0 ? a.z1 - a.z0 : L.nz + 2);
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int t0 = (blockIdx.x * XW + warp) * 32;
-  if (t0 >= nlines) return;
-  const int nl = min(32, nlines - t0);
-  const int t = t0 + min(lane, nl - 1);  // lanes past the end repeat the last line (never stored)
-  const int j = t % n1, k = a.z0 + t / n1;
-  const int my_off = (int)L.at(S.lo, j, k);  // unknown 0 of this lane's line
-  double* sb = sh_x + warp * (R * XS);
-  const double* __restrict__ src = a.src[fld];
-  double* __restrict__ dst = a.dst[fld];
-  const bool walls = !S.periodic;
-  const int f = chunk_first<CH>(S, s), e0 = f - W, skip = s - f;
-  int er[(R + 31) / 32];
-#pragma unroll
-  for (int p = 0; p < (R + 31) / 32; ++p) er[p] = chunk_row(S, e0 + lane + 32 * p);
-#pragma unroll 4
-  for (int l = 0; l < 32; ++l) {
-    const int off = __shfl_sync(0xffffffffu, my_off, l);
-#pragma unroll
-    for (int p = 0; p < (R + 31) / 32; ++p) {
-      const int q = lane + 32 * p;
-      if (q < R) {
-        if (er[p] >= 0) cp_async8(&sb[q * XS + l], src + off + er[p]);
-        else sb[q * XS + l] = 0.0;
-      }
-    }
-  }
-  cp_async_commit();
-  cp_async_wait<0>();
-  __syncwarp();
-  double r[R];
-#pragma unroll
-  for (int q = 0; q < R; ++q) r[q] = sb[q * XS + lane];
-  if (walls && (f == 0 || f + CH + W >= S.m)) {  // the BC rows take the sweep's face values
-    const int pl = j + n1 * k;
-    const double lo = a.face_lo[fld] ? a.face_scale * __ldg(a.face_lo[fld] + pl) : 0.0;
-    const double hi = a.face_hi[fld] ? a.face_scale * __ldg(a.face_hi[fld] + pl) : 0.0;
-#pragma unroll
-    for (int q = 0; q < R; ++q) {
-      if (e0 + q == 0) r[q] = lo;
-      if (e0 + q == S.m - 1) r[q] = hi;
-    }
-  }
-  chunk_solve<CH, W>(r, S, e0);
-#pragma unroll
-  for (int q = W; q < W + CH; ++q) sb[q * XS + lane] = r[q];
-  __syncwarp();
-  const int n = S.m - s, nc = min(n, CH);
-#pragma unroll 4
-  for (int l = 0; l < 32; ++l) {
-    const int off = __shfl_sync(0xffffffffu, my_off, l);
-    if (l < nl)
-      for (int q = lane; q < nc; q += 32) dst[off + s + q] = sb[(W + skip + q) * XS + l];
-  }
-  if (lane < nl) {
-    const double* xs = src + L.at(0, j, k);
-    double* xd = dst + L.at(0, j, k);
-    if (walls) {  // the carried slots
-      if (s == 0)
-        for (int i = 0; i < S.lo; ++i) xd[i] = xs[i];
-      if (n <= CH)
-        for (int i = S.lo + S.m; i <= L.nx + 1; ++i) xd[i] = xs[i];
-    } else {
-      if (s == 0) xd[L.nx + 1] = sb[W * XS + lane];             // slot n+1 <- slot 1
-      if (n <= CH) xd[0] = sb[(W + skip + n - 1) * XS + lane];  // slot 0 <- slot n
-    }
-  }
-}
-
-template <int CH, int W>
-cudaError_t launch_adi_chunk(int axis, const AdiArgs& a, cudaStream_t st) {
-  const int n1 = axis == 0 ? a.L.ny + 2 : a.L.nx + 2;
-  const int n2 = axis == 2 ? a.L.ny + 2 : (a.z1 > 0 ? a.z1 - a.z0 : a.L.nz + 2);
-  if (n2 <= 0) return cudaSuccess;
-  const int m = std::max(a.ch[0].m, std::max(a.ch[1].m, a.ch[2].m));
-  const dim3 grid((unsigned)((n1 * n2 + 127) / 128), (unsigned)((m + CH - 1) / CH), 3);
-  if (axis == 0) {
-    const size_t sm = (size_t)XW * (CH + 2 * W) * XS * sizeof(double);
-    cudaError_t e = cudaFuncSetAttribute(adi_chunk_x_kernel<CH, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    adi_chunk_x_kernel<CH, W><<<grid, 32 * XW, sm, st>>>(a);
-  } else if (axis == 1) {
-    adi_chunk_kernel<1, CH, W><<<grid, 128, 0, st>>>(a);
-  } else {
-    adi_chunk_kernel<2, CH, W><<<grid, 128, 0, st>>>(a);
-  }
-  return cudaGetLastError();
-}
-
-// ---------------------------------------------------------------------------
-// Chunked sweeps, whole lines in a CTA
-// ---------------------------------------------------------------------------
-// The same with a line's chunks in one CTA (32 lines, a thread CH unknowns of
-// one): what enters a chunk is worked out by its neighbour from its W
-// outermost unknowns and handed over through shared memory, so every
-// right-hand side is read once and takes part in 2 (CH + W) / CH FMAs: 2.5 at
-// CH 32, W 8, against 2.75 and a second read of the halos.  Bound by the FP64
-// unit, 75 to 80% busy.  Sweeps x, y, z in us (chunks with halos; whole lines
-// with one thread each): 256^3 278, 266, 267 (371, 317, 290; 512, 385, 369),
-// 128^3 52, 46, 49 (65, 58, 58), with walls 70, 61, 62 (82, 73, 73), 32^3 12,
-// 8, 8 (10, 11, 10).  The same in 58-bit integers with the exponent of the
-// line takes 319, 296, 292 at 256^3: the chain of a product waits longer there
-// than for an FMA.  The batch keeps the whole-line kernels: 185, 108, 107 us
-// for 64 blocks of 16 to 64 cells, in chunks of 18 172, 176, 155.
+// 0.002: 0.002), so what rows W = 8 to 16 away weigh in a row is below 2^-57.
+// A line's chunks of CH unknowns are solved in one CTA (32 lines, a thread a
+// chunk) in registers: what enters a chunk is worked out by its neighbour from
+// its W outermost unknowns and handed over through shared memory.  One read
+// and one write of the fields, no intermediate in memory, CH-fold parallelism
+// along the line, and a right-hand side takes part in 2 (CH + W) / CH FMAs:
+// they come scaled by the pivots (ChunkSys), one FMA each way.
+//
+// 2^-57 of a value W + 1 rows away is not always rounding: where the W rows
+// between are far below that value, it is what enters.  So a chunk compares
+// what it handed on with what it then ends on itself, and where they differ by
+// more than roundings (off) the neighbour adds the difference's part
+// (chunk_fwd_add, chunk_bwd_add): what is still left out lies below 2^-114.
+//
+// Bound by the FP64 unit, 75 to 80% busy.  Sweeps x, y, z in us (one thread a
+// line): 256^3 274, 259, 262 (512, 385, 369), 128^3 53, 46, 47, with walls 63,
+// 55, 55, 32^3 13, 8, 10; the comparison costs nothing (without it 279, 265,
+// 266 at 256^3).
+// The same in 58-bit integers with the exponent of the line takes 319, 296,
+// 292 at 256^3: the chain of a product waits longer there than for an FMA.
+// The batch keeps the whole-line kernels: 185, 108, 107 us for 64 blocks of 16
+// to 64 cells, in chunks of 18 172, 176, 155.
 // Chunks of a line in one CTA, at most: 10 of 26 unknowns (258: a wall line of
-// 256 cells), else 8.
-constexpr int line_chunks_max(int ch) { return ch == 26 ? 10 : 8; }
+// 256 cells), 8 of 16, and 8 of 32 at three CTAs an SM or 17 (a wall line of
+// 512 cells) at one.
+constexpr int line_chunks_max(int ch) { return ch == 26 ? 10 : (ch == 16 ? 8 : 17); }
 // Rows of a line's first end that may differ from the converged ones.
 __host__ __device__ constexpr int line_low(int W) { return W + 2; }
 // The system has its special rows where the kernels look for them: a few at
@@ -696,18 +502,53 @@ __device__ __forceinline__ double chunk_bwd(double (&r)[CH], const ChunkSys& S, 
   return x;
 }
 
+// Two roundings of one number differ by a few units, no more.
+__device__ __forceinline__ bool off(double a, double b) {
+  return (unsigned long long)(__double_as_longlong(a) - __double_as_longlong(b) + 4) > 8;
+}
+// The rare part, on a copy of the chunk in local memory (unrolled over the registers it made the kernels
+// too long for the instruction cache: the 128^3 box's step 10% slower, with no chunk taking it).
+// Forward: y that enters is d more than was taken; returns what the chunk then hands on backward.
+// low: rows before it are of the tables; ql: the line's last row, with its own factor.
+__device__ __noinline__ double chunk_fwd_add(double* r, const ChunkSys& S, int e0, int ch, int w, int low, int ql,
+                                             double d) {
+  const double* l = S.l + kAdiExt + e0;
+  const double* dm = S.dm + kAdiExt + e0;
+  const double* cu = S.cu + kAdiExt + e0;
+#pragma unroll 1
+  for (int q = 0; q < ch && q <= ql; ++q) {
+    d *= q == ql && q >= low ? -l[q] * dm[q] : -l[q];
+    r[q] += d;
+  }
+  double x = 0.0;
+#pragma unroll 1
+  for (int q = w - 1; q >= 0; --q) x = fma(-cu[q], x, q < low ? r[q] * dm[q] : r[q]);
+  return x;
+}
+__device__ __noinline__ void chunk_bwd_add(double* r, const ChunkSys& S, int e0, int ch, double d) {
+  const double* cu = S.cu + kAdiExt + e0;
+#pragma unroll 1
+  for (int q = ch - 1; q >= 0; --q) {
+    d *= -cu[q];
+    r[q] += d;
+  }
+}
+
 // r: the right-hand sides of chunk s of T (zero past the line's end), replaced by the solution.
 // sh: 16 bytes a thread.
 template <int CH, int W>
 __device__ __forceinline__ void chunk_line_solve(double (&r)[CH], const ChunkSys& S, int s, int T, int l, double* sh) {
   constexpr int LOW = line_low(W) < CH ? line_low(W) : CH;
-  double* ys = sh;
-  double* xs = sh + 32 * T;
+  double* ys = sh + l;
+  double* xs = sh + 32 * T + l;
   const int e0 = s * CH, ql = S.m - 1 - e0;
   const bool low = s == 0 && S.c0 > 0, end = e0 + CH > S.c1;
-  ys[32 * s + l] = chunk_fwd<CH, CH - W, CH, CH - W < LOW ? LOW : 0, false, false>(r, S, e0, 0, 0.0);
+  const int before = s > 0 ? s - 1 : (S.wrap_lo ? T - 1 : -1), after = s + 1 < T ? s + 1 : (S.wrap_hi ? 0 : -1);
+  const bool feeds_up = s + 1 < T || S.wrap_lo, feeds_down = s > 0 || S.wrap_hi;  // a chunk takes its y, its x
+  const double y = chunk_fwd<CH, CH - W, CH, CH - W < LOW ? LOW : 0, false, false>(r, S, e0, 0, 0.0);
+  ys[32 * s] = y;
   __syncthreads();
-  const double yi = s > 0 ? ys[32 * (s - 1) + l] : (S.wrap_lo ? ys[32 * (T - 1) + l] : 0.0);
+  const double yi = before >= 0 ? ys[32 * before] : 0.0;
   double x;
   if (!low && !end) {
     chunk_fwd<CH, 0, CH, 0, false, true>(r, S, e0, 0, yi);
@@ -722,11 +563,40 @@ __device__ __forceinline__ void chunk_line_solve(double (&r)[CH], const ChunkSys
     chunk_fwd<CH, 0, CH, LOW, true, true>(r, S, e0, ql, yi);
     x = 0.0;
   }
-  xs[32 * s + l] = x;
-  __syncthreads();
-  const double xi = s + 1 < T ? xs[32 * (s + 1) + l] : (S.wrap_hi ? xs[l] : 0.0);
+  xs[32 * s] = x;
+  const bool far_y = feeds_up && off(r[CH - 1], y);
+  if (__syncthreads_or(far_y)) {
+    ys[32 * s] = far_y ? r[CH - 1] - y : 0.0;
+    __syncthreads();
+    const double d = before >= 0 ? ys[32 * before] : 0.0;
+    if (d != 0.0) {
+      double t[CH];
+#pragma unroll
+      for (int q = 0; q < CH; ++q) t[q] = r[q];
+      x = chunk_fwd_add(t, S, e0, CH, W, low ? LOW : 0, end ? ql : CH, d);
+      xs[32 * s] = x;
+#pragma unroll
+      for (int q = 0; q < CH; ++q) r[q] = t[q];
+    }
+    __syncthreads();
+  }
+  const double xi = after >= 0 ? xs[32 * after] : 0.0;
   if (low) chunk_bwd<CH, 0, CH, LOW, true>(r, S, e0, xi);
   else chunk_bwd<CH, 0, CH, 0, true>(r, S, e0, xi);
+  const bool far_x = feeds_down && off(r[0], x);
+  if (__syncthreads_or(far_x)) {
+    ys[32 * s] = far_x ? r[0] - x : 0.0;
+    __syncthreads();
+    const double d = after >= 0 ? ys[32 * after] : 0.0;
+    if (d != 0.0) {
+      double t[CH];
+#pragma unroll
+      for (int q = 0; q < CH; ++q) t[q] = r[q];
+      chunk_bwd_add(t, S, e0, CH, d);
+#pragma unroll
+      for (int q = 0; q < CH; ++q) r[q] = t[q];
+    }
+  }
 }
 
 // Pivot ratio by which the last row's right-hand side of a wall line is given
@@ -867,8 +737,8 @@ size_t line_smem(int axis, int ch, int T) {
   return (size_t)T * 32 * 16 + (axis == 0 ? (size_t)32 * line_pitch(ch, T) * sizeof(double2) : 0);
 }
 
-template <int AXIS, int CH, int W>
-__global__ void __launch_bounds__(32 * line_chunks_max(CH), CH == 16 ? 4 : (CH == 26 ? 2 : 3))
+template <int AXIS, int CH, int W, int TMAX>
+__global__ void __launch_bounds__(32 * TMAX, TMAX == 17 ? 1 : (CH == 16 ? 4 : (CH == 26 ? 2 : 3)))
     adi_line_chunk_kernel(const __grid_constant__ AdiArgs a) {
   extern __shared__ __align__(16) double sh_line[];
   const int fld = blockIdx.y;
@@ -881,14 +751,13 @@ __global__ void __launch_bounds__(32 * line_chunks_max(CH), CH == 16 ? 4 : (CH =
   else line_chunks<AXIS, CH, W>(a.L, a.ch[fld], J, blockIdx.x * 32, sh_line);
 }
 
-template <int AXIS, int CH, int W>
-cudaError_t launch_adi_line_chunk(const AdiArgs& a, int m, cudaStream_t st) {
+template <int AXIS, int CH, int W, int TMAX>
+cudaError_t launch_adi_line_chunk(const AdiArgs& a, int T, cudaStream_t st) {
   const int n1 = AXIS == 0 ? a.L.ny + 2 : a.L.nx + 2;
   const int n2 = AXIS == 2 ? a.L.ny + 2 : (a.z1 > 0 ? a.z1 - a.z0 : a.L.nz + 2);
   if (n2 <= 0) return cudaSuccess;
-  const int T = (m + CH - 1) / CH;
   const size_t sm = line_smem(AXIS, CH, T);
-  auto kern = adi_line_chunk_kernel<AXIS, CH, W>;
+  auto kern = adi_line_chunk_kernel<AXIS, CH, W, TMAX>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
   kern<<<dim3((unsigned)((n1 * n2 + 31) / 32), 3), dim3(32, T), sm, st>>>(a);
@@ -898,22 +767,32 @@ cudaError_t launch_adi_line_chunk(const AdiArgs& a, int m, cudaStream_t st) {
 // Unknowns per chunk: 32 or 26, whichever computes fewer (130, the unknowns of
 // a wall line of 128 cells: 5 x 26), and 16 on boxes whose 32-unknown chunks
 // leave SMs idle (a 32^3 sweep: 8 to 12 us against 20 a whole line).
-// Lines that do not fit a CTA take the chunks that work out their own halos.
+int adi_chunk(const Layout& L, const ChunkSys (&S)[3], int W) {
+  const int m = std::max(S[0].m, std::max(S[1].m, S[2].m));
+  const long long cells = 3LL * (L.nx + 2) * (L.ny + 2) * (L.nz + 2);
+  auto fits = [&](int ch) {
+    for (const ChunkSys& s : S)
+      if (!line_chunk_ok(s, ch, W)) return false;
+    return true;
+  };
+  if (cells / 32 < 40000 && fits(16)) return 16;
+  auto work = [&](int ch) { return fits(ch) ? (m + ch - 1) / ch * (ch + W) : 1 << 30; };
+  const int ch = work(26) < work(32) ? 26 : 32;
+  return fits(ch) ? ch : (fits(16) ? 16 : 0);  // 16: cyclic lines of 16 cells in a large box
+}
+
 cudaError_t launch_adi_chunks(int axis, const AdiArgs& a, cudaStream_t st) {
   const int m = std::max(a.ch[0].m, std::max(a.ch[1].m, a.ch[2].m));
-  const long long cells = 3LL * (a.L.nx + 2) * (a.L.ny + 2) * (a.L.nz + 2);
-  const int W = std::max(a.halo, 8);
-  auto work = [&](int c) { return (m + c - 1) / c * (c + W); };
-  const int ch = cells / 32 < 40000 && m <= 16 * line_chunks_max(16) ? 16 : (work(26) < work(32) ? 26 : 32);
-  bool fits = true;
-  for (const ChunkSys& S : a.ch) fits = fits && line_chunk_ok(S, ch, W);
-  if (!fits) return a.halo <= 8 ? launch_adi_chunk<32, 8>(axis, a, st) : launch_adi_chunk<32, 16>(axis, a, st);
-#define NS_ADI_LINE(A, C, H) \
-  if (axis == A && ch == C && W == H) return launch_adi_line_chunk<A, C, H>(a, m, st);
-#define NS_ADI_LINES(C, H) NS_ADI_LINE(0, C, H) NS_ADI_LINE(1, C, H) NS_ADI_LINE(2, C, H)
-  NS_ADI_LINES(16, 8) NS_ADI_LINES(16, 10) NS_ADI_LINES(16, 12) NS_ADI_LINES(16, 16)
-  NS_ADI_LINES(32, 8) NS_ADI_LINES(32, 10) NS_ADI_LINES(32, 12) NS_ADI_LINES(32, 16)
-  NS_ADI_LINES(26, 8) NS_ADI_LINES(26, 10) NS_ADI_LINES(26, 12) NS_ADI_LINES(26, 16)
+  const int ch = adi_chunk(a.L, a.ch, a.halo);
+  if (!ch) return cudaErrorInvalidValue;
+  const int T = (m + ch - 1) / ch, tmax = ch == 26 ? 10 : (T <= 8 ? 8 : 17);
+#define NS_ADI_LINE(A, C, H, M) \
+  if (axis == A && ch == C && a.halo == H && tmax == M) return launch_adi_line_chunk<A, C, H, M>(a, T, st);
+#define NS_ADI_LINES(C, H, M) NS_ADI_LINE(0, C, H, M) NS_ADI_LINE(1, C, H, M) NS_ADI_LINE(2, C, H, M)
+  NS_ADI_LINES(16, 8, 8) NS_ADI_LINES(16, 10, 8) NS_ADI_LINES(16, 12, 8) NS_ADI_LINES(16, 16, 8)
+  NS_ADI_LINES(32, 8, 8) NS_ADI_LINES(32, 10, 8) NS_ADI_LINES(32, 12, 8) NS_ADI_LINES(32, 16, 8)
+  NS_ADI_LINES(26, 8, 10) NS_ADI_LINES(26, 10, 10) NS_ADI_LINES(26, 12, 10) NS_ADI_LINES(26, 16, 10)
+  NS_ADI_LINES(32, 8, 17) NS_ADI_LINES(32, 10, 17) NS_ADI_LINES(32, 12, 17) NS_ADI_LINES(32, 16, 17)
 #undef NS_ADI_LINES
 #undef NS_ADI_LINE
   return cudaErrorInvalidValue;

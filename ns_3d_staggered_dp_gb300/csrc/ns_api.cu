@@ -112,7 +112,7 @@ HostChunkSys build_chunk_system(int n, int bc, double h, double dt, double nu, b
   }
   S.c0 = q0 - ext;
   S.c1 = q1 - ext;
-  for (int w : {6, 8, 10, 12, 16}) {  // the weight of what lies w unknowns away
+  for (int w : {8, 10, 12, 16}) {  // the weight of what lies w unknowns away
     bool ok = true;
     for (int q = 0; q + w <= len && ok; ++q) {
       double pl = 1, pc = 1;
@@ -1192,7 +1192,8 @@ int build_line_tables(ns_handle* h, bool transposed, LineSys sys[3][3], double**
   return NS_OK;
 }
 
-// The chunked sweeps' tables, when every system's halo is at most 16.  Their
+// The chunked sweeps' tables, when every system's halo is at most 16 and its
+// lines fit a CTA (544 unknowns; a box's x axis may be longer).  Their
 // right-hand sides are scaled by the product of the pivots still to come, so
 // a session that hands out u* between the sweeps (keep_sweeps) keeps the
 // whole-line kernels.
@@ -1226,6 +1227,12 @@ int build_line_chunks(ns_handle* h, bool transposed, ChunkSys csys[3][3], int ha
       D.wrap_lo = q.wrap_lo; D.wrap_hi = q.wrap_hi; D.periodic = q.periodic;
       d[ax] = q.d;  // the converged pivot is the same for the three fields
       halo[ax] = std::max(halo[ax], q.halo);
+    }
+  for (int ax = 0; ax < 3; ++ax)
+    if (!adi_chunk(h->L, csys[ax], halo[ax])) {
+      halo[0] = halo[1] = halo[2] = 0;
+      d[0] = d[1] = d[2] = 1.0;
+      return NS_OK;
     }
   NS_CUDA(h, cudaMemcpyAsync(*buf, host.data(), total * sizeof(double), cudaMemcpyHostToDevice, h->stream));
   NS_CUDA(h, cudaStreamSynchronize(h->stream));

@@ -194,9 +194,9 @@ struct LineSys {
   int n;               // cells along the axis
   int pad;             // zero padding on each side of the factor tables
 };
-// The same system for the chunked sweeps: every chunk of a line is solved by
-// itself, from `halo` unknowns before it to `halo` after it, because what lies
-// further away enters with a weight below 2^-57.  The rows' right-hand sides
+// The same system for the chunked sweeps: what enters a chunk of a line is
+// worked out from the `halo` unknowns beside it, because what lies further away
+// enters with a weight below 2^-57.  The rows' right-hand sides
 // come scaled by 1 / (converged pivot), so that a row with the converged
 // factors takes one FMA each way: y' = r - lc y', x = y' - cc x.
 struct ChunkSys {
@@ -218,11 +218,13 @@ struct AdiArgs {
   const double* face_lo[3];  // BC row values per field (internal-slot planes), NULL -> 0
   const double* face_hi[3];
   int z0, z1;                // x and y sweeps: only the lines of z slots [z0, z1) (z1 = 0: all)
-  int halo;                  // chunked sweeps: unknowns beyond a chunk (6, 8, 10, 12 or 16; 0: the whole-line kernels)
+  int halo;                  // chunked sweeps: unknowns beyond a chunk (8, 10, 12 or 16; 0: the whole-line kernels)
   ChunkSys ch[3];
   double face_scale;         // chunked sweeps: the scale of this sweep's right-hand sides
 };
 cudaError_t launch_adi(int axis, const AdiArgs& a, cudaStream_t st);
+// Unknowns per chunk of one axis' chunked sweep of a box with halo W (0: its lines do not fit).
+int adi_chunk(const Layout& L, const ChunkSys (&S)[3], int W);
 // The tile loader's bounded mbarrier wait on a barrier that no copy fills (ns_predict.cu).
 cudaError_t launch_wait_selftest(unsigned long long limit_ns, int* gave_up, unsigned long long* waited_ns,
                                  cudaStream_t st);
