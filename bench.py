@@ -83,10 +83,9 @@ def fp64_per_cell(kernel, n):
 
 FP64_LANES_PER_CLK_SM = 2  # DFMA issue rate of this part (ncu ..._op_dfma_pred_on.sum.peak_sustained)
 
-# DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) of one
-# ncu capture of the predictor and its pass over the plane maxima at 128^3,
-# times the 8 times as many cells.
-NCU_TRAFFIC_256 = {"predict": 8 * 226.5e6}
+# DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum): one ncu
+# capture of the predictor at 256^3.
+NCU_TRAFFIC_256 = {"predict": 1052.9e6 + 793.6e6}
 
 
 @functools.lru_cache(maxsize=2)
