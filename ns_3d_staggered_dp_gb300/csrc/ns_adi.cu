@@ -453,9 +453,8 @@ cudaError_t launch_adi_batch(int axis, const BatchAdiArgs* tab, const BatchItem*
 // (chunk_fwd_add, chunk_bwd_add): what is still left out lies below 2^-114.
 //
 // Bound by the FP64 unit, 75 to 80% busy.  Sweeps x, y, z in us (one thread a
-// line): 256^3 274, 259, 262 (512, 385, 369), 128^3 53, 46, 47, with walls 63,
-// 55, 55, 32^3 13, 8, 10; the comparison costs nothing (without it 279, 265,
-// 266 at 256^3).
+// line): 256^3 291, 257, 260 (512, 385, 369), 128^3 55, 46, 49, with walls 64,
+// 55, 55, 32^3 13, 8, 9; without the comparison 280, 265, 267 at 256^3.
 // The same in 58-bit integers with the exponent of the line takes 319, 296,
 // 292 at 256^3: the chain of a product waits longer there than for an FMA.
 // The batch keeps the whole-line kernels: 185, 108, 107 us for 64 blocks of 16
@@ -506,6 +505,10 @@ __device__ __forceinline__ double chunk_bwd(double (&r)[CH], const ChunkSys& S, 
 __device__ __forceinline__ bool off(double a, double b) {
   return (unsigned long long)(__double_as_longlong(a) - __double_as_longlong(b) + 4) > 8;
 }
+// d more or less of a row's value y is no more than another rounding of it (and then of the rows behind,
+// which hear of it through y).  In noise a value that happens to be small is off in one CTA of a hundred;
+// the part run through all rows made the last CTA late (64 x 128 x 128: 30 us to 48, now 32).
+__device__ __forceinline__ bool small(double d, double y) { return fabs(d) <= 0x1p-56 * fabs(y); }
 // The rare part, on a copy of the chunk in local memory (unrolled over the registers it made the kernels
 // too long for the instruction cache: the 128^3 box's step 10% slower, with no chunk taking it).
 // Forward: y that enters is d more than was taken; returns what the chunk then hands on backward.
@@ -518,6 +521,7 @@ __device__ __noinline__ double chunk_fwd_add(double* r, const ChunkSys& S, int e
 #pragma unroll 1
   for (int q = 0; q < ch && q <= ql; ++q) {
     d *= q == ql && q >= low ? -l[q] * dm[q] : -l[q];
+    if (small(d, r[q])) break;
     r[q] += d;
   }
   double x = 0.0;
@@ -530,6 +534,7 @@ __device__ __noinline__ void chunk_bwd_add(double* r, const ChunkSys& S, int e0,
 #pragma unroll 1
   for (int q = ch - 1; q >= 0; --q) {
     d *= -cu[q];
+    if (small(d, r[q])) break;
     r[q] += d;
   }
 }
@@ -569,7 +574,7 @@ __device__ __forceinline__ void chunk_line_solve(double (&r)[CH], const ChunkSys
     ys[32 * s] = far_y ? r[CH - 1] - y : 0.0;
     __syncthreads();
     const double d = before >= 0 ? ys[32 * before] : 0.0;
-    if (d != 0.0) {
+    if (d != 0.0 && !small(d * __ldg(S.l + kAdiExt + e0), r[0])) {  // (noise: a small value beside others)
       double t[CH];
 #pragma unroll
       for (int q = 0; q < CH; ++q) t[q] = r[q];
@@ -588,7 +593,7 @@ __device__ __forceinline__ void chunk_line_solve(double (&r)[CH], const ChunkSys
     ys[32 * s] = far_x ? r[0] - x : 0.0;
     __syncthreads();
     const double d = after >= 0 ? ys[32 * after] : 0.0;
-    if (d != 0.0) {
+    if (d != 0.0 && !small(d * __ldg(S.cu + kAdiExt + e0 + CH - 1), r[CH - 1])) {
       double t[CH];
 #pragma unroll
       for (int q = 0; q < CH; ++q) t[q] = r[q];
